@@ -9,6 +9,7 @@
 #include <functional>
 #include <initializer_list>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -76,6 +77,16 @@ struct cfdb_ctx {
   // call of the same size neither allocates nor frees device memory.
   cudaMemPool_t pool = nullptr;
   std::unordered_map<void*, int64_t> ws;
+  // Scratch of the synchronous reductions (CFL step, FP64 totals): per-CTA
+  // partials, the last-CTA ticket and a page-locked word the kernel stores the
+  // result to.  A call holds the mutex until it has read its result, so calls
+  // on any stream or thread never share the scratch.
+  struct Reduce {
+    void* part = nullptr;
+    unsigned int* ticket = nullptr;
+    void* host = nullptr;
+    std::mutex mu;
+  } reduce;
   int* d_error = nullptr;  // device error word written by bounded waits
   // Bound of the sweep kernels' mbarrier waits (SM clock cycles) and the
   // missing-copy test hook (cfdb_ctx_set_wait_limit).
@@ -185,6 +196,10 @@ void cfdb_dev_free(cfdb_ctx* ctx, void* p);
 // Counts toward the allocation budget while live.
 int cfdb_ws_alloc(cfdb_ctx* ctx, int64_t bytes, void** out);
 void cfdb_ws_free(cfdb_ctx* ctx, void* p);
+// CFDB_ENOMEM when a workspace of `bytes` would exceed the allocation budget
+// (calls that use scratch the context already owns keep answering as if they
+// allocated it).
+int cfdb_ws_budget(cfdb_ctx* ctx, int64_t bytes);
 
 // ---- module loading ---------------------------------------------------------
 // CUDA loads a kernel at its first launch by default (lazy loading), which

@@ -14,50 +14,6 @@ CFDB_MODULE_ANCHOR
 
 namespace {
 
-__device__ __forceinline__ double bits_to_double(unsigned long long b) { return __longlong_as_double((long long)b); }
-
-__device__ __forceinline__ void comp_add(double& s, double& c, double x) {
-  const double t = s + x;
-  if (fabs(s) >= fabs(x)) c += (s - t) + x; else c += (x - t) + s;
-  s = t;
-}
-
-// Folds the per-CTA FP64 partials part[0 .. nblocks) into totals row `step`
-// with every thread of the calling CTA, in a fixed order: thread t takes
-// partials t, t + blockDim, ..., the lanes of each warp merge through
-// shuffles in a fixed pattern and thread 0 merges the warps in order, so the
-// totals do not depend on timing (one thread folding every partial serially
-// had cost ~13 us per step).
-__device__ void fold_partials(const Comp2* __restrict__ part, int nblocks, double* totals, long long step) {
-  __shared__ double sh[32][4];
-  double S0 = 0, C0 = 0, S1 = 0, C1 = 0;
-  for (int k = int(threadIdx.x); k < nblocks; k += int(blockDim.x)) {
-    const Comp2 q = part[k];
-    comp_add(S0, C0, q.s0); C0 += q.c0;
-    comp_add(S1, C1, q.s1); C1 += q.c1;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double a0 = __shfl_xor_sync(0xffffffffu, S0, o), b0 = __shfl_xor_sync(0xffffffffu, C0, o);
-    const double a1 = __shfl_xor_sync(0xffffffffu, S1, o), b1 = __shfl_xor_sync(0xffffffffu, C1, o);
-    comp_add(S0, C0, a0); C0 += b0;
-    comp_add(S1, C1, a1); C1 += b1;
-  }
-  const int w = int(threadIdx.x) >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    sh[w][0] = S0; sh[w][1] = C0; sh[w][2] = S1; sh[w][3] = C1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    S0 = C0 = S1 = C1 = 0;
-    for (int k = 0; k < int(blockDim.x / 32); ++k) {
-      comp_add(S0, C0, sh[k][0]); C0 += sh[k][1];
-      comp_add(S1, C1, sh[k][2]); C1 += sh[k][3];
-    }
-    totals[2 * step] = S0 + C0;
-    totals[2 * step + 1] = S1 + C1;
-  }
-}
-
 struct EulerPhys {
   static constexpr int NF = 5;
   static constexpr int MIN_BLOCKS = 2;  // 64x8 tile, 2 cells per thread: 256 threads at <= 128 registers

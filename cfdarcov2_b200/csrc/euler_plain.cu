@@ -29,8 +29,6 @@ template <class R> __device__ __forceinline__ Prim<R> prim(R rho, R mx, R my, R 
   return s;
 }
 
-__device__ __forceinline__ double bits_to_double(unsigned long long b) { return __longlong_as_double((long long)b); }
-
 template <class R> struct PlainEulerArgs {
   const int32_t* __restrict__ ids;
   const R* __restrict__ nalt;  // 3 x 6n
@@ -89,12 +87,6 @@ __global__ void __launch_bounds__(kThreads) euler_plain_step_k(PlainEulerArgs<R>
 #pragma unroll
     for (int c = 0; c < 5; ++c) Un[c * n + i] = dt * (-(acc[c] / V)) + U[c * n + i];
   }
-}
-
-__device__ __forceinline__ void comp_add(double& s, double& c, double x) {
-  const double t = s + x;
-  if (fabs(s) >= fabs(x)) c += (s - t) + x; else c += (x - t) + s;
-  s = t;
 }
 
 // Per-direction max speeds + Neumaier totals of U; the last CTA finalises.
@@ -166,37 +158,29 @@ __global__ void __launch_bounds__(kThreads) euler_reduce_k(const R* __restrict__
     is_last = atomicAdd(&ck->counter, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (is_last && threadIdx.x == 0) {
-    __threadfence();
-    double S0 = 0, C0 = 0, S1 = 0, C1 = 0;
-    for (unsigned k = 0; k < gridDim.x; ++k) {
-      const Comp2 p = part[k];
-      comp_add(S0, C0, p.s0); C0 += p.c0;
-      comp_add(S1, C1, p.s1); C1 += p.c1;
-    }
+  if (!is_last) return;
+  __threadfence();
+  long long step = 0;
+  if (!begin_mode) step = ck->steps[ts] + 1;
+  fold_partials(part, int(gridDim.x), totals, step);
+  if (threadIdx.x == 0) {
     ck->counter = 0;
-    if (begin_mode) {
-      totals[0] = S0 + C0;
-      totals[1] = S1 + C1;
-    } else {
+    if (!begin_mode) {
       const int ls = int(s % 3);
       const double lam[3] = {bits_to_double(ck->lam[ls][0]), bits_to_double(ck->lam[ls][1]), bits_to_double(ck->lam[ls][2])};
       bool last;
       const double t = ck->t[ts];
       const double dt = euler_dt(lam, dx, dy, dz, cfl, t, t_end, &last);
-      const long long step = ck->steps[ts] + 1;
       ck->t[ts ^ 1] = last ? t_end : t + dt;
       ck->steps[ts ^ 1] = step;
       ck->finished[ts ^ 1] = (last || !(t + dt < t_end) || step >= max_steps) ? 1 : 0;
-      totals[2 * step] = S0 + C0;
-      totals[2 * step + 1] = S1 + C1;
     }
   }
 }
 
 }  // namespace
 
-int euler_reduce_grid(const cfdb_euler* e) { return grid_for(e->ctx, e->mesh->n, kThreads, 2); }
+int euler_reduce_grid(const cfdb_euler* e) { return grid_for(e->ctx, e->mesh->n, kThreads, 4); }
 
 int euler_plain_step(cfdb_euler* e, const void* U, void* Un, int64_t s) {
   cfdb_ctx* ctx = e->ctx;

@@ -262,32 +262,87 @@ __global__ void bset_many_k(SetBatch<R> b, int64_t nx, int64_t ny, int64_t nz) {
 }
 
 // ---- reductions -------------------------------------------------------------
-__device__ __forceinline__ void atomic_min_pos(float* a, float v) { atomicMin(reinterpret_cast<int*>(a), __float_as_int(v)); }
-__device__ __forceinline__ void atomic_min_pos(double* a, double v) {
-  atomicMin(reinterpret_cast<unsigned long long*>(a), static_cast<unsigned long long>(__double_as_longlong(v)));
+// One launch each, result in page-locked host memory: every CTA leaves its
+// partial in the context's scratch and takes a ticket; the CTA that draws the
+// last one folds all partials with all its threads and stores the result
+// where the host reads it after the stream has been waited for.  (A second
+// launch in which one thread folded 296 partials in turn had cost 31 us per
+// total, and the two copies around the CFL minimum about 10 us per call.)  The
+// fold order depends on the grid only, so results repeat bit for bit.
+
+// true for every thread of the CTA that finishes last; tickets wrap to zero
+// by themselves, ready for the next launch
+__device__ __forceinline__ bool last_cta(unsigned int* ticket) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
 }
 
-// cfl_cu_k + thrust::min_element (src/cuda_operators.cu:138-235).
-template <class R>
-__global__ void cfl_k(R dl, R gamma, const R* __restrict__ p, const R* __restrict__ rho, const R* __restrict__ u,
-                      const R* __restrict__ v, const R* __restrict__ w, int64_t n, R* __restrict__ result) {
+// 4 consecutive values
+__device__ __forceinline__ void load4(const float* p, float* v) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void load4(const double* p, double* v) {
+  const double2 s = reinterpret_cast<const double2*>(p)[0], t = reinterpret_cast<const double2*>(p)[1];
+  v[0] = s.x; v[1] = s.y; v[2] = t.x; v[3] = t.y;
+}
+
+template <class R> __device__ __forceinline__ R block_max(R v) {
   __shared__ R red[kThreads / 32];
-  R best = R(INFINITY);
-  GRID_STRIDE(i, n) {
-    R vv = u[i] * u[i];
-    if (v) vv = vv + v[i] * v[i];
-    if (w) vv = vv + w[i] * w[i];
-    const R den = dl * (R(1) / (sqrt((gamma * p[i]) / rho[i]) + sqrt(vv)));
-    best = fmin(best, den);
-  }
-  for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = best;
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    best = threadIdx.x < blockDim.x / 32 ? red[threadIdx.x] : R(INFINITY);
-    for (int o = 16; o > 0; o >>= 1) best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (threadIdx.x == 0) atomic_min_pos(result, best);
+  v = red[threadIdx.x & (kThreads / 32 - 1)];
+  for (int o = kThreads / 64; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+// cfl_cu_k + thrust::min_element (src/cuda_operators.cu:138-235): the minimum
+// over the cells of dl (1 / s), s = sqrt(gamma p / rho) + |u|.  1 / s and the
+// product round monotonically, so the minimum is that of the largest s, and
+// the division is done once; a cell whose s is NaN drops out of both.
+// Bounds: 20 B (FP32) per cell read once; 4 cells per thread and pass keep
+// 20 loads in flight per thread (200^3 FP32: 48 us with one cell per thread
+// and a division in every cell).
+template <class R, bool VEC>
+__global__ void __launch_bounds__(kThreads) cfl_k(R dl, R gamma, const R* __restrict__ p, const R* __restrict__ rho,
+                                                  const R* __restrict__ u, const R* __restrict__ v,
+                                                  const R* __restrict__ w, int64_t n, R* __restrict__ part,
+                                                  unsigned int* __restrict__ ticket, R* __restrict__ result) {
+  R best = -R(INFINITY);
+  auto cell = [&](R pc, R rc, R uc, R vc, R wc) {
+    R vv = uc * uc;
+    if (v) vv = vv + vc * vc;
+    if (w) vv = vv + wc * wc;
+    best = fmax(best, sqrt((gamma * pc) / rc) + sqrt(vv));
+  };
+  const int64_t n4 = VEC ? n / 4 : 0;
+  GRID_STRIDE(q, n4) {
+    R a[4], b[4], c[4], d[4] = {}, e[4] = {};
+    load4(p + 4 * q, a);
+    load4(rho + 4 * q, b);
+    load4(u + 4 * q, c);
+    if (v) load4(v + 4 * q, d);
+    if (w) load4(w + 4 * q, e);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) cell(a[j], b[j], c[j], d[j], e[j]);
   }
+  for (int64_t i = 4 * n4 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    cell(p[i], rho[i], u[i], v ? v[i] : R(0), w ? w[i] : R(0));
+  best = block_max(best);
+  if (threadIdx.x == 0) part[blockIdx.x] = best;
+  if (!last_cta(ticket)) return;
+  best = -R(INFINITY);
+  for (int k = threadIdx.x; k < int(gridDim.x); k += kThreads) best = fmax(best, __ldcg(part + k));
+  best = block_max(best);
+  if (threadIdx.x == 0) *result = best >= R(0) ? dl * (R(1) / best) : R(INFINITY);
 }
 
 // Neumaier (compensated) accumulation of field * V in double.
@@ -301,31 +356,52 @@ __device__ __forceinline__ void comp_merge(Comp& a, Comp b) {
   comp_add(a, b.s);
   a.c += b.c;
 }
-
-template <class R>
-__global__ void total_k(const R* __restrict__ f, const R* __restrict__ vol, double vconst, int64_t n, Comp* __restrict__ part) {
+// the CTA's pairs merged in a fixed order; valid in thread 0
+__device__ __forceinline__ Comp comp_block(Comp a) {
   __shared__ Comp red[kThreads / 32];
-  Comp a{0.0, 0.0};
-  GRID_STRIDE(i, n) comp_add(a, double(f[i]) * (vol ? double(vol[i]) : vconst));
   for (int o = 16; o > 0; o >>= 1) {
     Comp b{__shfl_xor_sync(0xffffffffu, a.s, o), __shfl_xor_sync(0xffffffffu, a.c, o)};
     comp_merge(a, b);
   }
+  __syncthreads();
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    Comp t{0.0, 0.0};
-    for (int w = 0; w < int(blockDim.x / 32); ++w) comp_merge(t, red[w]);
-    part[blockIdx.x] = t;
-  }
+  Comp t{0.0, 0.0};
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kThreads / 32; ++w) comp_merge(t, red[w]);
+  return t;
 }
 
-__global__ void total_final_k(const Comp* __restrict__ part, int np, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    Comp t{0.0, 0.0};
-    for (int k = 0; k < np; ++k) comp_merge(t, part[k]);
-    out[0] = t.s + t.c;
+// Total of field * V.  A compensated sum is one dependent chain per
+// accumulator, so a thread keeps four (one per value of its 16- or 32-byte
+// load); one chain per thread had taken 36 us at 200^3 FP32 (32 MB).
+template <class R, bool VEC>
+__global__ void __launch_bounds__(kThreads) total_k(const R* __restrict__ f, const R* __restrict__ vol, double vconst,
+                                                    int64_t n, Comp* __restrict__ part,
+                                                    unsigned int* __restrict__ ticket, double* __restrict__ result) {
+  Comp a[4] = {};
+  const int64_t n4 = VEC ? n / 4 : 0;
+  GRID_STRIDE(q, n4) {
+    R x[4], y[4];
+    load4(f + 4 * q, x);
+    if (vol) load4(vol + 4 * q, y);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) comp_add(a[j], double(x[j]) * (vol ? double(y[j]) : vconst));
   }
+  for (int64_t i = 4 * n4 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+    comp_add(a[0], double(f[i]) * (vol ? double(vol[i]) : vconst));
+#pragma unroll
+  for (int j = 1; j < 4; ++j) comp_merge(a[0], a[j]);
+  Comp t = comp_block(a[0]);
+  if (threadIdx.x == 0) part[blockIdx.x] = t;
+  if (!last_cta(ticket)) return;
+  t = Comp{0.0, 0.0};
+  for (int k = threadIdx.x; k < int(gridDim.x); k += kThreads) {
+    const double2 q = __ldcg(reinterpret_cast<const double2*>(part + k));
+    comp_merge(t, Comp{q.x, q.y});
+  }
+  t = comp_block(t);
+  if (threadIdx.x == 0) *result = t.s + t.c;
 }
 
 // ---- the acoustic system on the general geometry ------------------------------
@@ -438,6 +514,15 @@ int check_ptrs(cfdb_ctx* ctx, const char* fn, std::initializer_list<const void*>
   for (const void* p : ps)
     if (!p) return cfdb_fail(ctx, CFDB_EINVAL, "%s: NULL field pointer", fn);
   return CFDB_OK;
+}
+
+// CTAs per SM of the reductions (the context holds partials for 8)
+constexpr int kReducePerSm = 4;
+
+bool aligned16(std::initializer_list<const void*> ps) {
+  uintptr_t bits = 0;
+  for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
+  return (bits & 15u) == 0;
 }
 
 int check_n(cfdb_ctx* ctx, int dtype, int64_t n, const char* fn) {
@@ -621,24 +706,21 @@ extern "C" int cfdb_cfl_dt(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, double cfl, d
   if (int rc = check_ptrs(ctx, "cfdb_cfl_dt", {p, rho, u, dt_out})) return rc;
   if ((v == nullptr) != (w == nullptr)) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_cfl_dt: give both v and w or neither");
   CFDB_CUDA(ctx, cudaSetDevice(ctx->device));
-  void* res = nullptr;
-  if (int rc = cfdb_ws_alloc(ctx, 8, &res)) return rc;
-  int rc = CFDB_OK;
+  if (int rc = cfdb_ws_budget(ctx, 8)) return rc;
   double host = 0;
+  std::lock_guard<std::mutex> lock(ctx->reduce.mu);
   DISPATCH(dtype, R, {
-    const R inf = R(INFINITY);
-    cudaMemcpyAsync(res, &inf, sizeof(R), cudaMemcpyHostToDevice, ctx->stream);
     const R dl = fmin(fmin(R(m->dx), R(m->dy)), R(m->dz));
-    cfl_k<R><<<grid_for(ctx, m->n, kThreads, 4), kThreads, 0, ctx->stream>>>(dl, R(gamma), (const R*)p, (const R*)rho,
-                                                                              (const R*)u, (const R*)v, (const R*)w, m->n, (R*)res);
-    R mn = 0;
-    cudaError_t e = cudaMemcpyAsync(&mn, res, sizeof(R), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) rc = cfdb_cuda_fail(ctx, e, "cfdb_cfl_dt");
-    host = double(R(cfl) * mn);
+    const bool vec = aligned16({p, rho, u, v, w});
+    const int grid = grid_for(ctx, vec ? (m->n + 3) / 4 : m->n, kThreads, kReducePerSm);
+    auto kern = vec ? cfl_k<R, true> : cfl_k<R, false>;
+    R* result = static_cast<R*>(ctx->reduce.host);
+    kern<<<grid, kThreads, 0, ctx->stream>>>(dl, R(gamma), (const R*)p, (const R*)rho, (const R*)u, (const R*)v, (const R*)w,
+                                             m->n, static_cast<R*>(ctx->reduce.part), ctx->reduce.ticket, result);
+    CFDB_LAUNCHED(ctx);
+    CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    host = double(R(cfl) * *static_cast<volatile R*>(result));
   });
-  cfdb_ws_free(ctx, res);
-  if (rc) return rc;
   if (!std::isfinite(host) || !(host > 0)) return cfdb_fail(ctx, CFDB_ENUMERIC, "cfdb_cfl_dt: non-finite or non-positive dt %g", host);
   *dt_out = host;
   return CFDB_OK;
@@ -655,17 +737,19 @@ extern "C" int cfdb_total_fp64(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const voi
     vol = m->plain[dtype == CFDB_F64 ? 1 : 0].volume;
   }
   const double vconst = m->dx * m->dy * m->dz;
-  const int grid = grid_for(ctx, m->n, kThreads, 2);
-  void* scratch = nullptr;
-  if (int rc = cfdb_ws_alloc(ctx, int64_t(sizeof(Comp)) * grid + 16, &scratch)) return rc;
-  Comp* part = static_cast<Comp*>(scratch);
-  double* res = reinterpret_cast<double*>(part + grid);
-  DISPATCH(dtype, R, total_k<R><<<grid, kThreads, 0, ctx->stream>>>((const R*)field, (const R*)vol, vconst, m->n, part));
-  total_final_k<<<1, 32, 0, ctx->stream>>>(part, grid, res);
-  cudaError_t e = cudaMemcpyAsync(out, res, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cfdb_ws_free(ctx, scratch);
-  if (e != cudaSuccess) return cfdb_cuda_fail(ctx, e, "cfdb_total_fp64");
+  const bool vec = aligned16({field, vol});
+  const int grid = grid_for(ctx, vec ? (m->n + 3) / 4 : m->n, kThreads, kReducePerSm);
+  if (int rc = cfdb_ws_budget(ctx, int64_t(sizeof(Comp)) * grid_for(ctx, m->n, kThreads, 2) + 16)) return rc;
+  std::lock_guard<std::mutex> lock(ctx->reduce.mu);
+  double* result = static_cast<double*>(ctx->reduce.host);
+  DISPATCH(dtype, R, {
+    auto kern = vec ? total_k<R, true> : total_k<R, false>;
+    kern<<<grid, kThreads, 0, ctx->stream>>>((const R*)field, (const R*)vol, vconst, m->n,
+                                             static_cast<Comp*>(ctx->reduce.part), ctx->reduce.ticket, result);
+  });
+  CFDB_LAUNCHED(ctx);
+  CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  *out = *static_cast<volatile double*>(result);
   return CFDB_OK;
 }
 

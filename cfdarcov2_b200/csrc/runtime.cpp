@@ -132,6 +132,61 @@ int make_pool(cfdb_ctx* ctx) {
   CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return CFDB_OK;
 }
+
+// Page-locked words the reduction kernels store their results to, one slot of
+// 64 bytes per context, from one page per process (page-locking costs 0.4 ms,
+// as much as the rest of a context).  The page stays for the life of the
+// process; slots go back when a context is destroyed, and a context beyond
+// the page's slots gets memory of its own.
+class HostSlots {
+ public:
+  int take(cfdb_ctx* ctx, void** out) {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!page_) CFDB_CUDA(ctx, cudaHostAlloc(&page_, kSlots * 64, cudaHostAllocPortable | cudaHostAllocMapped));
+    for (int k = 0; k < kSlots; ++k)
+      if (!used_[k]) {
+        used_[k] = true;
+        *out = static_cast<char*>(page_) + 64 * k;
+        return CFDB_OK;
+      }
+    CFDB_CUDA(ctx, cudaHostAlloc(out, 64, cudaHostAllocPortable | cudaHostAllocMapped));
+    return CFDB_OK;
+  }
+  void give(void* p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(mu_);
+    const ptrdiff_t off = static_cast<char*>(p) - static_cast<char*>(page_);
+    if (page_ && off >= 0 && off < kSlots * 64) used_[off / 64] = false;
+    else cudaFreeHost(p);
+  }
+
+ private:
+  static constexpr int kSlots = 64;
+  std::mutex mu_;
+  void* page_ = nullptr;
+  bool used_[kSlots] = {};
+};
+HostSlots& host_slots() {
+  static HostSlots* s = new HostSlots();  // not destroyed: contexts may outlive static destructors
+  return *s;
+}
+
+// Scratch of the synchronous reductions, held for the life of the context:
+// a 32-byte partial for up to 8 CTAs per SM from the pool, the ticket behind
+// the error word and a page-locked result.
+int make_reduce(cfdb_ctx* ctx) {
+  const size_t parts = size_t(32) * 8 * size_t(std::max(1, ctx->num_sms));
+  CFDB_CUDA(ctx, cudaMallocFromPoolAsync(&ctx->reduce.part, parts, ctx->pool, ctx->stream));
+  ctx->reduce.ticket = reinterpret_cast<unsigned int*>(ctx->d_error + 2);
+  if (int rc = host_slots().take(ctx, &ctx->reduce.host)) return rc;
+  CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the context's stream may change before the first use
+  return CFDB_OK;
+}
+
+void free_reduce(cfdb_ctx* ctx) {
+  if (ctx->reduce.part) cudaFreeAsync(ctx->reduce.part, ctx->stream);
+  host_slots().give(ctx->reduce.host);
+}
 }  // namespace
 
 int cfdb_register_module(const void* anchor_kernel) {
@@ -139,12 +194,17 @@ int cfdb_register_module(const void* anchor_kernel) {
   return 0;
 }
 
-int cfdb_ws_alloc(cfdb_ctx* ctx, int64_t bytes, void** out) {
-  *out = nullptr;
-  if (bytes <= 0) bytes = 16;
+int cfdb_ws_budget(cfdb_ctx* ctx, int64_t bytes) {
   if (ctx->budget > 0 && ctx->allocated + bytes > ctx->budget)
     return cfdb_fail(ctx, CFDB_ENOMEM, "workspace of %lld bytes exceeds the context budget (%lld of %lld used)",
                      (long long)bytes, (long long)ctx->allocated, (long long)ctx->budget);
+  return CFDB_OK;
+}
+
+int cfdb_ws_alloc(cfdb_ctx* ctx, int64_t bytes, void** out) {
+  *out = nullptr;
+  if (bytes <= 0) bytes = 16;
+  if (int rc = cfdb_ws_budget(ctx, bytes)) return rc;
   if (!ctx->pool)
     if (int rc = make_pool(ctx)) return rc;
   void* p = nullptr;
@@ -227,8 +287,10 @@ extern "C" int cfdb_ctx_create(int device, cfdb_ctx** out) {
     delete ctx;
     return r;
   }
-  if ((rc = make_pool(ctx))) {
+  if ((rc = make_pool(ctx)) || (rc = make_reduce(ctx))) {
     g_err_noctx = ctx->err;
+    free_reduce(ctx);
+    cudaStreamSynchronize(ctx->stream);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     cfdb_dev_free(ctx, ctx->d_error);
     delete ctx;
@@ -250,6 +312,7 @@ extern "C" int cfdb_ctx_destroy(cfdb_ctx* ctx) {
   for (auto& kv : children) kv.second();
   for (auto& kv : ctx->allocs) cudaFree(kv.first);
   ctx->allocs.clear();
+  free_reduce(ctx);
   if (ctx->pool) {
     for (auto& kv : ctx->ws) cudaFreeAsync(kv.first, ctx->stream);
     cudaStreamSynchronize(ctx->stream);
