@@ -48,6 +48,30 @@ struct PlainGeomDev {
   void* stab_tmp = nullptr;    // 3 * 6n, allocated on first stab call
 };
 
+// Geometry of a structured mesh along one axis, in double: edge lengths (n),
+// face-plane coordinates (n + 1), alpha of the face below cell i (n + 1) and
+// |x_f - x_P| of a cell's lower and upper face (n each).
+struct AxisTables {
+  std::vector<double> h, g, alpha, len_lo, len_hi;
+};
+// Fills t[0..2] (x, y, z) and returns the magnitude up to which an operand
+// overflows in no intermediate of the operators; NaN when the face arrays of
+// this mesh do not follow exactly from values per axis (geometry.cpp).
+double axis_tables(int64_t nx, int64_t ny, int64_t nz, double dx, double dy, double dz, bool f64, AxisTables t[3]);
+
+// The same tables on the device in one precision (box_ops.cu), in place of
+// the face arrays: h in double, the rest in the storage type; vol (n) is null
+// when every cell's volume rounds to v.
+struct BoxGeomDev {
+  int state = 0;  // 0 not built, 1 usable, 2 this mesh keeps the face arrays
+  void* tab = nullptr;
+  void* vol = nullptr;
+  const double* h[3] = {};
+  const void* alpha[3] = {};
+  const void* len[6] = {};  // x-, x+, y-, y+, z-, z+
+  double v = 0, limit = 0;
+};
+
 // Compact FP32 geometry of vertex meshes for the fused kernels: per cell the
 // outward area vector of its +x/+y/+z face and 1/V (10 fields), stored on
 // the lattice padded by one ghost layer below each axis (x and y) and by four
@@ -148,6 +172,7 @@ struct cfdb_mesh {
   int32_t* d_ids = nullptr;
   PlainGeomDev plain[2];
   CompactGeomDev compact;
+  BoxGeomDev box[2];  // structured meshes, by precision
   int lattice_state = 0;  // 0 not checked, 1 exact lattice, 2 not one
   cfdb_lattice_geometry lattice{};
 };
@@ -237,6 +262,13 @@ int plain_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void*
                     double cconst, int mode, double dt);
 int plain_wave_adjoint(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, const void* lam1, void* lam0,
                        const void* c, void* gc, double dt);
+// box_ops.cu: the same operators on structured meshes without face arrays.
+// *usable = false: this mesh takes the array kernels.
+int cfdb_mesh_need_box(cfdb_mesh* m, int dtype, bool* usable);
+int box_grad(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask);
+int box_lapl(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask);
+int box_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* Tn, double k, double dt);
+int box_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask);
 // fused_tma.cu
 int fused_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* Tn, double k, double dt,
                     const void* fixed = nullptr);

@@ -514,6 +514,8 @@ void cfdb_mesh_orphan(cfdb_mesh* m) {
   m->plain[1] = PlainGeomDev();
   m->d_ids = nullptr;
   m->compact = CompactGeomDev();
+  m->box[0] = BoxGeomDev();
+  m->box[1] = BoxGeomDev();
 }
 
 extern "C" int cfdb_mesh_destroy(cfdb_mesh* m) {
@@ -525,6 +527,10 @@ extern "C" int cfdb_mesh_destroy(cfdb_mesh* m) {
     free_plain(m->ctx, m->plain[1]);
     cfdb_dev_free(m->ctx, m->d_ids);
     cfdb_dev_free(m->ctx, m->compact.S);
+    for (BoxGeomDev& b : m->box) {
+      cfdb_dev_free(m->ctx, b.tab);
+      cfdb_dev_free(m->ctx, b.vol);
+    }
   }
   delete m;
   return CFDB_OK;

@@ -21,6 +21,9 @@ extern "C" int cfdb_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int path, 
   if (T == Tn) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_heat_step: T and T_next must differ (no in-place stencil writes)");
   if (!std::isfinite(k) || !std::isfinite(dt)) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_heat_step: k and dt must be finite");
   if (path == CFDB_PATH_FUSED) return fused_heat_step(ctx, m, dtype, T, Tn, k, dt);
+  bool box = false;
+  if (int rc = cfdb_mesh_need_box(m, dtype, &box)) return rc;
+  if (box) return box_heat_step(ctx, m, dtype, T, Tn, k, dt);
   if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
   PlainGeomDev& p = m->plain[dtype == CFDB_F64 ? 1 : 0];
   if (!p.stab_tmp)

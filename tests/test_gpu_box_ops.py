@@ -1,0 +1,65 @@
+"""The operators and plain steps on structured meshes without face arrays
+against the face-array kernels: a vertex mesh on the same lattice points with
+the reference's formulas has the same face arrays and takes the array
+kernels, so both must give the same bits (sizes around one cell per
+direction, ragged columns, several planes per thread; operands that are not
+finite or overflow)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+SHAPES = [((1, 1, 1), (0.5, 0.3, 0.2)), ((1, 4, 4), (1.0, 1.0, 1.0)), ((2, 3, 5), (1 / 13, 0.3, 1 / 7)),
+          ((33, 7, 9), (1 / 33, 1 / 33, 1 / 33)), ((5, 6, 130), (0.01, 0.02, 0.03)), ((101, 79, 83), (1 / 101, 1 / 101, 1 / 101)),
+          ((88, 84, 96), (0.125, 0.25, 0.5))]
+
+
+def pair(cfdb, ctx, shape, spacing):
+    ax = [np.arange(n + 1) * h for n, h in zip(shape, spacing)]
+    v = np.stack(np.meshgrid(*ax, indexing="ij"), -1)
+    return (cfdb.Mesh.structured(ctx, *shape, *spacing),
+            cfdb.Mesh.from_vertices(ctx, *shape, *spacing, v, compat_area=True))
+
+
+def same_bits(a, b):
+    t = torch.int32 if a.dtype == torch.float32 else torch.int64
+    return torch.equal(a.view(t), b.view(t))
+
+
+def field(n, dtype, seed, scale=1.0):
+    return torch.as_tensor(scale * np.random.default_rng(seed).standard_normal(n), dtype=dtype, device=DEV)
+
+
+@pytest.mark.parametrize("shape,spacing", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_operators_equal_the_face_arrays(cfdb, ctx, shape, spacing, dtype):
+    m, a = pair(cfdb, ctx, shape, spacing)
+    phi = field(m.n, dtype, 1)
+    for op in ("grad", "lapl", "stab"):
+        for mask in (7, 1, 2, 4, 6, 0):
+            got, ref = (getattr(ctx, op)(k, phi, mask=mask) for k in (m, a))
+            assert same_bits(got, ref), (op, mask)
+    out = [torch.empty_like(phi) for _ in range(2)]
+    for k, o in zip((m, a), out):
+        ctx.heat_step(k, phi, o, 0.7, 1e-5, path=cfdb.PLAIN)
+    assert same_bits(*out)
+
+
+@pytest.mark.parametrize("shape,spacing", [((9, 8, 11), (0.1, 0.1, 0.1)), ((101, 79, 83), (1 / 101, 1 / 101, 1 / 101))])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_operators_on_values_that_are_not_finite(cfdb, ctx, shape, spacing, dtype):
+    m, a = pair(cfdb, ctx, shape, spacing)
+    top = torch.finfo(dtype).max
+    for value in (float("inf"), float("nan"), -float("inf"), top, -0.6 * top):
+        phi = field(m.n, dtype, 2)
+        for i in (0, m.n // 2 + 3, m.n - 1):
+            phi[i] = value
+        for op in ("grad", "lapl", "stab"):
+            for mask in (7, 2, 0):
+                got, ref = (getattr(ctx, op)(k, phi, mask=mask) for k in (m, a))
+                assert torch.equal(torch.isnan(got), torch.isnan(ref)), (op, mask, value)
+                assert torch.equal(torch.nan_to_num(got, nan=0.0), torch.nan_to_num(ref, nan=0.0)), (op, mask, value)
