@@ -349,6 +349,150 @@ __global__ void __launch_bounds__(kThreads) box_stab_k(Box<R> g, const R* __rest
   }
 }
 
+// ---- the acoustic step (wave_plain_k) --------------------------------------------
+
+template <class R> struct WaveArgs {
+  const R* q;
+  R* qn;
+  const R* c;  // sound speed field, or null: cconst
+  R cconst, dt;
+  int mode;
+  R limit;     // magnitudes that overflow in no sum of two
+};
+
+// One face of slot F between the cell P = (p, u, v, w) and its neighbour N:
+// wave_plain_k's flux with the normal S e_D, times the area, added to acc.
+template <int F, class R>
+__device__ __forceinline__ void wave_face(const R P[4], const R N[4], R c2, R hc, R A, R acc[4]) {
+  constexpr int D = 2 - F / 2;
+  constexpr bool plus = F & 1;
+  const R uP = plus ? P[1 + D] : -P[1 + D], uN = plus ? N[1 + D] : -N[1 + D];
+  const R fp = c2 * (R(0.5) * (uP + uN)) - hc * (N[0] - P[0]);
+  const R pm = R(0.5) * (P[0] + N[0]);
+  acc[0] = acc[0] + fp * A;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const R diff = hc * (N[1 + e] - P[1 + e]);
+    const R fu = e == D ? (plus ? pm : -pm) - diff : -diff;
+    acc[1 + e] = acc[1 + e] + fu * A;
+  }
+}
+
+// The array form of one cell, every product by a normal's zero included.
+template <class R> __device__ __noinline__ void wave_full(const Box<R>& g, const WaveArgs<R>& a, int x, int y, int z) {
+  const Cell c{x, y, z};
+  const int64_t i = id_of(g, c), n = int64_t(g.nx) * g.plane;
+  const R cP = a.c ? a.c[i] : a.cconst, c2 = cP * cP;
+  const R pP = a.q[i], uP = a.q[n + i], vP = a.q[2 * n + i], wP = a.q[3 * n + i];
+  R ap = R(0), au = R(0), av = R(0), aw = R(0);
+  for (int f = 0; f < 6; ++f) {
+    const R nx = outward<R>(f, 0), ny = outward<R>(f, 1), nz = outward<R>(f, 2);
+    const R A = area_of(g, c, f);
+    const R unP = (uP * nx + vP * ny) + wP * nz;
+    const int64_t j = id_of(g, beyond(g, c, f));
+    R pN, uN, vN, wN, cN;
+    if (j != i) {
+      pN = a.q[j]; uN = a.q[n + j]; vN = a.q[2 * n + j]; wN = a.q[3 * n + j];
+      cN = a.c ? a.c[j] : a.cconst;
+    } else {
+      const R two_un = R(2) * unP;
+      pN = pP; uN = uP - two_un * nx; vN = vP - two_un * ny; wN = wP - two_un * nz; cN = cP;
+    }
+    const R unN = (uN * nx + vN * ny) + wN * nz;
+    const R cfc = a.mode == 0 ? fmax(cP, cN) : R(0.5) * (cP + cN);
+    const R hc = R(0.5) * cfc;
+    const R pm = R(0.5) * (pP + pN);
+    ap = ap + (c2 * (R(0.5) * (unP + unN)) - hc * (pN - pP)) * A;
+    au = au + (pm * nx - hc * (uN - uP)) * A;
+    av = av + (pm * ny - hc * (vN - vP)) * A;
+    aw = aw + (pm * nz - hc * (wN - wP)) * A;
+  }
+  const R V = g.volume(i);
+  a.qn[i] = a.dt * (-(ap / V)) + pP;
+  a.qn[n + i] = a.dt * (-(au / V)) + uP;
+  a.qn[2 * n + i] = a.dt * (-(av / V)) + vP;
+  a.qn[3 * n + i] = a.dt * (-(aw / V)) + wP;
+}
+
+// A wall neighbour is the cell with its wall-normal velocity negated: with
+// the normal S e_D, u - (2 (S u)) S = -u exactly.
+template <class R, int NX, bool CF>
+__global__ void __launch_bounds__(kThreads) box_wave_k(Box<R> g, WaveArgs<R> a) {
+  const Where w = where<NX>(g);
+  if (!w.ok) return;
+  const int64_t pl = g.plane, n = int64_t(g.nx) * pl;
+  const int y = w.y, z = w.z;
+  const bool ylo = y == 0, yhi = y == g.ny - 1, zlo = z == 0, zhi = z == g.nz - 1;
+  const int dym = ylo ? 0 : -g.nz, dyp = yhi ? 0 : g.nz, dzm = zlo ? 0 : -1, dzp = zhi ? 0 : 1;
+  const R* const q = a.q + w.i0;
+  const R* const cf = CF ? a.c + w.i0 : nullptr;
+  const double hy = g.hy[y], hz = g.hz[z];
+  const R Ax = R(hy * hz);
+  R prv[4], cur[4], nxt[4];
+#pragma unroll
+  for (int f = 0; f < 4; ++f) cur[f] = q[f * n];
+#pragma unroll
+  for (int f = 0; f < 4; ++f) prv[f] = q[f * n - (w.x0 > 0 ? pl : 0)];
+  if (w.x0 == 0) prv[1] = -prv[1];
+#pragma unroll
+  for (int j = 0; j < NX; ++j) {
+    const int x = w.x0 + j;
+    if (x >= g.nx) return;
+    const bool xhi = x == g.nx - 1;
+    const R* const b = q + j * pl;
+    const int64_t dxp = xhi ? 0 : pl;
+    R ym[4], yp[4], zm[4], zp[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      nxt[f] = b[f * n + dxp];
+      ym[f] = b[f * n + dym];
+      yp[f] = b[f * n + dyp];
+      zm[f] = b[f * n + dzm];
+      zp[f] = b[f * n + dzp];
+    }
+    const R V = g.volume(w.i0 + j * pl);
+    if (xhi) nxt[1] = -nxt[1];
+    if (ylo) ym[2] = -ym[2];
+    if (yhi) yp[2] = -yp[2];
+    if (zlo) zm[3] = -zm[3];
+    if (zhi) zp[3] = -zp[3];
+    bool fine = true;
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+      fine = fine && fabs(cur[f]) <= a.limit && fabs(prv[f]) <= a.limit && fabs(nxt[f]) <= a.limit &&
+             fabs(ym[f]) <= a.limit && fabs(yp[f]) <= a.limit && fabs(zm[f]) <= a.limit && fabs(zp[f]) <= a.limit;
+    if (fine) {
+      const R cP = CF ? cf[j * pl] : a.cconst;
+      const R c2 = cP * cP;
+      auto half_speed = [&](int64_t off) {
+        if (!CF) return R(0.5) * (a.mode == 0 ? cP : R(0.5) * (cP + cP));
+        const R cN = cf[j * pl + off];
+        return R(0.5) * (a.mode == 0 ? fmax(cP, cN) : R(0.5) * (cP + cN));
+      };
+      const double hx = g.hx[x];
+      const R Ay = R(hx * hz), Az = R(hx * hy);
+      R acc[4] = {R(0), R(0), R(0), R(0)};
+      wave_face<0>(cur, zm, c2, half_speed(dzm), Az, acc);
+      wave_face<1>(cur, zp, c2, half_speed(dzp), Az, acc);
+      wave_face<2>(cur, ym, c2, half_speed(dym), Ay, acc);
+      wave_face<3>(cur, yp, c2, half_speed(dyp), Ay, acc);
+      wave_face<4>(cur, prv, c2, half_speed(x > 0 ? -pl : 0), Ax, acc);
+      wave_face<5>(cur, nxt, c2, half_speed(dxp), Ax, acc);
+      R* const o = a.qn + w.i0 + j * pl;
+#pragma unroll
+      for (int f = 0; f < 4; ++f) o[f * n] = a.dt * (-(acc[f] / V)) + cur[f];
+    } else {
+      wave_full(g, a, x, y, z);
+    }
+    // the next plane: an x wall's ghost is never carried on (xhi ends the column)
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      prv[f] = cur[f];
+      cur[f] = nxt[f];
+    }
+  }
+}
+
 // ---- tables -------------------------------------------------------------------
 
 // Volume of a cell, the sum of cell_geometry() (geometry_cell.hpp): the face
@@ -542,5 +686,17 @@ int box_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out,
     auto kern = one ? box_stab_k<R, 1> : box_stab_k<R, NX>;
     const int nx = one ? 1 : NX;
     kern<<<grid_of(m, nx), kThreads, 0, ctx->stream>>>(box_of<R>(m, nx), static_cast<const R*>(phi), static_cast<R*>(out), mask);
+  });
+}
+
+int box_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* qn, const void* c, double cconst, int mode,
+                  double dt) {
+  return with_form(ctx, m, dtype, [&](auto r, bool one) {
+    using R = decltype(r);
+    WaveArgs<R> a{static_cast<const R*>(q), static_cast<R*>(qn), static_cast<const R*>(c), R(cconst), R(dt), mode,
+                  std::numeric_limits<R>::max() / R(16)};
+    auto kern = c ? (one ? box_wave_k<R, 1, true> : box_wave_k<R, 4, true>) : (one ? box_wave_k<R, 1, false> : box_wave_k<R, 4, false>);
+    const int nx = one ? 1 : 4;
+    kern<<<grid_of(m, nx), kThreads, 0, ctx->stream>>>(box_of<R>(m, nx), a);
   });
 }

@@ -767,6 +767,9 @@ extern "C" int cfdb_total_fp64(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const voi
 
 int plain_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* qn, const void* c, double cconst,
                     int mode, double dt) {
+  bool box = false;
+  if (int rc = cfdb_mesh_need_box(m, dtype, &box)) return rc;
+  if (box) return box_wave_step(ctx, m, dtype, q, qn, c, cconst, mode, dt);
   if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
   DISPATCH(dtype, R, wave_plain_k<R><<<grid_for(ctx, m->n, kThreads), kThreads, 0, ctx->stream>>>(
                          plain_args<R>(m, dtype), (const R*)q, (R*)qn, (const R*)c, R(cconst), mode, R(dt)));

@@ -47,6 +47,13 @@ def test_operators_equal_the_face_arrays(cfdb, ctx, shape, spacing, dtype):
     for k, o in zip((m, a), out):
         ctx.heat_step(k, phi, o, 0.7, 1e-5, path=cfdb.PLAIN)
     assert same_bits(*out)
+    q = field(4 * m.n, dtype, 3)
+    cf = torch.exp(field(m.n, dtype, 4, 0.1))
+    out = [torch.empty_like(q) for _ in range(2)]
+    for c, mode in ((None, 0), (None, 1), (cf, 0), (cf, 1)):
+        for k, o in zip((m, a), out):
+            ctx.wave_step(k, q, o, 1e-4, c=c, c_const=0.9, speed_mode=mode, path=cfdb.PLAIN)
+        assert same_bits(*out), mode
 
 
 @pytest.mark.parametrize("shape,spacing", [((9, 8, 11), (0.1, 0.1, 0.1)), ((101, 79, 83), (1 / 101, 1 / 101, 1 / 101))])
@@ -63,3 +70,11 @@ def test_operators_on_values_that_are_not_finite(cfdb, ctx, shape, spacing, dtyp
                 got, ref = (getattr(ctx, op)(k, phi, mask=mask) for k in (m, a))
                 assert torch.equal(torch.isnan(got), torch.isnan(ref)), (op, mask, value)
                 assert torch.equal(torch.nan_to_num(got, nan=0.0), torch.nan_to_num(ref, nan=0.0)), (op, mask, value)
+        q = field(4 * m.n, dtype, 5)
+        for i in (0, 2 * m.n - 1, 2 * m.n + m.n // 2, 4 * m.n - 40):
+            q[i] = value
+        out = [torch.empty_like(q) for _ in range(2)]
+        for k, o in zip((m, a), out):
+            ctx.wave_step(k, q, o, 1e-4, c_const=0.9, path=cfdb.PLAIN)
+        assert torch.equal(torch.isnan(out[0]), torch.isnan(out[1])), value
+        assert torch.equal(torch.nan_to_num(out[0], nan=0.0), torch.nan_to_num(out[1], nan=0.0)), value
