@@ -22,10 +22,19 @@
 // where more than one stage is chained, evaluate the cell by the full sums:
 // *_full below).
 //
-// Layout: a thread owns one (y, z) column and NX consecutive x planes, all of
-// whose loads are issued before the first result is needed; threads of a warp
-// are consecutive in z, x neighbours come from registers and y and z
-// neighbours through L1.  Compiled with --fmad=false like plain_ops.cu.
+// Layout: what bounds these kernels once the geometry is gone is instruction
+// issue, so every face is evaluated once.  A thread owns NY consecutive rows at
+// one z and marches a chunk of x planes: the face above a plane is carried in
+// registers as the next plane's face below, the faces between a thread's rows
+// are shared by them, and the z neighbours are the adjacent lanes of the warp.
+// The lanes run along z across row groups (32 consecutive (group, z) pairs,
+// the outer HZ on each side computing for their neighbours only), so rows of
+// any length waste no lanes; a lane at a z wall uses no neighbour.  Warps never
+// wait for one another.  (One cell per thread with neighbours through L1, the
+// first form, took 45, 50 and 262 us for the gradient, Laplacian and
+// stabilisation at 200^3 FP32, 139 and 565 instructions per cell.)
+// Compiled with --fmad=false like plain_ops.cu.
+#include <algorithm>
 #include <cmath>
 #include <limits>
 
@@ -39,144 +48,21 @@ constexpr int kThreads = 256;
 
 template <class R> struct Box {
   int nx, ny, nz;
-  unsigned plane, chunks;   // ny nz; x chunks of NX planes
+  unsigned plane;           // ny nz
+  int groups;               // row groups of NY rows
+  unsigned tiles, chunks;   // warps across (group, z) and along x
   const double *hx, *hy, *hz;   // edge lengths
   const R *ax, *ay, *az;        // alpha of the face below cell i (entry i), 0 .. n
   const R *lmx, *lpx, *lmy, *lpy, *lmz, *lpz;  // |x_f - x_P| of the - and + faces
   const R* vol;                 // cell volumes, or null: v for every cell
-  R v;
+  R v, rv;                      // rv = 1 / v
   R limit;                      // magnitudes up to this overflow in no intermediate
+  // one value per direction for the whole mesh (UNI kernels)
+  R A[3], al[3], lm[3], lp[3];
   __device__ R volume(int64_t i) const { return vol ? vol[i] : v; }
 };
 
 template <class R> __device__ __forceinline__ bool finite(R v) { return fabs(v) <= std::numeric_limits<R>::max(); }
-
-// The column and the x chunk of a thread.
-struct Where {
-  int x0, y, z;
-  int64_t i0;      // cell (x0, y, z)
-  bool ok;
-};
-template <int NX, class R> __device__ __forceinline__ Where where(const Box<R>& g) {
-  const unsigned t = blockIdx.x * kThreads + threadIdx.x;
-  const unsigned chunk = t / g.plane, col = t - chunk * g.plane;
-  Where w;
-  w.ok = chunk < g.chunks;
-  w.x0 = int(chunk) * NX;
-  w.y = int(col / unsigned(g.nz));
-  w.z = int(col) - w.y * g.nz;
-  w.i0 = int64_t(w.x0) * g.plane + col;
-  return w;
-}
-
-// GradVar (grad_k): sum over the masked directions of (sum_f itp n_d A) / V.
-template <class R, int NX>
-__global__ void __launch_bounds__(kThreads) box_grad_k(Box<R> g, const R* __restrict__ phi, R* __restrict__ out, int mask) {
-  const Where w = where<NX>(g);
-  if (!w.ok) return;
-  const R* p = phi + w.i0;
-  const int64_t pl = g.plane;
-  const int dym = w.y > 0 ? -g.nz : 0, dyp = w.y < g.ny - 1 ? g.nz : 0;
-  const int dzm = w.z > 0 ? -1 : 0, dzp = w.z < g.nz - 1 ? 1 : 0;
-  R c[NX + 2], ym[NX], yp[NX], zm[NX], zp[NX], V[NX];
-  int xs[NX];
-  c[0] = w.x0 > 0 ? p[-pl] : p[0];
-#pragma unroll
-  for (int j = 0; j < NX; ++j) {
-    xs[j] = min(w.x0 + j, g.nx - 1);
-    const R* q = p + (xs[j] - w.x0) * pl;
-    c[j + 1] = q[0];
-    ym[j] = q[dym];
-    yp[j] = q[dyp];
-    zm[j] = q[dzm];
-    zp[j] = q[dzp];
-    V[j] = g.volume(w.i0 + (xs[j] - w.x0) * pl);
-  }
-  c[NX + 1] = p[(min(w.x0 + NX, g.nx - 1) - w.x0) * pl];
-  const double hy = g.hy[w.y], hz = g.hz[w.z];
-  const R Ax = R(hy * hz);
-#pragma unroll
-  for (int j = 0; j < NX; ++j) {
-    if (w.x0 + j >= g.nx) return;
-    const double hx = g.hx[xs[j]];
-    const R Ay = R(hx * hz), Az = R(hx * hy);
-    const R P = c[j + 1];
-    const R itp[6] = {(P + zm[j]) * R(0.5), (P + zp[j]) * R(0.5), (P + ym[j]) * R(0.5),
-                      (P + yp[j]) * R(0.5), (P + c[j]) * R(0.5),  (P + c[j + 2]) * R(0.5)};
-    const R A[3] = {Ax, Ay, Az};
-    R res = R(0);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      if (!(mask & (1 << d))) continue;
-      const int f = 4 - 2 * d;
-      const R acc = (R(0) + (-itp[f]) * A[d]) + itp[f + 1] * A[d];
-      res = res + acc / V[j];
-    }
-    const R sum = ((itp[0] + itp[1]) + (itp[2] + itp[3])) + (itp[4] + itp[5]);
-    if (!finite(sum)) {  // a face value times the zero components of its normal, in the other directions' sums
-      for (int f = 0; f < 6; ++f)
-        if (!finite(itp[f]) && (mask & ~(1 << (2 - f / 2)))) res = sum - sum;  // NaN
-    }
-    out[w.i0 + j * pl] = res;
-  }
-}
-
-// Grad2Var (lapl_k): sum over the masked directions of (sum_f (sn_f n_d) A) / V,
-// sn_f = (phi_N - phi_P) alpha_f, with the unsigned normal +e_d on both faces.
-// HEAT: the heat step dt (k L) + phi of heat_update_k in the same pass.
-template <class R, int NX, bool HEAT = false>
-__global__ void __launch_bounds__(kThreads) box_lapl_k(Box<R> g, const R* __restrict__ phi, R* __restrict__ out, int mask,
-                                                       R k = R(0), R dt = R(0)) {
-  const Where w = where<NX>(g);
-  if (!w.ok) return;
-  const R* p = phi + w.i0;
-  const int64_t pl = g.plane;
-  const int dym = w.y > 0 ? -g.nz : 0, dyp = w.y < g.ny - 1 ? g.nz : 0;
-  const int dzm = w.z > 0 ? -1 : 0, dzp = w.z < g.nz - 1 ? 1 : 0;
-  R c[NX + 2], ym[NX], yp[NX], zm[NX], zp[NX], V[NX];
-  int xs[NX];
-  c[0] = w.x0 > 0 ? p[-pl] : p[0];
-#pragma unroll
-  for (int j = 0; j < NX; ++j) {
-    xs[j] = min(w.x0 + j, g.nx - 1);
-    const R* q = p + (xs[j] - w.x0) * pl;
-    c[j + 1] = q[0];
-    ym[j] = q[dym];
-    yp[j] = q[dyp];
-    zm[j] = q[dzm];
-    zp[j] = q[dzp];
-    V[j] = g.volume(w.i0 + (xs[j] - w.x0) * pl);
-  }
-  c[NX + 1] = p[(min(w.x0 + NX, g.nx - 1) - w.x0) * pl];
-  const double hy = g.hy[w.y], hz = g.hz[w.z];
-  const R Ax = R(hy * hz);
-  const R aym = g.ay[w.y], ayp = g.ay[w.y + 1], azm = g.az[w.z], azp = g.az[w.z + 1];
-#pragma unroll
-  for (int j = 0; j < NX; ++j) {
-    if (w.x0 + j >= g.nx) return;
-    const double hx = g.hx[xs[j]];
-    const R Ay = R(hx * hz), Az = R(hx * hy);
-    const R P = c[j + 1];
-    const R sn[6] = {(zm[j] - P) * azm,           (zp[j] - P) * azp, (ym[j] - P) * aym,
-                     (yp[j] - P) * ayp,           (c[j] - P) * g.ax[xs[j]], (c[j + 2] - P) * g.ax[xs[j] + 1]};
-    const R A[3] = {Ax, Ay, Az};
-    R res = R(0);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      if (!(mask & (1 << d))) continue;
-      const int f = 4 - 2 * d;
-      const R acc = (R(0) + sn[f] * A[d]) + sn[f + 1] * A[d];
-      res = res + acc / V[j];
-    }
-    const R sum = ((sn[0] + sn[1]) + (sn[2] + sn[3])) + (sn[4] + sn[5]);
-    if (!finite(sum)) {  // a face value times the zero components of its normal, in the other directions' sums
-      for (int f = 0; f < 6; ++f)
-        if (!finite(sn[f]) && (mask & ~(1 << (2 - f / 2)))) res = sum - sum;  // NaN
-    }
-    if constexpr (HEAT) res = dt * (k * res) + P;
-    out[w.i0 + j * pl] = res;
-  }
-}
 
 // ---- the array form of one cell, for operands that are not finite ------------
 
@@ -242,110 +128,336 @@ template <class R> __device__ __noinline__ R stab_full(const Box<R>& g, const R*
   return res;
 }
 
-// One direction of StabVar from the five values along it: b2 b1 P a1 a2 (below
-// and above; beyond a wall the wall cell repeats), the face area, the volumes
-// of the three cells and the face distances (own - and +, the lower
-// neighbour's + and the upper neighbour's -).
-template <class R>
-__device__ __forceinline__ R grad1(R lo, R P, R hi, R A, R V) {
-  return ((R(0) + (-((P + lo) * R(0.5))) * A) + ((P + hi) * R(0.5)) * A) / V;
+template <class R> __device__ __noinline__ R grad_sum_full(const Box<R>& g, const R* phi, int x, int y, int z, int mask) {
+  R res = R(0);
+  for (int d = 0; d < 3; ++d)
+    if (mask & (1 << d)) res = res + grad_full(g, phi, Cell{x, y, z}, d);
+  return res;
 }
-template <class R>
-__device__ __forceinline__ R stab1(R b1, R P, R a1, R gP, R gB, R gA, R A, R V, R lm, R lp, R lpB, R lmA) {
-  const R um = P + -(lm * gP), up = P + lp * gP;
-  const R cm = b1 + lpB * gB, cp = a1 + -(lmA * gA);
-  const R sm = R(0.5) * (um - cm), sp = R(0.5) * (up - cp);
-  return ((R(0) + sm * A) + sp * A) / V;
+
+template <class R> __device__ __noinline__ R lapl_full(const Box<R>& g, const R* phi, int x, int y, int z, int mask) {
+  const Cell c{x, y, z};
+  const int64_t i = id_of(g, c);
+  const R alpha[6] = {g.az[z], g.az[z + 1], g.ay[y], g.ay[y + 1], g.ax[x], g.ax[x + 1]};
+  R res = R(0);
+  for (int d = 0; d < 3; ++d) {
+    if (!(mask & (1 << d))) continue;
+    R acc = R(0);
+    for (int f = 0; f < 6; ++f) {
+      const R sn = (phi[id_of(g, beyond(g, c, f))] - phi[i]) * alpha[f];
+      acc = acc + sn * fabs(outward<R>(f, d)) * area_of(g, c, f);
+    }
+    res = res + acc / g.volume(i);
+  }
+  return res;
+}
+
+// Division by a cell volume. The volume divides several sums of a cell, so its
+// reciprocal r = fl(1 / v) is formed once and each quotient takes a product and
+// two corrections by the exact remainder: with r correctly rounded and the
+// quotient within one unit in the last place, fl(q + fl(a - q v) r) is the
+// correctly rounded quotient (P. Markstein, IBM J. Res. Dev. 34(1), 1990).  That
+// needs remainders that do not underflow: a smaller nonzero dividend is divided
+// directly, and volumes are in [2^-80, 2^24] (other meshes keep the array
+// kernels).  A result that is not finite is computed again by the callers.
+// (Three IEEE divisions had been about 60 of the gradient's 102 instructions
+// per cell.)
+template <class R> struct Volume {
+  R v, r;
+  __device__ __forceinline__ R quot(R a) const {
+    R q = a * r;
+    q = fma(fma(-q, v, a), r, q);
+    return fma(fma(-q, v, a), r, q);
+  }
+  // a[d] = fl(a[d] / v) for N sums of one cell, one branch for all of them
+  template <int N> __device__ __forceinline__ void divide(R a[N]) const {
+    R least = fabs(a[0]);
+#pragma unroll
+    for (int d = 1; d < N; ++d) least = fmin(least, fabs(a[d]));
+    bool direct = false;
+    if (least < (sizeof(R) == 8 ? R(1e-288) : R(1e-30))) {  // zero divides exactly
+#pragma unroll
+      for (int d = 0; d < N; ++d) direct = direct || (fabs(a[d]) < (sizeof(R) == 8 ? R(1e-288) : R(1e-30)) && a[d] != R(0));
+    }
+    if (direct) {
+#pragma unroll
+      for (int d = 0; d < N; ++d) a[d] = a[d] / v;
+    } else {
+#pragma unroll
+      for (int d = 0; d < N; ++d) a[d] = quot(a[d]);
+    }
+  }
+};
+
+// ---- the march ------------------------------------------------------------------
+
+constexpr unsigned kWarp = 0xffffffffu;
+
+// A thread's place: NY rows from y0 at one z, planes [x0, x1).  off[HY + r] is
+// row y0 + r within a plane, r = -HY .. NY + HY - 1, walls repeated (a wall
+// face's neighbour is the cell itself, and so are rows beyond the last).
+template <int NY, int HY, int HZ> struct March {
+  int y0, z, x0, x1;
+  int off[NY + 2 * HY];
+  bool out, zlo, zhi;
+  template <class R> __device__ __forceinline__ bool start(const Box<R>& g) {
+    const unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= g.tiles * g.chunks) return false;  // whole warps
+    const unsigned chunk = w / g.tiles, tile = w - chunk * g.tiles;
+    const int S = g.groups * g.nz;
+    int s = int(tile) * (32 - 2 * HZ) + int(lane) - HZ;
+    out = int(lane) >= HZ && int(lane) < 32 - HZ && s < S;
+    s = min(max(s, 0), S - 1);
+    const int grp = s / g.nz;
+    z = s - grp * g.nz;
+    y0 = grp * NY;
+#pragma unroll
+    for (int r = -HY; r < NY + HY; ++r) off[r + HY] = min(max(y0 + r, 0), g.ny - 1) * g.nz + z;
+    x0 = int(int64_t(chunk) * g.nx / g.chunks);
+    x1 = int(int64_t(chunk + 1) * g.nx / g.chunks);
+    zlo = z == 0;
+    zhi = z == g.nz - 1;
+    return true;
+  }
+};
+
+enum { OP_GRAD = 0, OP_LAPL = 1, OP_HEAT = 2 };
+
+// GradVar (grad_k): sum over the masked directions of (sum_f itp_f n_d A) / V,
+// itp = (phi_P + phi_N) / 2, and Grad2Var (lapl_k): the same with
+// sn_f = (phi_N - phi_P) alpha_f and the unsigned normal +e_d on both faces.
+// With F the face value between the lower and the upper cell times the area,
+// both sum to ((0 - F_lower) + F_upper) / V per direction: the lower face enters
+// with the opposite sign, which rounds alike.  HEAT: the update dt (k L) + phi
+// of heat_update_k in the same pass.  UNI: one area, alpha and volume for the
+// whole mesh.  A result that is not finite (every face value reaches it: FULL
+// sums all three directions, and the others are summed to look at) is computed
+// again by the full sums.
+// 200^3 FP32 (64 MB): floor 10 us.
+template <class R, int OP, int NY, bool UNI, bool FULL>
+__global__ void __launch_bounds__(kThreads) box_sum_k(const __grid_constant__ Box<R> g, const R* __restrict__ phi, R* __restrict__ out, int mask_,
+                                                      R k, R dt) {
+  March<NY, 1, 1> w;
+  if (!w.start(g)) return;
+  const int mask = FULL ? 7 : mask_;
+  const int64_t pl = g.plane;
+  auto face = [](R lo, R hi, R alpha, R A) {
+    if constexpr (OP == OP_GRAD) return ((lo + hi) * R(0.5)) * A;
+    else return ((hi - lo) * alpha) * A;
+  };
+  R Ax[NY], ayv[NY + 1];
+  double hy[NY];
+  const double hz = UNI ? 0.0 : g.hz[w.z];
+#pragma unroll
+  for (int r = 0; r < NY; ++r) {
+    const int y = min(w.y0 + r, g.ny - 1);
+    hy[r] = UNI ? 0.0 : g.hy[y];
+    Ax[r] = UNI ? g.A[0] : R(hy[r] * hz);
+  }
+#pragma unroll
+  for (int r = 0; r <= NY; ++r) ayv[r] = OP == OP_GRAD ? R(0) : UNI ? g.al[1] : g.ay[min(w.y0 + r, g.ny)];
+  const R azl = OP == OP_GRAD ? R(0) : UNI ? g.al[2] : g.az[w.z], azh = OP == OP_GRAD ? R(0) : UNI ? g.al[2] : g.az[w.z + 1];
+  const R* q = phi + w.x0 * pl;
+  R cur[NY], nxt[NY], fx[NY];
+  {
+    const int64_t back = w.x0 > 0 ? pl : 0;
+    const R alpha = OP == OP_GRAD ? R(0) : UNI ? g.al[0] : g.ax[w.x0];
+#pragma unroll
+    for (int r = 0; r < NY; ++r) {
+      cur[r] = q[w.off[1 + r]];
+      fx[r] = face(q[w.off[1 + r] - back], cur[r], alpha, Ax[r]);
+    }
+  }
+  for (int x = w.x0; x < w.x1; ++x, q += pl) {
+    const R* qn = q + (x < g.nx - 1 ? pl : 0);
+    const R lo = q[w.off[0]], hi = q[w.off[NY + 1]];
+#pragma unroll
+    for (int r = 0; r < NY; ++r) nxt[r] = qn[w.off[1 + r]];
+    const double hx = UNI ? 0.0 : g.hx[x];
+    const R Ay = UNI ? g.A[1] : R(hx * hz);
+    const R axv = OP == OP_GRAD ? R(0) : UNI ? g.al[0] : g.ax[x + 1];
+    R fy = face(lo, cur[0], ayv[0], Ay);
+#pragma unroll
+    for (int r = 0; r < NY; ++r) {
+      const R P = cur[r];
+      const int64_t i = x * pl + w.off[1 + r];
+      const R vol = UNI ? g.v : g.volume(i);
+      const Volume<R> V{vol, UNI ? g.rv : R(1) / vol};
+      const R Az = UNI ? g.A[2] : R(hx * hy[r]);
+      R zm = __shfl_up_sync(kWarp, P, 1), zp = __shfl_down_sync(kWarp, P, 1);
+      zm = w.zlo ? P : zm;
+      zp = w.zhi ? P : zp;
+      const R fxh = face(P, nxt[r], axv, Ax[r]);
+      const R fyh = face(P, r + 1 < NY ? cur[r + 1] : hi, ayv[r + 1], Ay);
+      R acc[3] = {(R(0) - fx[r]) + fxh, (R(0) - fy) + fyh, (R(0) - face(zm, P, azl, Az)) + face(P, zp, azh, Az)};
+      const R all = FULL ? R(0) : (acc[0] + acc[1]) + acc[2];
+      V.template divide<3>(acc);
+      fx[r] = fxh;
+      fy = fyh;
+      R res = R(0);
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (mask & (1 << d)) res = res + acc[d];
+      const bool rows = w.y0 + r < g.ny;
+      if (w.out && rows) {
+        if (!finite(res) || (!FULL && !finite(all)))
+          res = OP == OP_GRAD ? grad_sum_full(g, phi, x, w.y0 + r, w.z, mask) : lapl_full(g, phi, x, w.y0 + r, w.z, mask);
+        out[i] = OP == OP_HEAT ? dt * (k * res) + P : res;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < NY; ++r) cur[r] = nxt[r];
+  }
 }
 
 // StabVar, both stages at once (stab1_k + stab2_k, whose 18 values per cell
-// between the stages made 3.5 GB of traffic at 200^3 FP32): along each
-// direction the sum needs the gradients of the cell and of its two
-// neighbours, which five values give.
-template <class R, int NX>
-__global__ void __launch_bounds__(kThreads) box_stab_k(Box<R> g, const R* __restrict__ phi, R* __restrict__ out, int mask) {
-  const Where w = where<NX>(g);
-  if (!w.ok) return;
-  const R* p = phi + w.i0;
+// between the stages made 3.5 GB of traffic at 200^3 FP32).  Along a direction,
+// with g the cell gradient and a cell's face values up = phi + len g on its
+// upper face and um = phi - len g on its lower, a face between B (below) and
+// A (above) contributes E = (0.5 (up_B - um_A)) A: ((0 - E_lower) + E_upper) / V.
+// A wall cell faces itself (E from its own up and um).
+// Planes x + 1 and x + 2 are in registers while plane x is finished (its x
+// neighbours' gradients need them).  `fine` is kept per plane and warp: all
+// values of the rows and lanes that the array form would have touched are small
+// enough that no intermediate overflows; a plane within two of one that is
+// not is computed by the full sums.
+template <class R, int NY, bool UNI, bool FULL>
+__global__ void __launch_bounds__(128) box_stab_k(const __grid_constant__ Box<R> g, const R* __restrict__ phi, R* __restrict__ out, int mask_) {
+  constexpr int NR = NY + 4;  // rows -2 .. NY + 1
+  March<NY, 2, 2> w;
+  if (!w.start(g)) return;
+  const int mask = FULL ? 7 : mask_;
   const int64_t pl = g.plane;
-  const int y = w.y, z = w.z;
-  const int dym = y > 0 ? -g.nz : 0, dyp = y < g.ny - 1 ? g.nz : 0;
-  const int dym2 = y > 1 ? -2 * g.nz : dym, dyp2 = y < g.ny - 2 ? 2 * g.nz : dyp;
-  const int dzm = z > 0 ? -1 : 0, dzp = z < g.nz - 1 ? 1 : 0;
-  const int dzm2 = z > 1 ? -2 : dzm, dzp2 = z < g.nz - 2 ? 2 : dzp;
-  auto at = [&](int k) { return min(max(w.x0 + k, 0), g.nx - 1) - w.x0; };  // plane k of the chunk, walls repeated
-  // values of planes -2 .. NX+1 of the column and -1 .. NX of its four
-  // neighbours; `fine`: magnitudes for which no intermediate of the two stages
-  // overflows, over every cell the array form touches
-  R c[NX + 4], ym[NX + 2], yp[NX + 2], zm[NX + 2], zp[NX + 2];
-  R ym2[NX], yp2[NX], zm2[NX], zp2[NX];
-  bool fine = true;
-  auto look = [&](R v) { fine = fine && fabs(v) <= g.limit; };
+  const double hz = UNI ? 0.0 : g.hz[w.z];
+  auto plane = [&](int x) { return phi + int64_t(min(max(x, 0), g.nx - 1)) * pl; };
+  unsigned fine = 0;  // bit k: plane (newest - k) is fine
+  auto load = [&](int x, R v[NR]) {
+    const R* q = plane(x);
+    bool ok = true;
 #pragma unroll
-  for (int k = -2; k < NX + 2; ++k) look(c[k + 2] = p[at(k) * pl]);
+    for (int r = 0; r < NR; ++r) {
+      v[r] = q[w.off[r]];
+      ok = ok && fabs(v[r]) <= g.limit;
+    }
+    fine = fine << 1 | (__all_sync(kWarp, ok) ? 1u : 0u);
+  };
+  auto vol_at = [&](int x, int r) {  // row r of plane x (walls repeated)
+    const R v = UNI ? g.v : g.volume(int64_t(min(max(x, 0), g.nx - 1)) * pl + w.off[r + 2]);
+    return Volume<R>{v, UNI ? g.rv : R(1) / v};
+  };
+  auto over = [](const Volume<R>& V, R a) {
+    V.template divide<1>(&a);
+    return a;
+  };
+  auto mean = [](R a, R b, R A) { return ((a + b) * R(0.5)) * A; };
+  auto edge = [](R up, R um, R A) { return (R(0.5) * (up - um)) * A; };
+  auto row = [&](int r) { return min(max(w.y0 + r, 0), g.ny - 1); };
+  auto len_lo = [&](int d, int i) { return UNI ? g.lm[d] : d == 0 ? g.lmx[i] : d == 1 ? g.lmy[i] : g.lmz[i]; };
+  auto len_hi = [&](int d, int i) { return UNI ? g.lp[d] : d == 0 ? g.lpx[i] : d == 1 ? g.lpy[i] : g.lpz[i]; };
+  R Ax[NY];
 #pragma unroll
-  for (int k = -1; k < NX + 1; ++k) {
-    const R* q = p + at(k) * pl;
-    look(ym[k + 1] = q[dym]);
-    look(yp[k + 1] = q[dyp]);
-    look(zm[k + 1] = q[dzm]);
-    look(zp[k + 1] = q[dzp]);
+  for (int r = 0; r < NY; ++r) Ax[r] = UNI ? g.A[0] : R(g.hy[row(r)] * hz);
+  R cur[NR], n1[NR], n2[NR], fx[NY], gx[NY], ex[NY];  // fx: face (x, x + 1); gx: gradient of plane x; ex: E between x - 1 and x
+  {
+    R b2[NR], b1[NR];
+    load(w.x0 - 2, b2);
+    load(w.x0 - 1, b1);
+    load(w.x0, cur);
+    load(w.x0 + 1, n1);
+#pragma unroll
+    for (int r = 0; r < NY; ++r) {
+      const R flo = mean(b1[r + 2], cur[r + 2], Ax[r]);  // at x = 0 the wall face: b1 repeats cur
+      fx[r] = mean(cur[r + 2], n1[r + 2], Ax[r]);
+      gx[r] = over(vol_at(w.x0, r), (R(0) - flo) + fx[r]);
+      const R um = cur[r + 2] - len_lo(0, w.x0) * gx[r];
+      R up;
+      if (w.x0 > 0) {
+        const R gB = over(vol_at(w.x0 - 1, r), (R(0) - mean(b2[r + 2], b1[r + 2], Ax[r])) + flo);
+        up = b1[r + 2] + len_hi(0, w.x0 - 1) * gB;
+      } else {
+        up = cur[r + 2] + len_hi(0, w.x0) * gx[r];
+      }
+      ex[r] = edge(up, um, Ax[r]);
+    }
   }
+  for (int x = w.x0; x < w.x1; ++x) {
+    load(x + 2, n2);
+    const bool all_fine = (fine & 31u) == 31u;
+    const double hx = UNI ? 0.0 : g.hx[x];
+    const R Ay = UNI ? g.A[1] : R(hx * hz);
+    const bool xhi = x == g.nx - 1;
+    const int xn = min(x + 1, g.nx - 1);
+    // y direction, rolling over the rows: gradient and face values of the row
+    // below the thread's first, then of each row and the one above it
+    R fy = mean(cur[1], cur[2], Ay), upB;
+    {
+      const R gB = over(vol_at(x, -1), (R(0) - mean(cur[0], cur[1], Ay)) + fy);
+      upB = cur[1] + len_hi(1, row(-1)) * gB;
+    }
+    R fyh = mean(cur[2], cur[3], Ay);
+    R gy = over(vol_at(x, 0), (R(0) - fy) + fyh);
 #pragma unroll
-  for (int k = 0; k < NX; ++k) {
-    const R* q = p + at(k) * pl;
-    look(ym2[k] = q[dym2]);
-    look(yp2[k] = q[dyp2]);
-    look(zm2[k] = q[dzm2]);
-    look(zp2[k] = q[dzp2]);
-    look(q[dym + dzm]);
-    look(q[dym + dzp]);
-    look(q[dyp + dzm]);
-    look(q[dyp + dzp]);
-  }
-  const double hy = g.hy[y], hz = g.hz[z];
-  const R A0 = R(hy * hz);
-  // x gradients of planes -1 .. NX (a wall cell's neighbour is itself)
-  R gx[NX + 2];
+    for (int r = 0; r < NY; ++r) {
+      const R P = cur[r + 2];
+      const int y = w.y0 + r;
+      const int64_t i = x * pl + w.off[r + 2];
+      const Volume<R> V = vol_at(x, r);
+      const R Az = UNI ? g.A[2] : R(hx * g.hy[row(r)]);
+      R zm = __shfl_up_sync(kWarp, P, 1), zp = __shfl_down_sync(kWarp, P, 1);
+      zm = w.zlo ? P : zm;
+      zp = w.zhi ? P : zp;
+      // the gradients this row needs next: of its x neighbour above, its y
+      // neighbour above and its own along z
+      const R fx2 = mean(n1[r + 2], n2[r + 2], Ax[r]), fy2 = mean(cur[r + 3], cur[r + 4], Ay);
+      R gr[3] = {(R(0) - fx[r]) + fx2, (R(0) - fyh) + fy2, (R(0) - mean(zm, P, Az)) + mean(P, zp, Az)};
+      if constexpr (UNI) {
+        V.template divide<3>(gr);
+      } else {
+        gr[0] = over(vol_at(x + 1, r), gr[0]);
+        gr[1] = over(vol_at(x, r + 1), gr[1]);
+        gr[2] = over(V, gr[2]);
+      }
+      R s3[3];
+      {  // x
+        const R up = P + len_hi(0, x) * gx[r];
+        const R um1 = xhi ? P - len_lo(0, x) * gx[r] : n1[r + 2] - len_lo(0, xn) * gr[0];
+        const R e = edge(up, um1, Ax[r]);
+        s3[0] = (R(0) - ex[r]) + e;
+        ex[r] = e;
+        fx[r] = fx2;
+        gx[r] = gr[0];
+      }
+      {  // y
+        const R um = P - len_lo(1, row(r)) * gy, up = P + len_hi(1, row(r)) * gy;
+        const R umA = y >= g.ny - 1 ? um : cur[r + 3] - len_lo(1, row(r + 1)) * gr[1];
+        if (y == 0) upB = up;
+        s3[1] = (R(0) - edge(upB, um, Ay)) + edge(up, umA, Ay);
+        upB = up;
+        fyh = fy2;
+        gy = gr[1];
+      }
+      {  // z
+        const R um = P - len_lo(2, w.z) * gr[2], up = P + len_hi(2, w.z) * gr[2];
+        R upb = __shfl_up_sync(kWarp, up, 1), uma = __shfl_down_sync(kWarp, um, 1);
+        upb = w.zlo ? up : upb;
+        uma = w.zhi ? um : uma;
+        s3[2] = (R(0) - edge(upb, um, Az)) + edge(up, uma, Az);
+      }
+      V.template divide<3>(s3);
+      R res = R(0);
 #pragma unroll
-  for (int k = -1; k < NX + 1; ++k) gx[k + 1] = grad1(c[k + 1], c[k + 2], c[k + 3], A0, g.volume(w.i0 + at(k) * pl));
-  const int yb = max(y - 1, 0), ya = min(y + 1, g.ny - 1), zb = max(z - 1, 0), za = min(z + 1, g.nz - 1);
-  const R lmy = g.lmy[y], lpy = g.lpy[y], lpyB = g.lpy[yb], lmyA = g.lmy[ya];
-  const R lmz = g.lmz[z], lpz = g.lpz[z], lpzB = g.lpz[zb], lmzA = g.lmz[za];
+      for (int d = 0; d < 3; ++d)
+        if (mask & (1 << d)) res = res + s3[d];
+      if (w.out && y < g.ny) {
+        if (!all_fine) res = stab_full(g, phi, x, y, w.z, mask);
+        out[i] = res;
+      }
+    }
 #pragma unroll
-  for (int j = 0; j < NX; ++j) {
-    const int x = w.x0 + j;
-    if (x >= g.nx) return;
-    const int64_t i = w.i0 + j * pl;
-    if (!fine) {
-      out[i] = stab_full(g, phi, x, y, z, mask);
-      continue;
+    for (int r = 0; r < NR; ++r) {
+      cur[r] = n1[r];
+      n1[r] = n2[r];
     }
-    const double hx = g.hx[x];
-    const R V = g.volume(i);
-    const R P = c[j + 2];
-    R res = R(0);
-    if (mask & 1) {
-      const R gP = gx[j + 1];
-      const R gB = x == 0 ? gP : gx[j], gA = x == g.nx - 1 ? gP : gx[j + 2];
-      res = res + stab1(c[j + 1], P, c[j + 3], gP, gB, gA, A0, V, g.lmx[x], g.lpx[x], g.lpx[max(x - 1, 0)],
-                        g.lmx[min(x + 1, g.nx - 1)]);
-    }
-    if (mask & 2) {
-      const R A = R(hx * hz);
-      const R gP = grad1(ym[j + 1], P, yp[j + 1], A, V);
-      const R gB = y == 0 ? gP : grad1(ym2[j], ym[j + 1], P, A, g.volume(i + dym));
-      const R gA = y == g.ny - 1 ? gP : grad1(P, yp[j + 1], yp2[j], A, g.volume(i + dyp));
-      res = res + stab1(ym[j + 1], P, yp[j + 1], gP, gB, gA, A, V, lmy, lpy, lpyB, lmyA);
-    }
-    if (mask & 4) {
-      const R A = R(hx * hy);
-      const R gP = grad1(zm[j + 1], P, zp[j + 1], A, V);
-      const R gB = z == 0 ? gP : grad1(zm2[j], zm[j + 1], P, A, g.volume(i + dzm));
-      const R gA = z == g.nz - 1 ? gP : grad1(P, zp[j + 1], zp2[j], A, g.volume(i + dzp));
-      res = res + stab1(zm[j + 1], P, zp[j + 1], gP, gB, gA, A, V, lmz, lpz, lpzB, lmzA);
-    }
-    out[i] = res;
   }
 }
 
@@ -357,26 +469,7 @@ template <class R> struct WaveArgs {
   const R* c;  // sound speed field, or null: cconst
   R cconst, dt;
   int mode;
-  R limit;     // magnitudes that overflow in no sum of two
 };
-
-// One face of slot F between the cell P = (p, u, v, w) and its neighbour N:
-// wave_plain_k's flux with the normal S e_D, times the area, added to acc.
-template <int F, class R>
-__device__ __forceinline__ void wave_face(const R P[4], const R N[4], R c2, R hc, R A, R acc[4]) {
-  constexpr int D = 2 - F / 2;
-  constexpr bool plus = F & 1;
-  const R uP = plus ? P[1 + D] : -P[1 + D], uN = plus ? N[1 + D] : -N[1 + D];
-  const R fp = c2 * (R(0.5) * (uP + uN)) - hc * (N[0] - P[0]);
-  const R pm = R(0.5) * (P[0] + N[0]);
-  acc[0] = acc[0] + fp * A;
-#pragma unroll
-  for (int e = 0; e < 3; ++e) {
-    const R diff = hc * (N[1 + e] - P[1 + e]);
-    const R fu = e == D ? (plus ? pm : -pm) - diff : -diff;
-    acc[1 + e] = acc[1 + e] + fu * A;
-  }
-}
 
 // The array form of one cell, every product by a normal's zero included.
 template <class R> __device__ __noinline__ void wave_full(const Box<R>& g, const WaveArgs<R>& a, int x, int y, int z) {
@@ -414,81 +507,168 @@ template <class R> __device__ __noinline__ void wave_full(const Box<R>& g, const
   a.qn[3 * n + i] = a.dt * (-(aw / V)) + wP;
 }
 
-// A wall neighbour is the cell with its wall-normal velocity negated: with
-// the normal S e_D, u - (2 (S u)) S = -u exactly.
-template <class R, int NX, bool CF>
-__global__ void __launch_bounds__(kThreads) box_wave_k(Box<R> g, WaveArgs<R> a) {
-  const Where w = where<NX>(g);
-  if (!w.ok) return;
+// The flux of wave_plain_k through the face with normal +e_D between L (below)
+// and H (above), times the area, as it enters L's sums with a plus and H's with
+// a minus sign (each rounds like the array form's own evaluation from that side).
+// With a c field the two cells' c^2 differ, so the pressure flux comes as its two
+// parts, fp[0] = (u_L + u_H) / 2 and fp[1] = hc (p_H - p_L).
+template <int D, bool CF, class R>
+__device__ __forceinline__ void wave_face(const R L[4], const R H[4], R c2, R hc, R A, R F[4], R fp[2]) {
+  fp[0] = R(0.5) * (L[1 + D] + H[1 + D]);
+  fp[1] = hc * (H[0] - L[0]);
+  if (!CF) F[0] = (c2 * fp[0] - fp[1]) * A;
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    const R diff = hc * (H[1 + e] - L[1 + e]);
+    F[1 + e] = (e == D ? R(0.5) * (L[0] + H[0]) - diff : -diff) * A;
+  }
+}
+// The cell beyond a wall: the wall-normal velocity reflected, u - (2 u).
+template <int D, class R> __device__ __forceinline__ void wave_ghost(const R P[4], R G[4]) {
+#pragma unroll
+  for (int f = 0; f < 4; ++f) G[f] = P[f];
+  G[1 + D] = P[1 + D] - R(2) * P[1 + D];
+}
+
+// A value that is not finite (or overflows) reaches one of the cell's four
+// results, which are then computed again by the full sums.
+// 100 x 90 x 96 FP64 (55 MB): floor 9 us.
+template <class R, int NY, bool UNI, bool CF>
+__global__ void __launch_bounds__(128) box_wave_k(const __grid_constant__ Box<R> g, const __grid_constant__ WaveArgs<R> a) {
+  March<NY, 1, 1> w;
+  if (!w.start(g)) return;
   const int64_t pl = g.plane, n = int64_t(g.nx) * pl;
-  const int y = w.y, z = w.z;
-  const bool ylo = y == 0, yhi = y == g.ny - 1, zlo = z == 0, zhi = z == g.nz - 1;
-  const int dym = ylo ? 0 : -g.nz, dyp = yhi ? 0 : g.nz, dzm = zlo ? 0 : -1, dzp = zhi ? 0 : 1;
-  const R* const q = a.q + w.i0;
-  const R* const cf = CF ? a.c + w.i0 : nullptr;
-  const double hy = g.hy[y], hz = g.hz[z];
-  const R Ax = R(hy * hz);
-  R prv[4], cur[4], nxt[4];
+  const double hz = UNI ? 0.0 : g.hz[w.z];
+  auto load = [&](int64_t i, R v[4]) {
 #pragma unroll
-  for (int f = 0; f < 4; ++f) cur[f] = q[f * n];
+    for (int f = 0; f < 4; ++f) v[f] = a.q[f * n + i];
+  };
+  auto half = [&](R cP, R cN) { return R(0.5) * (a.mode == 0 ? fmax(cP, cN) : R(0.5) * (cP + cN)); };
+  const R c0 = a.cconst, c20 = c0 * c0, hc0 = half(c0, c0);
+  R Ax[NY];
 #pragma unroll
-  for (int f = 0; f < 4; ++f) prv[f] = q[f * n - (w.x0 > 0 ? pl : 0)];
-  if (w.x0 == 0) prv[1] = -prv[1];
+  for (int r = 0; r < NY; ++r) Ax[r] = UNI ? g.A[0] : R(g.hy[min(w.y0 + r, g.ny - 1)] * hz);
+  R cur[NY][4], nxt[NY][4], tx[NY][4], px[NY][2];  // tx, px: the face between planes x - 1 and x
+  R cc[NY], cn[NY];
 #pragma unroll
-  for (int j = 0; j < NX; ++j) {
-    const int x = w.x0 + j;
-    if (x >= g.nx) return;
-    const bool xhi = x == g.nx - 1;
-    const R* const b = q + j * pl;
-    const int64_t dxp = xhi ? 0 : pl;
-    R ym[4], yp[4], zm[4], zp[4];
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      nxt[f] = b[f * n + dxp];
-      ym[f] = b[f * n + dym];
-      yp[f] = b[f * n + dyp];
-      zm[f] = b[f * n + dzm];
-      zp[f] = b[f * n + dzp];
-    }
-    const R V = g.volume(w.i0 + j * pl);
-    if (xhi) nxt[1] = -nxt[1];
-    if (ylo) ym[2] = -ym[2];
-    if (yhi) yp[2] = -yp[2];
-    if (zlo) zm[3] = -zm[3];
-    if (zhi) zp[3] = -zp[3];
-    bool fine = true;
-#pragma unroll
-    for (int f = 0; f < 4; ++f)
-      fine = fine && fabs(cur[f]) <= a.limit && fabs(prv[f]) <= a.limit && fabs(nxt[f]) <= a.limit &&
-             fabs(ym[f]) <= a.limit && fabs(yp[f]) <= a.limit && fabs(zm[f]) <= a.limit && fabs(zp[f]) <= a.limit;
-    if (fine) {
-      const R cP = CF ? cf[j * pl] : a.cconst;
-      const R c2 = cP * cP;
-      auto half_speed = [&](int64_t off) {
-        if (!CF) return R(0.5) * (a.mode == 0 ? cP : R(0.5) * (cP + cP));
-        const R cN = cf[j * pl + off];
-        return R(0.5) * (a.mode == 0 ? fmax(cP, cN) : R(0.5) * (cP + cN));
-      };
-      const double hx = g.hx[x];
-      const R Ay = R(hx * hz), Az = R(hx * hy);
-      R acc[4] = {R(0), R(0), R(0), R(0)};
-      wave_face<0>(cur, zm, c2, half_speed(dzm), Az, acc);
-      wave_face<1>(cur, zp, c2, half_speed(dzp), Az, acc);
-      wave_face<2>(cur, ym, c2, half_speed(dym), Ay, acc);
-      wave_face<3>(cur, yp, c2, half_speed(dyp), Ay, acc);
-      wave_face<4>(cur, prv, c2, half_speed(x > 0 ? -pl : 0), Ax, acc);
-      wave_face<5>(cur, nxt, c2, half_speed(dxp), Ax, acc);
-      R* const o = a.qn + w.i0 + j * pl;
-#pragma unroll
-      for (int f = 0; f < 4; ++f) o[f * n] = a.dt * (-(acc[f] / V)) + cur[f];
+  for (int r = 0; r < NY; ++r) {
+    const int64_t i = w.x0 * pl + w.off[1 + r];
+    load(i, cur[r]);
+    cc[r] = CF ? a.c[i] : c0;
+    R B[4], cB = cc[r];
+    if (w.x0 > 0) {
+      load(i - pl, B);
+      if (CF) cB = a.c[i - pl];
     } else {
-      wave_full(g, a, x, y, z);
+      wave_ghost<0>(cur[r], B);
     }
-    // the next plane: an x wall's ghost is never carried on (xhi ends the column)
+    wave_face<0, CF>(B, cur[r], c20, CF ? half(cc[r], cB) : hc0, Ax[r], tx[r], px[r]);
+  }
+  for (int x = w.x0; x < w.x1; ++x) {
+    const int64_t b = x * pl;
+    const bool xhi = x == g.nx - 1;
+    R lo[4], hi[4], clo = c0, chi = c0;
+    load(b + w.off[0], lo);
+    load(b + w.off[NY + 1], hi);
+    if (CF) {
+      clo = a.c[b + w.off[0]];
+      chi = a.c[b + w.off[NY + 1]];
+    }
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      prv[f] = cur[f];
-      cur[f] = nxt[f];
+    for (int r = 0; r < NY; ++r) {
+      if (!xhi) {
+        load(b + pl + w.off[1 + r], nxt[r]);
+        cn[r] = CF ? a.c[b + pl + w.off[1 + r]] : c0;
+      } else {
+        wave_ghost<0>(cur[r], nxt[r]);
+        cn[r] = cc[r];
+      }
+    }
+    const double hx = UNI ? 0.0 : g.hx[x];
+    const R Ay = UNI ? g.A[1] : R(hx * hz);
+    R ty[4], py[2];
+    if (w.y0 == 0) wave_ghost<1>(cur[0], lo);
+    wave_face<1, CF>(lo, cur[0], c20, CF ? half(cc[0], clo) : hc0, Ay, ty, py);
+#pragma unroll
+    for (int r = 0; r < NY; ++r) {
+      const R* P = cur[r];
+      const int y = w.y0 + r;
+      const int64_t i = b + w.off[1 + r];
+      const R vol = UNI ? g.v : g.volume(i);
+      const Volume<R> V{vol, UNI ? g.rv : R(1) / vol};
+      const R Az = UNI ? g.A[2] : R(hx * g.hy[min(y, g.ny - 1)]);
+      const R c2 = CF ? cc[r] * cc[r] : c20;
+      // z: the face above, and the one below from the lane below
+      R Z[4], tz[4], pz[2], tzl[4], pzl[2];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) Z[f] = __shfl_down_sync(kWarp, P[f], 1);
+      R cz = CF ? __shfl_down_sync(kWarp, cc[r], 1) : c0;
+      if (w.zhi) {
+        wave_ghost<2>(P, Z);
+        cz = cc[r];
+      }
+      wave_face<2, CF>(P, Z, c20, CF ? half(cc[r], cz) : hc0, Az, tz, pz);
+#pragma unroll
+      for (int f = 0; f < 4; ++f) tzl[f] = __shfl_up_sync(kWarp, tz[f], 1);
+      if (CF) {
+        pzl[0] = __shfl_up_sync(kWarp, pz[0], 1);
+        pzl[1] = __shfl_up_sync(kWarp, pz[1], 1);
+      }
+      if (w.zlo) {
+        wave_ghost<2>(P, Z);
+        wave_face<2, CF>(Z, P, c20, CF ? half(cc[r], cc[r]) : hc0, Az, tzl, pzl);
+      }
+      // y and x: the faces above
+      R th[4], ph[2], tu[4], pu[2], N[4];
+      R cN = cc[r];
+      if (y >= g.ny - 1) {
+        wave_ghost<1>(P, N);
+      } else {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) N[f] = r + 1 < NY ? cur[r + 1 < NY ? r + 1 : r][f] : hi[f];
+        if (CF) cN = r + 1 < NY ? cc[r + 1 < NY ? r + 1 : r] : chi;
+      }
+      wave_face<1, CF>(P, N, c20, CF ? half(cc[r], cN) : hc0, Ay, th, ph);
+      wave_face<0, CF>(P, nxt[r], c20, CF ? half(cc[r], cn[r]) : hc0, Ax[r], tu, pu);
+      if (CF) {  // the pressure flux with this cell's c^2
+        tzl[0] = (c2 * pzl[0] - pzl[1]) * Az;
+        tz[0] = (c2 * pz[0] - pz[1]) * Az;
+        ty[0] = (c2 * py[0] - py[1]) * Ay;
+        th[0] = (c2 * ph[0] - ph[1]) * Ay;
+        tx[r][0] = (c2 * px[r][0] - px[r][1]) * Ax[r];
+        tu[0] = (c2 * pu[0] - pu[1]) * Ax[r];
+      }
+      R o[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) o[f] = (((((R(0) - tzl[f]) + tz[f]) - ty[f]) + th[f]) - tx[r][f]) + tu[f];
+      V.template divide<4>(o);
+      bool ok = true;
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        o[f] = a.dt * (-o[f]) + P[f];
+        ok = ok && finite(o[f]);
+        ty[f] = th[f];
+        tx[r][f] = tu[f];
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        py[j] = ph[j];
+        px[r][j] = pu[j];
+      }
+      if (w.out && y < g.ny) {
+        if (ok) {
+#pragma unroll
+          for (int f = 0; f < 4; ++f) a.qn[f * n + i] = o[f];
+        } else {
+          wave_full(g, a, x, y, w.z);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < NY; ++r) {
+      cc[r] = cn[r];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) cur[r][f] = nxt[r][f];
     }
   }
 }
@@ -527,30 +707,45 @@ __global__ void __launch_bounds__(kThreads) box_volume_k(int nx, int ny, int nz,
   if (other) atomicOr(differs, 1);
 }
 
-template <class R> Box<R> box_of(const cfdb_mesh* m, int nx_per_thread) {
+// Kernel arguments for NY rows per thread, HZ halo lanes and blocks of
+// `threads`; *blocks = the grid.  x is cut into chunks for about 32 warps per
+// SM (one wave at 64 registers; 24 and 48 measured within 10 %), each at least
+// two planes long: a chunk evaluates the face below it a second time.
+template <class R> Box<R> box_of(const cfdb_ctx* ctx, const cfdb_mesh* m, int NY, int HZ, int threads, unsigned* blocks) {
   const BoxGeomDev& b = m->box[sizeof(R) == 8 ? 1 : 0];
   Box<R> g;
   g.nx = int(m->nx); g.ny = int(m->ny); g.nz = int(m->nz);
   g.plane = unsigned(m->ny * m->nz);
-  g.chunks = unsigned((m->nx + nx_per_thread - 1) / nx_per_thread);
+  g.groups = int((m->ny + NY - 1) / NY);
+  const int64_t lanes = int64_t(g.groups) * m->nz;
+  g.tiles = unsigned((lanes + 32 - 2 * HZ - 1) / (32 - 2 * HZ));
+  const int64_t want = std::max<int64_t>(1, int64_t(ctx->num_sms) * 32 / g.tiles);
+  g.chunks = unsigned(std::min<int64_t>(std::min(want, int64_t(m->nx)), std::max<int64_t>(1, m->nx / 2)));
+  *blocks = unsigned((int64_t(g.tiles) * g.chunks * 32 + threads - 1) / threads);
   g.hx = b.h[0]; g.hy = b.h[1]; g.hz = b.h[2];
   auto t = [](const void* p) { return static_cast<const R*>(p); };
   g.ax = t(b.alpha[0]); g.ay = t(b.alpha[1]); g.az = t(b.alpha[2]);
   g.lmx = t(b.len[0]); g.lpx = t(b.len[1]); g.lmy = t(b.len[2]); g.lpy = t(b.len[3]); g.lmz = t(b.len[4]); g.lpz = t(b.len[5]);
   g.vol = t(b.vol);
   g.v = R(b.v);
+  g.rv = R(1) / g.v;
   g.limit = R(b.limit);
+  for (int d = 0; d < 3; ++d) {
+    g.A[d] = R(b.uA[d]);
+    g.al[d] = R(b.ual[d]);
+    g.lm[d] = R(b.ulm[d]);
+    g.lp[d] = R(b.ulp[d]);
+  }
   return g;
 }
 
-unsigned grid_of(const cfdb_mesh* m, int nx) {
-  const int64_t threads = ((m->nx + nx - 1) / nx) * m->ny * m->nz;
-  return unsigned((threads + kThreads - 1) / kThreads);
+// Rows per thread: two share the face between them (200^3 FP32: gradient 33
+// against 40 us, stabilisation 80 against 97), once the mesh gives every SM its
+// warps; in double the registers of a second row cost more warps than it saves
+// (100 x 90 x 96: stabilisation 33 against 37 us, acoustic step 21 against 27).
+template <class R> int rows_per_thread(const cfdb_ctx* ctx, const cfdb_mesh* m) {
+  return sizeof(R) == 4 && m->n >= int64_t(ctx->num_sms) * 8192 ? 2 : 1;
 }
-
-// Fields of a few hundred thousand cells fill the SMs only with one cell per
-// thread; larger ones want the loads of several planes in flight.
-bool one_cell(const cfdb_ctx* ctx, const cfdb_mesh* m) { return m->n < int64_t(ctx->num_sms) * 4096; }
 
 template <class R>
 int build_box(cfdb_mesh* m, BoxGeomDev& b) {
@@ -622,6 +817,26 @@ int build_box(cfdb_mesh* m, BoxGeomDev& b) {
   }
   b.limit = limit;
   b.state = 1;
+  // one value per direction?  (products round monotonically: the extremes decide)
+  auto range = [](const std::vector<double>& v, double lim[2]) {
+    lim[0] = *std::min_element(v.begin(), v.end());
+    lim[1] = *std::max_element(v.begin(), v.end());
+  };
+  double h[3][2];
+  for (int d = 0; d < 3; ++d) range(t[d].h, h[d]);
+  b.uni = !back.differs;
+  for (int d = 0; d < 3; ++d) {
+    const int e = d == 0 ? 1 : 0, f = d == 2 ? 1 : 2;
+    b.uA[d] = double(R(h[e][0] * h[f][0]));
+    b.uni = b.uni && R(h[e][0] * h[f][0]) == R(h[e][1] * h[f][1]);
+    auto one = [&](const double* p, size_t count, double* out) {
+      *out = count ? double(R(p[0])) : 1.0;
+      for (size_t k = 0; k < count; ++k) b.uni = b.uni && R(p[k]) == R(p[0]);
+    };
+    one(t[d].alpha.data() + 1, t[d].alpha.size() - 2, &b.ual[d]);  // interior faces; a wall face multiplies zero
+    one(t[d].len_lo.data(), t[d].len_lo.size(), &b.ulm[d]);
+    one(t[d].len_hi.data(), t[d].len_hi.size(), &b.ulp[d]);
+  }
   return CFDB_OK;
 }
 
@@ -643,60 +858,73 @@ int cfdb_mesh_need_box(cfdb_mesh* m, int dtype, bool* usable) {
   return CFDB_OK;
 }
 
-// f(R(), NX) with the precision and the planes per thread of this mesh
-template <class F> int with_form(cfdb_ctx* ctx, const cfdb_mesh* m, int dtype, F f) {
-  if (dtype == CFDB_F64) f(double(), one_cell(ctx, m));
-  else f(float(), one_cell(ctx, m));
+// The kernel of a mesh: one value per direction and all directions, all
+// directions, or neither; NY = 2 rows per thread in FP32 only.
+#define BOX_FORMS(kernel, ...)                                   \
+  (uni && mask == 7 ? kernel<__VA_ARGS__, true, true> : mask == 7 ? kernel<__VA_ARGS__, false, true> : kernel<__VA_ARGS__, false, false>)
+
+template <class R, int OP> int launch_sum(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask, double k, double dt) {
+  constexpr int NY = sizeof(R) == 4 ? 2 : 1;
+  const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
+  const int rows = rows_per_thread<R>(ctx, m);
+  unsigned blocks = 0;
+  const Box<R> g = box_of<R>(ctx, m, rows, 1, kThreads, &blocks);
+  auto kern = rows == 1 ? BOX_FORMS(box_sum_k, R, OP, 1) : BOX_FORMS(box_sum_k, R, OP, NY);
+  kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
+  CFDB_LAUNCHED(ctx);
+  return CFDB_OK;
+}
+
+template <class R> int launch_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask) {
+  constexpr int NY = sizeof(R) == 4 ? 2 : 1;
+  const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
+  const int rows = rows_per_thread<R>(ctx, m);
+  unsigned blocks = 0;
+  const Box<R> g = box_of<R>(ctx, m, rows, 2, 128, &blocks);
+  auto kern = rows == 1 ? BOX_FORMS(box_stab_k, R, 1) : BOX_FORMS(box_stab_k, R, NY);
+  kern<<<blocks, 128, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask);
+  CFDB_LAUNCHED(ctx);
+  return CFDB_OK;
+}
+
+template <class R, int NY> auto wave_kernel(bool uni, bool c) {
+  return uni ? (c ? box_wave_k<R, NY, true, true> : box_wave_k<R, NY, true, false>)
+             : (c ? box_wave_k<R, NY, false, true> : box_wave_k<R, NY, false, false>);
+}
+template <class R>
+int launch_wave(cfdb_ctx* ctx, cfdb_mesh* m, const void* q, void* qn, const void* c, double cconst, int mode, double dt) {
+  constexpr int NY = sizeof(R) == 4 ? 2 : 1;
+  const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
+  const int rows = rows_per_thread<R>(ctx, m);
+  unsigned blocks = 0;
+  const Box<R> g = box_of<R>(ctx, m, rows, 1, 128, &blocks);
+  const WaveArgs<R> a{static_cast<const R*>(q), static_cast<R*>(qn), static_cast<const R*>(c), R(cconst), R(dt), mode};
+  auto kern = rows == 1 ? wave_kernel<R, 1>(uni, c != nullptr) : wave_kernel<R, NY>(uni, c != nullptr);
+  kern<<<blocks, 128, 0, ctx->stream>>>(g, a);
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
 }
 
 int box_grad(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
-  return with_form(ctx, m, dtype, [&](auto r, bool one) {
-    using R = decltype(r);
-    auto kern = one ? box_grad_k<R, 1> : box_grad_k<R, 4>;
-    const int nx = one ? 1 : 4;
-    kern<<<grid_of(m, nx), kThreads, 0, ctx->stream>>>(box_of<R>(m, nx), static_cast<const R*>(phi), static_cast<R*>(out), mask);
-  });
+  return dtype == CFDB_F64 ? launch_sum<double, OP_GRAD>(ctx, m, phi, out, mask, 0, 0)
+                           : launch_sum<float, OP_GRAD>(ctx, m, phi, out, mask, 0, 0);
 }
 
 int box_lapl(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
-  return with_form(ctx, m, dtype, [&](auto r, bool one) {
-    using R = decltype(r);
-    auto kern = one ? box_lapl_k<R, 1> : box_lapl_k<R, 4>;
-    const int nx = one ? 1 : 4;
-    kern<<<grid_of(m, nx), kThreads, 0, ctx->stream>>>(box_of<R>(m, nx), static_cast<const R*>(phi), static_cast<R*>(out), mask,
-                                                       R(0), R(0));
-  });
+  return dtype == CFDB_F64 ? launch_sum<double, OP_LAPL>(ctx, m, phi, out, mask, 0, 0)
+                           : launch_sum<float, OP_LAPL>(ctx, m, phi, out, mask, 0, 0);
 }
 
 int box_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* Tn, double k, double dt) {
-  return with_form(ctx, m, dtype, [&](auto r, bool one) {
-    using R = decltype(r);
-    auto kern = one ? box_lapl_k<R, 1, true> : box_lapl_k<R, 4, true>;
-    const int nx = one ? 1 : 4;
-    kern<<<grid_of(m, nx), kThreads, 0, ctx->stream>>>(box_of<R>(m, nx), static_cast<const R*>(T), static_cast<R*>(Tn), 7, R(k), R(dt));
-  });
+  return dtype == CFDB_F64 ? launch_sum<double, OP_HEAT>(ctx, m, T, Tn, 7, k, dt) : launch_sum<float, OP_HEAT>(ctx, m, T, Tn, 7, k, dt);
 }
 
 int box_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
-  return with_form(ctx, m, dtype, [&](auto r, bool one) {
-    using R = decltype(r);
-    constexpr int NX = sizeof(R) == 8 ? 2 : 4;
-    auto kern = one ? box_stab_k<R, 1> : box_stab_k<R, NX>;
-    const int nx = one ? 1 : NX;
-    kern<<<grid_of(m, nx), kThreads, 0, ctx->stream>>>(box_of<R>(m, nx), static_cast<const R*>(phi), static_cast<R*>(out), mask);
-  });
+  return dtype == CFDB_F64 ? launch_stab<double>(ctx, m, phi, out, mask) : launch_stab<float>(ctx, m, phi, out, mask);
 }
 
 int box_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* qn, const void* c, double cconst, int mode,
                   double dt) {
-  return with_form(ctx, m, dtype, [&](auto r, bool one) {
-    using R = decltype(r);
-    WaveArgs<R> a{static_cast<const R*>(q), static_cast<R*>(qn), static_cast<const R*>(c), R(cconst), R(dt), mode,
-                  std::numeric_limits<R>::max() / R(16)};
-    auto kern = c ? (one ? box_wave_k<R, 1, true> : box_wave_k<R, 4, true>) : (one ? box_wave_k<R, 1, false> : box_wave_k<R, 4, false>);
-    const int nx = one ? 1 : 4;
-    kern<<<grid_of(m, nx), kThreads, 0, ctx->stream>>>(box_of<R>(m, nx), a);
-  });
+  return dtype == CFDB_F64 ? launch_wave<double>(ctx, m, q, qn, c, cconst, mode, dt)
+                           : launch_wave<float>(ctx, m, q, qn, c, cconst, mode, dt);
 }

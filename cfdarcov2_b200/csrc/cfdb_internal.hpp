@@ -70,6 +70,10 @@ struct BoxGeomDev {
   const void* alpha[3] = {};
   const void* len[6] = {};  // x-, x+, y-, y+, z-, z+
   double v = 0, limit = 0;
+  // every cell's volume, areas, interior alphas and lengths round to one value
+  // per direction (uA: the face normal to x, y, z)
+  bool uni = false;
+  double uA[3] = {}, ual[3] = {}, ulm[3] = {}, ulp[3] = {};
 };
 
 // Compact FP32 geometry of vertex meshes for the fused kernels: per cell the

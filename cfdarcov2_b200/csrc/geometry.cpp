@@ -161,7 +161,11 @@ double axis_tables(int64_t nx, int64_t ny, int64_t nz, double dx, double dy, dou
   // every table value, converted, is finite (a product by zero stays zero)
   const double top = f64 ? std::numeric_limits<double>::max() : double(std::numeric_limits<float>::max());
   const double max_a = std::max(max_h[0] * max_h[1], std::max(max_h[0] * max_h[2], max_h[1] * max_h[2]));
-  const double min_v = min_h[0] * min_h[1] * min_h[2];
+  // volumes by whose reciprocal the kernels divide (box_ops.cu); the volume
+  // itself is a sum of rounded terms, within a few parts in 10^3 of the product
+  // on any mesh whose cells are not lost in the rounding of its coordinates
+  const double min_v = min_h[0] * min_h[1] * min_h[2], max_v = max_h[0] * max_h[1] * max_h[2];
+  if (!(min_v > 0x1p-79) || !(max_v < 0x1p23)) return bad;
   if (!(max_a < 0.5 * top) || !(1.0 / min_d < 0.5 * top) || !(max_len < 0.5 * top)) return bad;
   // magnitudes below `limit` overflow in no intermediate of the operators:
   // gradient 2 |phi| A / V, face value |phi| + len |gradient|, their products by A / V

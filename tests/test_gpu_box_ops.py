@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 SHAPES = [((1, 1, 1), (0.5, 0.3, 0.2)), ((1, 4, 4), (1.0, 1.0, 1.0)), ((2, 3, 5), (1 / 13, 0.3, 1 / 7)),
           ((33, 7, 9), (1 / 33, 1 / 33, 1 / 33)), ((5, 6, 130), (0.01, 0.02, 0.03)), ((101, 79, 83), (1 / 101, 1 / 101, 1 / 101)),
-          ((88, 84, 96), (0.125, 0.25, 0.5))]
+          ((88, 84, 96), (0.125, 0.25, 0.5)), ((161, 95, 82), (1.0, 1.0, 1.0))]
 
 
 def pair(cfdb, ctx, shape, spacing):
@@ -39,6 +39,7 @@ def field(n, dtype, seed, scale=1.0):
 def test_operators_equal_the_face_arrays(cfdb, ctx, shape, spacing, dtype):
     m, a = pair(cfdb, ctx, shape, spacing)
     phi = field(m.n, dtype, 1)
+    phi[: m.n // 3] *= 1e-36 if dtype == torch.float32 else 1e-300  # sums below the reciprocal's range
     for op in ("grad", "lapl", "stab"):
         for mask in (7, 1, 2, 4, 6, 0):
             got, ref = (getattr(ctx, op)(k, phi, mask=mask) for k in (m, a))
