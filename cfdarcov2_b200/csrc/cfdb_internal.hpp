@@ -285,6 +285,9 @@ int fused_d2t_step(cfdb_ctx* ctx, cfdb_mesh* m, const void* u, const void* u_pre
 // when the mesh does not fit (nothing launched).
 int heat_resident_run(cfdb_ctx* ctx, cfdb_mesh* m, const void* Ta, void* Tb, double k, double dt, int32_t steps,
                       int* launched);
+// The same with several steps per pass over the field (heat_blocked.cu).
+int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, double dt, int32_t steps, int use_graph,
+                     bool keep_other);
 int fused_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* qn, const void* c,
                     double cconst, int mode, double dt);
 // distorted.cu

@@ -1,0 +1,32 @@
+"""Several heat steps per pass (cfdb_heat_run on fields too large for one
+cluster) against the one-step sweep, bit for bit: every pass length, tiles with
+and without walls on their sides, odd rows, single planes and columns, and the
+buffers the result may and may not touch."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("shape", [(1, 128, 64), (2, 65, 128), (9, 127, 132), (33, 123, 248), (4, 1, 4096), (70, 129, 36),
+                                   (160, 130, 100), (300, 33, 392)])
+def test_passes_equal_single_steps(cfdb, ctx, shape):
+    X, Y, Z = shape
+    m = cfdb.Mesh.structured(ctx, X, Y, Z, 1 / X, 1 / Y, 1 / Z)
+    T0 = torch.as_tensor(np.random.default_rng(3).uniform(-1, 1, m.n), dtype=torch.float32, device=DEV)
+    T0[::7] = 0.0
+    k, dt = 0.01, 0.1 * min(1 / X, 1 / Y, 1 / Z) ** 2 / 0.01
+    p, q = T0.clone(), torch.empty_like(T0)
+    for steps in range(1, 12):
+        ctx.heat_step(m, p, q, k, dt)
+        p, q = q, p
+        for graph in (True, False):
+            a, b = T0.clone(), torch.full_like(T0, float("nan"))
+            final = ctx.heat_run(m, a, b, k, dt, steps, use_graph=graph)
+            assert (final is b) == bool(steps & 1)
+            assert torch.equal(final, p), steps
+    ctx.sync()
