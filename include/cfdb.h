@@ -115,11 +115,8 @@ int cfdb_ctx_trim(cfdb_ctx* ctx);
  * copies it issued land, and reports CFDB_ETIMEOUT through cfdb_sync; its
  * results are then invalid and the context stays usable.  missing_plane >= 0
  * is a test hook: the first CTA of every later sweep arms that plane's
- * barrier without issuing its copy, and the second cluster of the
- * cluster-resident heat solver (cfdb_heat_run) does not publish its edge
- * planes of that step, so a wait runs out without any fault (-1 turns it
- * off).  The resident solver's waits (for a neighbouring cluster's planes)
- * have the same bound.  Drops the context's cached step graphs.  No reference
+ * barrier without issuing its copy, so a wait runs out without any fault (-1
+ * turns it off).  Drops the context's cached step graphs.  No reference
  * counterpart: the reference's kernels have no waits, and gpuAssert exits
  * the process on any CUDA error (include/cuda_operators.hpp:29-36). */
 int cfdb_ctx_set_wait_limit(cfdb_ctx* ctx, int64_t cycles, int32_t missing_plane);
@@ -318,10 +315,10 @@ int cfdb_wave_step(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, int path, const vo
  * graph (after two eager steps that perform any one-time setup) and replays
  * it, so host launch latency never gaps the device.  Asynchronous.
  * cfdb_heat_run, fused FP32: a uniform mesh whose field fits twice into the
- * shared memory of one thread-block cluster (e.g. 64^3), or else of four
- * co-resident clusters (e.g. 128 x 64 x 64), runs all steps in one launch
- * instead, field resident on chip; same arithmetic, same result.  Only the
- * buffer *final_in_b names is defined afterwards. */
+ * shared memory of one thread-block cluster (e.g. 64^3) runs all steps in one
+ * launch, field resident on chip; a larger one takes two or three steps per
+ * pass over the field; same arithmetic, same result.  Only the buffer
+ * *final_in_b names is defined afterwards. */
 int cfdb_heat_run(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, int path, void* T_a, void* T_b, double k, double dt,
                   int32_t steps, int use_graph, int* final_in_b);
 int cfdb_wave_run(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, int path, void* q_a, void* q_b, const void* c_field,
