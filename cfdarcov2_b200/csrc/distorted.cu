@@ -179,10 +179,18 @@ int compact_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, voi
     const float cs = float(cconst);
     const DistFacePhys::Params p{float(dt), 0.5f * cs * cs, 0.5f * cs};
     const stencil::PaddedGeom pg{cg.S, cg.zp, cg.yp, m->nx + 1, cg.np};
-    // 64-wide z tiles (two cells per thread) unless 32-wide ones pad the z rows less
-    const int64_t pad64 = (m->nz + 63) / 64 * 64 - m->nz, pad32 = (m->nz + 31) / 32 * 32 - m->nz;
-    if (m->nz > 32 && pad64 <= pad32) return stencil::launch_face_sweep<DistFacePhys, 64, 8, 3, 2>(ctx, m, q, pg, qn, p, 0);
-    return stencil::launch_face_sweep<DistFacePhys, 32, 8, 3, 1>(ctx, m, q, pg, qn, p, 0);
+    // The tile width by the cells per row it covers with its padding, times its
+    // cost per covered cell: 64 x 8 (two cells per thread) 1, 96 x 4 1.05 (half the
+    // rows: more halo), 48 x 8 1.13, 32 x 8 1.12 (fewer threads per CTA).  96^3: 12.4 us
+    // with 96, 14.5 with 32 and one cell per thread, 15.5 with 64; 96 x 96 x 48: 8.4 with
+    // 48, 10.1 with 64; 128^3: 29.4 with 64, 31.6 with 32, 40.4 with 96.
+    auto cover = [&](int64_t tz) { return double((m->nz + tz - 1) / tz * tz); };
+    const double c64 = cover(64), c96 = 1.05 * cover(96), c48 = 1.13 * cover(48), c32 = 1.12 * cover(32);
+    const double least = std::min(std::min(c64, c96), std::min(c48, c32));
+    if (c64 == least) return stencil::launch_face_sweep<DistFacePhys, 64, 8, 3, 2>(ctx, m, q, pg, qn, p, 0);
+    if (c96 == least) return stencil::launch_face_sweep<DistFacePhys, 96, 4, 3, 2>(ctx, m, q, pg, qn, p, 0);
+    if (c48 == least) return stencil::launch_face_sweep<DistFacePhys, 48, 8, 3, 2>(ctx, m, q, pg, qn, p, 0);
+    return stencil::launch_face_sweep<DistFacePhys, 32, 8, 3, 2>(ctx, m, q, pg, qn, p, 0);
   }
   CompactArgs a{cg.S, cg.np, cg.yp, cg.zp, int(m->nx), int(m->ny), int(m->nz), (long long)m->n};
   compact_wave_k<<<grid_for(ctx, m->n, kThreads, 8), kThreads, 0, ctx->stream>>>(

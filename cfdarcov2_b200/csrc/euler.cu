@@ -267,7 +267,7 @@ constexpr int kEulerVZ = 2;
 
 static_assert(kEulerVZ == 2, "EulerPhys provides its per-cell update only as packed pairs");
 
-template <int TZ>
+template <int TZ, int TY>
 int launch_euler(cfdb_euler* e, const void* U, void* Un, int64_t s) {
   cfdb_mesh* m = e->mesh;
   EulerPhys::Params p;
@@ -283,23 +283,30 @@ int launch_euler(cfdb_euler* e, const void* U, void* Un, int64_t s) {
   const stencil::PaddedGeom none{nullptr, 0, 0, 0, 0};
   int grid = 0;
   const int rc =
-      stencil::launch_face_sweep<EulerPhys, TZ, 8, 4, kEulerVZ>(e->ctx, m, U, none, Un, p, kEulerCtasPerSm, &grid);
+      stencil::launch_face_sweep<EulerPhys, TZ, TY, 4, kEulerVZ>(e->ctx, m, U, none, Un, p, kEulerCtasPerSm, &grid);
   if (rc) return rc;
   if (grid > e->part_cap) return cfdb_fail(e->ctx, CFDB_ECUDA, "fused Euler grid %d beyond its %d partials", grid, e->part_cap);
   e->fused_grid = grid;
-  e->fused_threads = (TZ / kEulerVZ) * 8;
+  e->fused_threads = (TZ / kEulerVZ) * TY;
   return CFDB_OK;
 }
 
-int tz_for(const cfdb_mesh* m) { return m->nz >= 64 ? 64 : 32; }
+// Tiles of 64 x 8 or 32 x 16 cells (256 threads either way), whichever covers
+// fewer cells with its padding of rows and columns: 96^3 14.3 us per step with 32,
+// 17.4 with 64; 128 x 64 x 32 7.8 against 11.4 (a 32 x 8 tile left half of the SM's
+// threads out); 100^3 20.0 with 32, 19.5 with 64; 512 x 64 x 64 the same.
+bool wide_tiles(const cfdb_mesh* m) {
+  auto cover = [&](int64_t tz, int64_t ty) { return double((m->nz + tz - 1) / tz * tz) * double((m->ny + ty - 1) / ty * ty); };
+  return cover(64, 8) <= 1.05 * cover(32, 16);
+}
 
 }  // namespace
 
 // Upper bound of the fused Euler grid (sizes the per-CTA partials): at most
 // kEulerCtasPerSm resident CTAs per SM are ever requested.
 int euler_fused_grid(const cfdb_euler* e) {
-  const int tz = tz_for(e->mesh);
-  const stencil::SweepShape sh = stencil::sweep_shape(e->ctx, e->mesh, tz, 8, kEulerCtasPerSm);
+  const bool wide = wide_tiles(e->mesh);
+  const stencil::SweepShape sh = stencil::sweep_shape(e->ctx, e->mesh, wide ? 64 : 32, wide ? 8 : 16, kEulerCtasPerSm);
   return sh.tiles * sh.chunks;
 }
 
@@ -316,10 +323,7 @@ int euler_fold_pending(cfdb_euler* e) {
 }
 
 int euler_fused_step(cfdb_euler* e, const void* U, void* Un, int64_t s) {
-  switch (tz_for(e->mesh)) {
-    case 64: return launch_euler<64>(e, U, Un, s);
-    default: return launch_euler<32>(e, U, Un, s);
-  }
+  return wide_tiles(e->mesh) ? launch_euler<64, 8>(e, U, Un, s) : launch_euler<32, 16>(e, U, Un, s);
 }
 
 // ---------------------------------------------------------------------------

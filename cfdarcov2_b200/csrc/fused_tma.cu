@@ -4,6 +4,7 @@
 // Replaces the reference's per-equation JIT kernel (src/fvm3d.cpp:1219-1394),
 // which streamed ~180 B/cell of geometry per step; on a uniform mesh the
 // geometry reduces to three spacings.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <string>
@@ -215,22 +216,48 @@ int dispatch_tz(cfdb_ctx* ctx, const cfdb_mesh* m, const void* q, void* out, con
   return stencil::launch_sweep<Phys, 32, 8, S>(ctx, m, q, nullptr, c, out, prm, ctas_per_sm);
 }
 
-// Tile width of the wave-template sweeps and of the heat sweep with the
-// boundary copy: 64 where it pads the z rows less than 128 (nz = 400: 448
-// against 512 cells per row; 126 against 156 us per d2t step, 158 against
-// 176 us per heat step with the copy), else as dispatch_tz.  The plain heat
-// sweep keeps 128 at nz = 400 (112 us against 123 us with 64).
+// Tile of the leapfrog sweep and of the heat sweep with the boundary copy, by
+// the cells it covers with its padding of rows and columns, times its cost per
+// covered cell (128- and 64-wide tiles of 8 rows 1, 40 and 32 wide ones of 16 rows
+// 1.07: more of their loads are halo).  200^3 d2t: 19.0 us with 40 (no padding),
+// 22.3 with 128 or 64 (256 cells per row), 21.4 with 32; 200 x 200 x 96: 10.2 us
+// with 32 against 12.2; 200 x 200 x 300: 27.6 us with 64 against 29.7 with 40.  (The
+// plain heat sweep keeps its own, below.)
 template <class Phys>
 int dispatch_padded(cfdb_ctx* ctx, const cfdb_mesh* m, const void* u, void* u_next, const typename Phys::Params& prm) {
-  const int64_t pad64 = (m->nz + 63) / 64 * 64, pad128 = (m->nz + 127) / 128 * 128;
-  if (m->nz >= 128 && pad64 < pad128)
-    return stencil::launch_sweep<Phys, 64, 8, 6>(ctx, m, u, nullptr, nullptr, u_next, prm, 0);
-  return dispatch_tz<Phys, 6>(ctx, m, u, u_next, nullptr, prm, 0);
+  auto cover = [&](int64_t tz, int64_t ty) { return double((m->nz + tz - 1) / tz * tz) * double((m->ny + ty - 1) / ty * ty); };
+  const double c128 = m->nz >= 128 ? cover(128, 8) : INFINITY, c64 = m->nz >= 64 ? cover(64, 8) : INFINITY;
+  const double c40 = 1.07 * cover(40, 16), c32 = 1.07 * cover(32, 16);
+  const double least = std::min(std::min(c128, c64), std::min(c40, c32));
+  if (c128 == least) return stencil::launch_sweep<Phys, 128, 8, 6>(ctx, m, u, nullptr, nullptr, u_next, prm, 0);
+  if (c64 == least) return stencil::launch_sweep<Phys, 64, 8, 6>(ctx, m, u, nullptr, nullptr, u_next, prm, 0);
+  if (c40 == least) return stencil::launch_sweep<Phys, 40, 16, 6>(ctx, m, u, nullptr, nullptr, u_next, prm, 0);
+  return stencil::launch_sweep<Phys, 32, 16, 6>(ctx, m, u, nullptr, nullptr, u_next, prm, 0);
+}
+
+// Tile of the acoustic sweeps, by the cells it covers with its padding times its
+// cost per covered cell: 128 x 8 and 64 x 8 tiles 1 (the wider one first where
+// they tie with constant c, the narrower with a c field, whose fifth staged field
+// leaves it one more CTA per SM), 32 x 16 1.08, 40 x 16 and 48 x 8 1.15.  Constant c /
+// c field, us per step: 96^3 6.5 / 8.4 with 32, 7.9 / 10.9 with 64; 200^3 48.6 / 59.5
+// with 40, 56.3 / 70.6 with 128; 60 x 72 x 48 5.7 / 5.9 with 48, 7.2 / 7.7 with 32;
+// 128^3 11.2 / 16.3 with 128, 11.4 / 16.1 with 32; 100^3 9.1 with 128, 10.9 with 32.
+template <class Phys>
+int dispatch_wave(cfdb_ctx* ctx, const cfdb_mesh* m, const void* q, void* qn, const void* c, const typename Phys::Params& p) {
+  auto cover = [&](int64_t tz, int64_t ty) { return double((m->nz + tz - 1) / tz * tz) * double((m->ny + ty - 1) / ty * ty); };
+  const double c128 = (Phys::HAS_C ? 1.01 : 1.0) * cover(128, 8), c64 = (Phys::HAS_C ? 1.0 : 1.01) * cover(64, 8);
+  const double c48 = 1.15 * cover(48, 8), c40 = 1.15 * cover(40, 16), c32 = 1.08 * cover(32, 16);
+  const double least = std::min({c128, c64, c48, c40, c32});
+  if (c128 == least) return stencil::launch_sweep<Phys, 128, 8, 3>(ctx, m, q, nullptr, c, qn, p, 0);
+  if (c64 == least) return stencil::launch_sweep<Phys, 64, 8, 4>(ctx, m, q, nullptr, c, qn, p, 0);
+  if (c48 == least) return stencil::launch_sweep<Phys, 48, 8, 4>(ctx, m, q, nullptr, c, qn, p, 0);
+  if (c40 == least) return stencil::launch_sweep<Phys, 40, 16, 4>(ctx, m, q, nullptr, c, qn, p, 0);
+  return stencil::launch_sweep<Phys, 32, 16, 4>(ctx, m, q, nullptr, c, qn, p, 0);
 }
 
 // Tile shape of the constant-c wave sweep.  CFDB_WAVE_TILE=TZxTYxS picks one of
-// the instantiated shapes (for tuning sweeps); the default is 128x8x3 (three
-// staged planes: the shape that measured fastest on meshes beyond L2).
+// the instantiated shapes (for tuning sweeps); three staged planes at 128x8
+// measured fastest on meshes beyond L2.
 int dispatch_wave_tiles(cfdb_ctx* ctx, const cfdb_mesh* m, const void* q, void* qn,
                         const WavePhys<false>::Params& p) {
   using W = WavePhys<false>;
@@ -243,8 +270,7 @@ int dispatch_wave_tiles(cfdb_ctx* ctx, const cfdb_mesh* m, const void* q, void* 
     if (t == "128x8x4v2") return stencil::launch_sweep<W, 128, 8, 4, 2>(ctx, m, q, nullptr, nullptr, qn, p, 0);
     if (t == "64x8x4v1") return stencil::launch_sweep<W, 64, 8, 4, 1>(ctx, m, q, nullptr, nullptr, qn, p, 0);
   }
-  if (m->nz >= 128) return stencil::launch_sweep<W, 128, 8, 3>(ctx, m, q, nullptr, nullptr, qn, p, 0);
-  return dispatch_tz<W, 4>(ctx, m, q, qn, nullptr, p, 0);
+  return dispatch_wave<W>(ctx, m, q, qn, nullptr, p);
 }
 
 }  // namespace
@@ -332,7 +358,7 @@ int fused_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void*
   const double ih[3] = {1.0 / m->dx, 1.0 / m->dy, 1.0 / m->dz};
   if (c) {
     WavePhys<true>::Params p{float(dt), {float(ih[0]), float(ih[1]), float(ih[2])}, 0.f, mode, {}, {}, {}};
-    return dispatch_tz<WavePhys<true>, 4>(ctx, m, q, qn, c, p, 0);
+    return dispatch_wave<WavePhys<true>>(ctx, m, q, qn, c, p);
   }
   WavePhys<false>::Params p{float(dt), {float(ih[0]), float(ih[1]), float(ih[2])}, float(cconst), mode, {}, {}, {}};
   for (int d = 0; d < 3; ++d) {
