@@ -200,7 +200,7 @@ template <int NY, int HY, int HZ> struct March {
   int y0, z, x0, x1;
   int off[NY + 2 * HY];
   bool out, zlo, zhi;
-  template <class R> __device__ __forceinline__ bool start(const Box<R>& g) {
+  template <class G> __device__ __forceinline__ bool start(const G& g) {
     const unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= g.tiles * g.chunks) return false;  // whole warps
     const unsigned chunk = w / g.tiles, tile = w - chunk * g.tiles;
@@ -461,6 +461,216 @@ __global__ void __launch_bounds__(128) box_stab_k(const __grid_constant__ Box<R>
   }
 }
 
+// ---- vertex meshes: every face's geometry once ------------------------------------
+//
+// The N x 6 arrays hold each interior face twice, with its normal once as it is
+// (normal) and once turned outward (normal_alt): 62 values and six neighbour ids
+// per cell.  Both cells of a face compute its normal, area and alpha from the same
+// vertices in the same order, so the values are the same bits up to the normal's
+// sign (cells are checked not to be tangled): one normal along +axis, one area and
+// one alpha per face, three faces per cell, serve both.  The face enters the lower
+// cell's sums with a plus and the upper cell's with a minus sign, which rounds like
+// the array form from either side; sums run over the slots in the array form's
+// order, no product is left out, so the results are its bits for any operand.
+// What bounds these kernels is the geometry still read, 16 values per cell for the
+// Laplacian (FP64 80 x 72 x 66: 49 MB, from L2; array kernels 18, 36 and 90 us for
+// gradient, Laplacian and stabilisation).
+
+template <class R> struct Vert {
+  int nx, ny, nz;
+  unsigned plane;
+  int groups;
+  unsigned tiles, chunks;
+  const R* nrm[3][3];  // axis, component: unit normal along +axis
+  const R* area[3];
+  const R* alpha[3];
+  const R* len[6];     // |x_f - x_P| by slot, per cell
+  const R* vol;
+  // the face below cell (x, y, z) along each axis; the one above is a step further
+  __device__ int64_t face(int axis, int x, int y, int z) const {
+    return axis == 0 ? (int64_t(x) * ny + y) * nz + z : axis == 1 ? (int64_t(x) * (ny + 1) + y) * nz + z
+                                                                  : (int64_t(x) * ny + y) * (nz + 1) + z;
+  }
+};
+
+// a[d] = fl(a[d] / v), any dividends
+template <class R> __device__ __forceinline__ void divide_any(R a[3], R v) {
+  const Volume<R> V{v, R(1) / v};
+  R q[3] = {a[0], a[1], a[2]};
+  V.template divide<3>(q);
+  if (finite((q[0] + q[1]) + q[2])) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) a[d] = q[d];
+  } else {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) a[d] = a[d] / v;
+  }
+}
+
+enum { OUT_SUM = 0, OUT_GRADIENT = 1 };
+
+// Gradient (OP_GRAD) or Laplacian (OP_LAPL, OP_HEAT) of every cell; OUT_GRADIENT
+// stores the three gradient components (arrays of n) instead of their masked sum.
+template <class R, int OP, int OUT>
+__global__ void __launch_bounds__(128) vert_sum_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
+                                                  R* __restrict__ out, int mask, R k, R dt) {
+  March<1, 1, 1> w;
+  if (!w.start(g)) return;
+  const int64_t pl = g.plane, n = int64_t(g.nx) * pl;
+  const int y = w.y0, z = w.z;
+  // F[d] = (face value n_d) A between the lower and the upper cell
+  auto face = [&](int axis, int64_t f, R lo, R hi, R F[3]) __attribute__((always_inline)) {
+    R v;
+    if constexpr (OP == OP_GRAD) v = (lo + hi) * R(0.5);
+    else v = (hi - lo) * g.alpha[axis][f];
+    const R A = g.area[axis][f];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) F[d] = (v * g.nrm[axis][d][f]) * A;
+  };
+  const R* q = phi + w.x0 * pl;
+  R P = q[w.off[1]], Fx[3];
+  face(0, g.face(0, w.x0, y, z), q[w.off[1] - (w.x0 > 0 ? pl : 0)], P, Fx);
+  for (int x = w.x0; x < w.x1; ++x, q += pl) {
+    const R N = q[w.off[1] + (x < g.nx - 1 ? pl : 0)];
+    const R below = q[w.off[0]], above = q[w.off[2]];
+    const int64_t i = x * pl + w.off[1];
+    const R V = g.vol[i];
+    R Fh[3], Fyl[3], Fyh[3], Fzl[3], Fzh[3];
+    face(0, g.face(0, x + 1, y, z), P, N, Fh);
+    const int64_t fy = g.face(1, x, y, z), fz = g.face(2, x, y, z);
+    face(1, fy, below, P, Fyl);
+    face(1, fy + g.nz, P, above, Fyh);
+    const R zp = __shfl_down_sync(kWarp, P, 1);
+    face(2, fz + 1, P, w.zhi ? P : zp, Fzh);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) Fzl[d] = __shfl_up_sync(kWarp, Fzh[d], 1);
+    if (w.zlo) face(2, fz, P, P, Fzl);
+    R acc[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) acc[d] = (((((R(0) - Fzl[d]) + Fzh[d]) - Fyl[d]) + Fyh[d]) - Fx[d]) + Fh[d];
+    divide_any(acc, V);
+    if (w.out) {
+      if constexpr (OUT == OUT_GRADIENT) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) out[d * n + i] = acc[d];
+      } else {
+        R res = R(0);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+          if (mask & (1 << d)) res = res + acc[d];
+        out[i] = OP == OP_HEAT ? dt * (k * res) + P : res;
+      }
+    }
+    P = N;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) Fx[d] = Fh[d];
+  }
+}
+
+// StabVar's second stage from the cell gradients (grad: three arrays of n): with
+// up = phi + (len g) n on a face's lower side and um = phi + (len g) (-n) on its
+// upper side, the face carries E = ((0.5 (up_L - um_H)) n) A.  On a wall the other
+// side is the cell's own value on its opposite face (the reference's ids point
+// back to the cell).
+template <class R>
+__global__ void __launch_bounds__(128) vert_stab_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
+                                                   const R* __restrict__ grad, R* __restrict__ out, int mask) {
+  March<1, 1, 1> w;
+  if (!w.start(g)) return;
+  const int64_t pl = g.plane, n = int64_t(g.nx) * pl;
+  const int y = w.y0, z = w.z;
+  struct Side {
+    R phi, g[3];
+  };
+  auto at = [&](int64_t i) __attribute__((always_inline)) {
+    return Side{phi[i], {grad[i], grad[n + i], grad[2 * n + i]}};
+  };
+  struct Normal {
+    R n[3], A;
+  };
+  auto normal = [&](int axis, int64_t f) __attribute__((always_inline)) {
+    return Normal{{g.nrm[axis][0][f], g.nrm[axis][1][f], g.nrm[axis][2][f]}, g.area[axis][f]};
+  };
+  auto up = [](const Side& s, R len, const Normal& m, int d) { return s.phi + (len * s.g[d]) * m.n[d]; };
+  auto um = [](const Side& s, R len, const Normal& m, int d) { return s.phi + (len * s.g[d]) * -m.n[d]; };
+  auto edge = [](R lo, R hi, const Normal& m, int d) { return ((R(0.5) * (lo - hi)) * m.n[d]) * m.A; };
+  Side P = at(w.x0 * pl + w.off[1]);
+  Normal mx = normal(0, g.face(0, w.x0, y, z));  // the x face below
+  R Ex[3];
+  if (w.x0 > 0) {
+    const int64_t j = (w.x0 - 1) * pl + w.off[1];
+    const Side B = at(j);
+    const R lb = g.len[5][j], la = g.len[4][j + pl];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) Ex[d] = edge(up(B, lb, mx, d), um(P, la, mx, d), mx, d);
+  }
+  for (int x = w.x0; x < w.x1; ++x) {
+    const int64_t i = x * pl + w.off[1];
+    const bool xlo = x == 0, xhi = x == g.nx - 1, ylo = y == 0, yhi = y == g.ny - 1;
+    R l[6];
+#pragma unroll
+    for (int f = 0; f < 6; ++f) l[f] = g.len[f][i];
+    R acc[3];
+    {  // z: faces 0 and 1
+      const int64_t f = g.face(2, x, y, z);
+      const Normal mh = normal(2, f + 1);
+      Side H;
+      H.phi = __shfl_down_sync(kWarp, P.phi, 1);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) H.g[d] = __shfl_down_sync(kWarp, P.g[d], 1);
+      const R lh = __shfl_down_sync(kWarp, l[0], 1);
+      const bool wall = w.zlo || w.zhi;
+      Normal ml = mh;
+      if (wall) ml = normal(2, f);  // the cell's lower face
+      R Eh[3], El[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        Eh[d] = edge(up(P, l[1], mh, d), w.zhi ? um(P, l[0], ml, d) : um(H, lh, mh, d), mh, d);
+        El[d] = __shfl_up_sync(kWarp, Eh[d], 1);
+        if (w.zlo) El[d] = edge(up(P, l[1], mh, d), um(P, l[0], ml, d), ml, d);
+        acc[d] = (R(0) - El[d]) + Eh[d];
+      }
+    }
+    {  // y: faces 2 and 3
+      const int64_t f = g.face(1, x, y, z);
+      const Normal ml = normal(1, f), mh = normal(1, f + g.nz);
+      const Side B = at(x * pl + w.off[0]), H = at(x * pl + w.off[2]);
+      const R lb = g.len[3][x * pl + w.off[0]], lh = g.len[2][x * pl + w.off[2]];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const R upP = up(P, l[3], mh, d), umP = um(P, l[2], ml, d);
+        const R El = edge(ylo ? upP : up(B, lb, ml, d), umP, ml, d);
+        const R Eh = edge(upP, yhi ? umP : um(H, lh, mh, d), mh, d);
+        acc[d] = (acc[d] - El) + Eh;
+      }
+    }
+    {  // x: faces 4 and 5
+      const Normal mh = normal(0, g.face(0, x + 1, y, z));
+      const int64_t j = i + (xhi ? 0 : pl);
+      const Side N = at(j);
+      const R ln = g.len[4][j];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const R upP = up(P, l[5], mh, d), umP = um(P, l[4], mx, d);
+        if (xlo) Ex[d] = edge(upP, umP, mx, d);
+        const R Eh = edge(upP, xhi ? umP : um(N, ln, mh, d), mh, d);
+        acc[d] = (acc[d] - Ex[d]) + Eh;
+        Ex[d] = Eh;
+      }
+      P = N;
+      mx = mh;
+    }
+    divide_any(acc, g.vol[i]);
+    if (w.out) {
+      R res = R(0);
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (mask & (1 << d)) res = res + acc[d];
+      out[i] = res;
+    }
+  }
+}
+
 // ---- the acoustic step (wave_plain_k) --------------------------------------------
 
 template <class R> struct WaveArgs {
@@ -707,21 +917,28 @@ __global__ void __launch_bounds__(kThreads) box_volume_k(int nx, int ny, int nz,
   if (other) atomicOr(differs, 1);
 }
 
+// Warps of a march over `groups` row groups: tiles of 32 - 2 HZ lanes along
+// (group, z), x cut into chunks for about 32 warps per SM (one wave at 64
+// registers; 24 and 48 measured within 10 %), each at least two planes long: a
+// chunk evaluates the face below it a second time.
+void march_grid(const cfdb_ctx* ctx, const cfdb_mesh* m, int HZ, int threads, unsigned* tiles, unsigned* chunks, unsigned* blocks,
+                int64_t groups = 0) {
+  const int64_t lanes = (groups ? groups : m->ny) * m->nz;
+  *tiles = unsigned((lanes + 32 - 2 * HZ - 1) / (32 - 2 * HZ));
+  const int64_t want = std::max<int64_t>(1, int64_t(ctx->num_sms) * 32 / *tiles);
+  *chunks = unsigned(std::min<int64_t>(std::min(want, int64_t(m->nx)), std::max<int64_t>(1, m->nx / 2)));
+  *blocks = unsigned((int64_t(*tiles) * *chunks * 32 + threads - 1) / threads);
+}
+
 // Kernel arguments for NY rows per thread, HZ halo lanes and blocks of
-// `threads`; *blocks = the grid.  x is cut into chunks for about 32 warps per
-// SM (one wave at 64 registers; 24 and 48 measured within 10 %), each at least
-// two planes long: a chunk evaluates the face below it a second time.
+// `threads`; *blocks = the grid.
 template <class R> Box<R> box_of(const cfdb_ctx* ctx, const cfdb_mesh* m, int NY, int HZ, int threads, unsigned* blocks) {
   const BoxGeomDev& b = m->box[sizeof(R) == 8 ? 1 : 0];
   Box<R> g;
   g.nx = int(m->nx); g.ny = int(m->ny); g.nz = int(m->nz);
   g.plane = unsigned(m->ny * m->nz);
   g.groups = int((m->ny + NY - 1) / NY);
-  const int64_t lanes = int64_t(g.groups) * m->nz;
-  g.tiles = unsigned((lanes + 32 - 2 * HZ - 1) / (32 - 2 * HZ));
-  const int64_t want = std::max<int64_t>(1, int64_t(ctx->num_sms) * 32 / g.tiles);
-  g.chunks = unsigned(std::min<int64_t>(std::min(want, int64_t(m->nx)), std::max<int64_t>(1, m->nx / 2)));
-  *blocks = unsigned((int64_t(g.tiles) * g.chunks * 32 + threads - 1) / threads);
+  march_grid(ctx, m, HZ, threads, &g.tiles, &g.chunks, blocks, g.groups);
   g.hx = b.h[0]; g.hy = b.h[1]; g.hz = b.h[2];
   auto t = [](const void* p) { return static_cast<const R*>(p); };
   g.ax = t(b.alpha[0]); g.ay = t(b.alpha[1]); g.az = t(b.alpha[2]);
@@ -840,6 +1057,23 @@ int build_box(cfdb_mesh* m, BoxGeomDev& b) {
   return CFDB_OK;
 }
 
+template <class R> Vert<R> vert_of(const cfdb_ctx* ctx, const cfdb_mesh* m, unsigned* blocks) {
+  const FaceGeomDev& b = m->faces[sizeof(R) == 8 ? 1 : 0];
+  Vert<R> g;
+  g.nx = int(m->nx); g.ny = int(m->ny); g.nz = int(m->nz);
+  g.plane = unsigned(m->ny * m->nz);
+  g.groups = g.ny;
+  march_grid(ctx, m, 1, 128, &g.tiles, &g.chunks, blocks);
+  for (int a = 0; a < 3; ++a) {
+    for (int d = 0; d < 3; ++d) g.nrm[a][d] = static_cast<const R*>(b.normal[a]) + d * b.count[a];
+    g.area[a] = static_cast<const R*>(b.area[a]);
+    g.alpha[a] = static_cast<const R*>(b.alpha[a]);
+  }
+  for (int f = 0; f < 6; ++f) g.len[f] = static_cast<const R*>(b.len) + f * m->n;
+  g.vol = static_cast<const R*>(b.vol);
+  return g;
+}
+
 }  // namespace
 
 int cfdb_mesh_need_box(cfdb_mesh* m, int dtype, bool* usable) {
@@ -927,4 +1161,45 @@ int box_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* q
                   double dt) {
   return dtype == CFDB_F64 ? launch_wave<double>(ctx, m, q, qn, c, cconst, mode, dt)
                            : launch_wave<float>(ctx, m, q, qn, c, cconst, mode, dt);
+}
+
+template <class R, int OP, int OUT>
+int launch_vert_sum(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask, double k, double dt) {
+  unsigned blocks = 0;
+  const Vert<R> g = vert_of<R>(ctx, m, &blocks);
+  vert_sum_k<R, OP, OUT><<<blocks, 128, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
+  CFDB_LAUNCHED(ctx);
+  return CFDB_OK;
+}
+
+int vert_grad(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
+  return dtype == CFDB_F64 ? launch_vert_sum<double, OP_GRAD, OUT_SUM>(ctx, m, phi, out, mask, 0, 0)
+                           : launch_vert_sum<float, OP_GRAD, OUT_SUM>(ctx, m, phi, out, mask, 0, 0);
+}
+
+int vert_lapl(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
+  return dtype == CFDB_F64 ? launch_vert_sum<double, OP_LAPL, OUT_SUM>(ctx, m, phi, out, mask, 0, 0)
+                           : launch_vert_sum<float, OP_LAPL, OUT_SUM>(ctx, m, phi, out, mask, 0, 0);
+}
+
+int vert_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* Tn, double k, double dt) {
+  return dtype == CFDB_F64 ? launch_vert_sum<double, OP_HEAT, OUT_SUM>(ctx, m, T, Tn, 7, k, dt)
+                           : launch_vert_sum<float, OP_HEAT, OUT_SUM>(ctx, m, T, Tn, 7, k, dt);
+}
+
+template <class R> int launch_vert_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask) {
+  FaceGeomDev& b = m->faces[sizeof(R) == 8 ? 1 : 0];
+  if (!b.grad)
+    if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(R)) * 3 * m->n, &b.grad)) return rc;
+  if (int rc = launch_vert_sum<R, OP_GRAD, OUT_GRADIENT>(ctx, m, phi, b.grad, 7, 0, 0)) return rc;
+  unsigned blocks = 0;
+  const Vert<R> g = vert_of<R>(ctx, m, &blocks);
+  vert_stab_k<R><<<blocks, 128, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<const R*>(b.grad),
+                                                  static_cast<R*>(out), mask);
+  CFDB_LAUNCHED(ctx);
+  return CFDB_OK;
+}
+
+int vert_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
+  return dtype == CFDB_F64 ? launch_vert_stab<double>(ctx, m, phi, out, mask) : launch_vert_stab<float>(ctx, m, phi, out, mask);
 }

@@ -76,6 +76,21 @@ struct BoxGeomDev {
   double uA[3] = {}, ual[3] = {}, ulm[3] = {}, ulp[3] = {};
 };
 
+// Geometry of a vertex mesh with every face held once (box_ops.cu), in one
+// precision: per axis the faces' unit normals along +axis (3 count), areas and
+// alphas (count each; the face below cell i along its axis is entry i, one more
+// entry than cells), per cell the six |x_f - x_P| (slot after slot) and the volume.
+struct FaceGeomDev {
+  int state = 0;  // 0 not built, 1 usable, 2 this mesh keeps the N x 6 arrays
+  int64_t count[3] = {};
+  void* normal[3] = {};
+  void* area[3] = {};
+  void* alpha[3] = {};
+  void* len = nullptr;
+  void* vol = nullptr;
+  void* grad = nullptr;  // 3 n, allocated on the first stab call
+};
+
 // Compact FP32 geometry of vertex meshes for the fused kernels: per cell the
 // outward area vector of its +x/+y/+z face and 1/V (10 fields), stored on
 // the lattice padded by one ghost layer below each axis (x and y) and by four
@@ -177,6 +192,7 @@ struct cfdb_mesh {
   PlainGeomDev plain[2];
   CompactGeomDev compact;
   BoxGeomDev box[2];  // structured meshes, by precision
+  FaceGeomDev faces[2];  // vertex meshes, by precision
   int lattice_state = 0;  // 0 not checked, 1 exact lattice, 2 not one
   cfdb_lattice_geometry lattice{};
 };
@@ -275,6 +291,14 @@ int box_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* T
 int box_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* qn, const void* c, double cconst, int mode,
                   double dt);
 int box_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask);
+// The same on vertex meshes with every face's geometry held once.  *usable =
+// false: this mesh takes the array kernels.
+int cfdb_mesh_need_faces(cfdb_mesh* m, int dtype, bool* usable);
+int cfdb_build_faces_device(cfdb_mesh* m, int dtype, FaceGeomDev& b);  // geometry_dev.cu
+int vert_grad(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask);
+int vert_lapl(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask);
+int vert_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* Tn, double k, double dt);
+int vert_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask);
 // fused_tma.cu
 int fused_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* Tn, double k, double dt,
                     const void* fixed = nullptr);

@@ -91,6 +91,86 @@ int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p) {
   return CFDB_OK;
 }
 
+// ---- every face once ---------------------------------------------------------
+namespace {
+
+template <class T> struct FaceArrays {
+  T* normal[3];
+  T* area[3];
+  T* alpha[3];
+  int64_t count[3];
+  T* len;
+  T* vol;
+};
+
+// A cell stores its upper faces, and its lower ones where they are walls; both
+// cells of a face compute the same values (geometry_cell.hpp: the same corners in
+// the same order, alpha from centre distances that differ in sign only).
+template <class T>
+__global__ void __launch_bounds__(128) face_geometry_k(Lattice L, int mode, FaceArrays<T> a) {
+  const int64_t n = L.nx * L.ny * L.nz, plane = L.ny * L.nz;
+  auto center_of = [&](int64_t x, int64_t y, int64_t z) { return L.center(x, y, z); };
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t x = i / plane, r = i - x * plane, y = r / L.nz, z = r - y * L.nz;
+    bool bnd = false;
+    auto store = [&](int f, const CellFace& o) {
+      a.len[f * n + i] = T(o.len);
+      const int axis = 2 - f / 2, up = f & 1;
+      const int64_t at = axis == 0 ? x : axis == 1 ? y : z;
+      if (!up && at > 0) return;
+      const int64_t k = axis == 0 ? ((x + up) * L.ny + y) * L.nz + z
+                      : axis == 1 ? (x * (L.ny + 1) + y + up) * L.nz + z : (x * L.ny + y) * (L.nz + 1) + z + up;
+      a.normal[axis][k] = T(o.uns.x);
+      a.normal[axis][a.count[axis] + k] = T(o.uns.y);
+      a.normal[axis][2 * a.count[axis] + k] = T(o.uns.z);
+      a.area[axis][k] = T(o.area);
+      a.alpha[axis][k] = T(o.alpha);
+    };
+    a.vol[i] = T(cfdb_geom::cell_geometry(L, x, y, z, mode, center_of, store, &bnd));
+  }
+}
+
+template <class T> int build_faces(cfdb_mesh* m, FaceGeomDev& b) {
+  cfdb_ctx* ctx = m->ctx;
+  b.count[0] = (m->nx + 1) * m->ny * m->nz;
+  b.count[1] = m->nx * (m->ny + 1) * m->nz;
+  b.count[2] = m->nx * m->ny * (m->nz + 1);
+  FaceArrays<T> a{};
+  for (int d = 0; d < 3; ++d) {
+    const int64_t bytes = int64_t(sizeof(T)) * b.count[d];
+    if (int rc = cfdb_dev_alloc(ctx, 3 * bytes, &b.normal[d])) return rc;
+    if (int rc = cfdb_dev_alloc(ctx, bytes, &b.area[d])) return rc;
+    if (int rc = cfdb_dev_alloc(ctx, bytes, &b.alpha[d])) return rc;
+    a.normal[d] = static_cast<T*>(b.normal[d]);
+    a.area[d] = static_cast<T*>(b.area[d]);
+    a.alpha[d] = static_cast<T*>(b.alpha[d]);
+    a.count[d] = b.count[d];
+  }
+  if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(T)) * 6 * m->n, &b.len)) return rc;
+  if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(T)) * m->n, &b.vol)) return rc;
+  a.len = static_cast<T*>(b.len);
+  a.vol = static_cast<T*>(b.vol);
+  void* dverts = nullptr;
+  const int64_t vb = int64_t(sizeof(double)) * int64_t(m->verts.size());
+  if (int rc = cfdb_dev_alloc(ctx, vb, &dverts)) return rc;
+  cudaError_t e = cudaMemcpyAsync(dverts, m->verts.data(), size_t(vb), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) {
+    const Lattice L{m->nx, m->ny, m->nz, m->dx, m->dy, m->dz, static_cast<const double*>(dverts)};
+    face_geometry_k<T><<<unsigned(grid_for(ctx, m->n, 128, 16)), 128, 0, ctx->stream>>>(L, m->geom_mode, a);
+    ++ctx->launches;
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  cfdb_dev_free(ctx, dverts);
+  return e == cudaSuccess ? CFDB_OK : cfdb_cuda_fail(ctx, e, "face geometry");
+}
+
+}  // namespace
+
+int cfdb_build_faces_device(cfdb_mesh* m, int dtype, FaceGeomDev& b) {
+  return dtype == CFDB_F64 ? build_faces<double>(m, b) : build_faces<float>(m, b);
+}
+
 // ---- exact lattices --------------------------------------------------------
 namespace {
 

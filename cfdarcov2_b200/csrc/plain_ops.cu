@@ -503,15 +503,21 @@ __global__ void wave_adjoint_plain_k(PlainArgs<R> g, const R* __restrict__ q, co
   }
 }
 
-// Checks a mesh operator's handles; with `box` given, builds the tables of a
-// structured mesh (*box = true) instead of the face arrays where they serve.
-int need(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, bool* box = nullptr) {
+// Which geometry a mesh operator runs on.
+enum class Geom { Arrays, Box, Faces };
+
+// Checks a mesh operator's handles; with `geom` given, builds the tables of a
+// structured mesh or the faces of a vertex mesh instead of the N x 6 arrays where
+// they serve.
+int need(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, Geom* geom = nullptr) {
   if (int rc = cfdb_check_mesh(ctx, m)) return rc;
   if (!dtype_ok(dtype)) return cfdb_fail(ctx, CFDB_EINVAL, "unknown dtype %d", dtype);
   CFDB_CUDA(ctx, cudaSetDevice(ctx->device));
-  if (box) {
-    if (int rc = cfdb_mesh_need_box(m, dtype, box)) return rc;
-    if (*box) return CFDB_OK;
+  if (geom) {
+    bool usable = false;
+    if (int rc = m->uniform ? cfdb_mesh_need_box(m, dtype, &usable) : cfdb_mesh_need_faces(m, dtype, &usable)) return rc;
+    *geom = !usable ? Geom::Arrays : m->uniform ? Geom::Box : Geom::Faces;
+    if (usable) return CFDB_OK;
   }
   return cfdb_mesh_need_plain(m, dtype);
 }
@@ -554,11 +560,12 @@ int check_n(cfdb_ctx* ctx, int dtype, int64_t n, const char* fn) {
   }
 
 extern "C" int cfdb_op_grad(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
-  bool box = false;
-  if (int rc = need(ctx, m, dtype, &box)) return rc;
+  Geom geom = Geom::Arrays;
+  if (int rc = need(ctx, m, dtype, &geom)) return rc;
   if (int rc = check_ptrs(ctx, "cfdb_op_grad", {phi, out})) return rc;
   if (mask < 0 || mask > 7) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_op_grad: dims_mask %d out of range", mask);
-  if (box) return box_grad(ctx, m, dtype, phi, out, mask);
+  if (geom == Geom::Box) return box_grad(ctx, m, dtype, phi, out, mask);
+  if (geom == Geom::Faces) return vert_grad(ctx, m, dtype, phi, out, mask);
   const int grid = grid_for(ctx, m->n, kThreads);
   DISPATCH(dtype, R, grad_k<R><<<grid, kThreads, 0, ctx->stream>>>(plain_args<R>(m, dtype), (const R*)phi, (R*)out, mask));
   CFDB_LAUNCHED(ctx);
@@ -573,20 +580,22 @@ int plain_lapl(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* ou
 }
 
 extern "C" int cfdb_op_lapl(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
-  bool box = false;
-  if (int rc = need(ctx, m, dtype, &box)) return rc;
+  Geom geom = Geom::Arrays;
+  if (int rc = need(ctx, m, dtype, &geom)) return rc;
   if (int rc = check_ptrs(ctx, "cfdb_op_lapl", {phi, out})) return rc;
   if (mask < 0 || mask > 7) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_op_lapl: dims_mask %d out of range", mask);
-  if (box) return box_lapl(ctx, m, dtype, phi, out, mask);
+  if (geom == Geom::Box) return box_lapl(ctx, m, dtype, phi, out, mask);
+  if (geom == Geom::Faces) return vert_lapl(ctx, m, dtype, phi, out, mask);
   return plain_lapl(ctx, m, dtype, phi, out, mask);
 }
 
 extern "C" int cfdb_op_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
-  bool box = false;
-  if (int rc = need(ctx, m, dtype, &box)) return rc;
+  Geom geom = Geom::Arrays;
+  if (int rc = need(ctx, m, dtype, &geom)) return rc;
   if (int rc = check_ptrs(ctx, "cfdb_op_stab", {phi, out})) return rc;
   if (mask < 0 || mask > 7) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_op_stab: dims_mask %d out of range", mask);
-  if (box) return box_stab(ctx, m, dtype, phi, out, mask);
+  if (geom == Geom::Box) return box_stab(ctx, m, dtype, phi, out, mask);
+  if (geom == Geom::Faces) return vert_stab(ctx, m, dtype, phi, out, mask);
   PlainGeomDev& p = m->plain[dtype == CFDB_F64 ? 1 : 0];
   if (!p.stab_tmp)
     if (int rc = cfdb_dev_alloc(ctx, int64_t(dtype_size(dtype)) * 18 * m->n, &p.stab_tmp)) return rc;
@@ -745,8 +754,13 @@ extern "C" int cfdb_total_fp64(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const voi
   CFDB_CUDA(ctx, cudaSetDevice(ctx->device));
   const void* vol = nullptr;
   if (!m->uniform) {
-    if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
-    vol = m->plain[dtype == CFDB_F64 ? 1 : 0].volume;
+    bool faces = false;  // either geometry holds the volumes
+    const int p = dtype == CFDB_F64 ? 1 : 0;
+    if (!m->plain[p].ready)
+      if (int rc = cfdb_mesh_need_faces(m, dtype, &faces)) return rc;
+    if (!faces)
+      if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
+    vol = faces ? m->faces[p].vol : m->plain[p].volume;
   }
   const double vconst = m->dx * m->dy * m->dz;
   const bool vec = aligned16({field, vol});

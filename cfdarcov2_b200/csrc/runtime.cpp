@@ -498,6 +498,18 @@ extern "C" int cfdb_mesh_create_from_vertices(cfdb_ctx* ctx, int64_t nx, int64_t
   return CFDB_OK;
 }
 
+static void free_faces(cfdb_ctx* ctx, FaceGeomDev& b) {
+  for (int d = 0; d < 3; ++d) {
+    cfdb_dev_free(ctx, b.normal[d]);
+    cfdb_dev_free(ctx, b.area[d]);
+    cfdb_dev_free(ctx, b.alpha[d]);
+  }
+  cfdb_dev_free(ctx, b.len);
+  cfdb_dev_free(ctx, b.vol);
+  cfdb_dev_free(ctx, b.grad);
+  b = FaceGeomDev();
+}
+
 static void free_plain(cfdb_ctx* ctx, PlainGeomDev& p) {
   void** ptrs[] = {&p.normal, &p.normal_alt, &p.area, &p.alpha, &p.len, &p.volume, &p.isb, &p.stab_tmp};
   for (void** q : ptrs) {
@@ -516,6 +528,8 @@ void cfdb_mesh_orphan(cfdb_mesh* m) {
   m->compact = CompactGeomDev();
   m->box[0] = BoxGeomDev();
   m->box[1] = BoxGeomDev();
+  m->faces[0] = FaceGeomDev();
+  m->faces[1] = FaceGeomDev();
 }
 
 extern "C" int cfdb_mesh_destroy(cfdb_mesh* m) {
@@ -527,6 +541,7 @@ extern "C" int cfdb_mesh_destroy(cfdb_mesh* m) {
     free_plain(m->ctx, m->plain[1]);
     cfdb_dev_free(m->ctx, m->d_ids);
     cfdb_dev_free(m->ctx, m->compact.S);
+    for (FaceGeomDev& b : m->faces) free_faces(m->ctx, b);
     for (BoxGeomDev& b : m->box) {
       cfdb_dev_free(m->ctx, b.tab);
       cfdb_dev_free(m->ctx, b.vol);
@@ -617,6 +632,30 @@ int cfdb_mesh_need_plain(cfdb_mesh* m, int dtype) {
     return rc;
   }
   p.ready = true;
+  return CFDB_OK;
+}
+
+int cfdb_mesh_need_faces(cfdb_mesh* m, int dtype, bool* usable) {
+  FaceGeomDev& b = m->faces[dtype == CFDB_F64 ? 1 : 0];
+  *usable = false;
+  if (m->uniform) return CFDB_OK;
+  if (b.state == 0) {
+    // the sums are divided by the volume's reciprocal (box_ops.cu), which wants
+    // volumes far from the ends of the storage type's range
+    if (int rc = cfdb_mesh_need_host_geom(m)) return rc;
+    const auto ext = std::minmax_element(m->geom->volume.begin(), m->geom->volume.end());
+    if (!(*ext.first > 0x1p-79) || !(*ext.second < 0x1p23)) {
+      b.state = 2;
+    } else {
+      CFDB_CUDA(m->ctx, cudaSetDevice(m->ctx->device));
+      if (int rc = cfdb_build_faces_device(m, dtype, b)) {
+        free_faces(m->ctx, b);
+        return rc;
+      }
+      b.state = 1;
+    }
+  }
+  *usable = b.state == 1;
   return CFDB_OK;
 }
 

@@ -24,6 +24,9 @@ extern "C" int cfdb_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int path, 
   bool box = false;
   if (int rc = cfdb_mesh_need_box(m, dtype, &box)) return rc;
   if (box) return box_heat_step(ctx, m, dtype, T, Tn, k, dt);
+  bool faces = false;
+  if (int rc = cfdb_mesh_need_faces(m, dtype, &faces)) return rc;
+  if (faces) return vert_heat_step(ctx, m, dtype, T, Tn, k, dt);
   if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
   PlainGeomDev& p = m->plain[dtype == CFDB_F64 ? 1 : 0];
   if (!p.stab_tmp)

@@ -79,3 +79,36 @@ def test_operators_on_values_that_are_not_finite(cfdb, ctx, shape, spacing, dtyp
             ctx.wave_step(k, q, o, 1e-4, c_const=0.9, path=cfdb.PLAIN)
         assert torch.equal(torch.isnan(out[0]), torch.isnan(out[1])), value
         assert torch.equal(torch.nan_to_num(out[0], nan=0.0), torch.nan_to_num(out[1], nan=0.0)), value
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 3, 5), (17, 9, 33), (40, 31, 62)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_faces_held_once_equal_the_face_arrays(cfdb, ctx, shape, dtype):
+    """Vertex meshes with every face's geometry held once against the N x 6
+    arrays: the same jittered mesh scaled by 2^-30 has volumes outside the
+    range of the reciprocal division and keeps the arrays, and every result
+    scales by an exact power of two."""
+    rng = np.random.default_rng(9)
+    h = 1.0 / 64
+    ax = [np.arange(n + 1) * h for n in shape]
+    v = np.stack(np.meshgrid(*ax, indexing="ij"), -1)
+    v += rng.uniform(-0.2, 0.2, v.shape) * h
+    s = 2.0 ** -30
+    m = cfdb.Mesh.from_vertices(ctx, *shape, h, h, h, v)
+    a = cfdb.Mesh.from_vertices(ctx, *shape, h * s, h * s, h * s, v * s)
+    for bad in (None, float("inf"), float("nan")):
+        phi = field(m.n, dtype, 6)
+        if bad is not None:
+            phi[m.n // 2] = bad
+        for op, scale in (("grad", s), ("lapl", s * s), ("stab", s)):
+            for mask in (7, 1, 6, 0):
+                got = getattr(ctx, op)(m, phi, mask=mask)
+                ref = getattr(ctx, op)(a, phi, mask=mask) * scale
+                assert torch.equal(torch.isnan(got), torch.isnan(ref)), (op, mask, bad)
+                assert torch.equal(torch.nan_to_num(got, nan=0.0), torch.nan_to_num(ref, nan=0.0)), (op, mask, bad)
+    phi = field(m.n, dtype, 7)
+    out = [torch.empty_like(phi) for _ in range(2)]
+    ctx.heat_step(m, phi, out[0], 0.7, 1e-5, path=cfdb.PLAIN)
+    ctx.heat_step(a, phi, out[1], 0.7, 1e-5 * s * s, path=cfdb.PLAIN)
+    assert torch.equal(*out)
+    assert ctx.total_fp64(m, phi) == pytest.approx(ctx.total_fp64(a, phi) / s ** 3, rel=1e-12)
