@@ -4,6 +4,7 @@
 // epilogue, reduces the new state's per-direction signal speeds (for the next
 // dt) and its FP64 Neumaier totals.  The plain path lives in euler_plain.cu.
 #include <cmath>
+#include <cstring>
 #include <new>
 
 #include "euler_internal.hpp"
@@ -253,13 +254,33 @@ struct EulerPhys {
   }
 };
 
-// The fold of the partials the last launch left, for a reader of the totals
-// after the last step (cfdb_euler_totals, the run loop's health check).
-__global__ void euler_fold_k(EulerClock* ck, const Comp2* __restrict__ part, int stride, int nblocks,
-                             double* totals, int prev) {
-  const long long step = ck->pending[prev];
-  if (step <= 0) return;
-  fold_partials(part + size_t(prev) * size_t(stride), nblocks, totals, step);
+// What the host reads of a solver, stored to page-locked memory by one launch
+// (a check had cost four copies and as many waits, about 45 us; one launch and one
+// wait take 12).
+struct EulerReport {
+  double t, mass, energy;  // clock, totals of the latest step
+  long long steps;
+  int finished, error;
+};
+static_assert(sizeof(EulerReport) <= 64, "one slot of the context's page-locked words");
+
+// With prev >= 0, first the fold of the partials the last fused launch left (a
+// no-op when a later launch folded them, or it did not step).
+__global__ void euler_report_k(const EulerClock* ck, const Comp2* __restrict__ part, int stride, int nblocks, double* totals,
+                               int prev, int slot, const int* err, EulerReport* out) {
+  if (prev >= 0) {
+    const long long step = ck->pending[prev];
+    if (step > 0) fold_partials(part + size_t(prev) * size_t(stride), nblocks, totals, step);
+  }
+  if (threadIdx.x == 0) {
+    const long long steps = ck->steps[slot];
+    out->t = ck->t[slot];
+    out->steps = steps;
+    out->finished = ck->finished[slot];
+    out->error = *err;
+    out->mass = totals[2 * steps];
+    out->energy = totals[2 * steps + 1];
+  }
 }
 
 constexpr int kEulerCtasPerSm = 2;
@@ -310,16 +331,21 @@ int euler_fused_grid(const cfdb_euler* e) {
   return sh.tiles * sh.chunks;
 }
 
-// Folds the partials the last fused launch left into its totals row (a
-// no-op when that launch already had its totals folded by a later one, or
-// did not step).
-int euler_fold_pending(cfdb_euler* e) {
-  if (e->path != CFDB_PATH_FUSED || e->launches < 1 || e->fused_grid < 1) return CFDB_OK;
-  const int prev = int((e->launches - 1) & 1);
-  euler_fold_k<<<1, e->fused_threads, 0, e->ctx->stream>>>(e->clock, e->part, e->part_cap, e->fused_grid, e->totals,
-                                                          prev);
-  CFDB_LAUNCHED(e->ctx);
-  return CFDB_OK;
+// Synchronous; `fold` brings the totals up to the latest step.
+static int euler_report(cfdb_euler* e, bool fold, EulerReport* out) {
+  cfdb_ctx* ctx = e->ctx;
+  const bool pending = fold && e->path == CFDB_PATH_FUSED && e->launches >= 1 && e->fused_grid >= 1;
+  {
+    std::lock_guard<std::mutex> lock(ctx->reduce.mu);
+    EulerReport* host = static_cast<EulerReport*>(ctx->reduce.host);
+    euler_report_k<<<1, pending ? e->fused_threads : 32, 0, ctx->stream>>>(
+        e->clock, e->part, e->part_cap, e->fused_grid, e->totals, pending ? int((e->launches - 1) & 1) : -1,
+        euler_slot(e->launches), ctx->d_error, host);
+    CFDB_LAUNCHED(ctx);
+    CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    std::memcpy(out, host, sizeof(*out));
+  }
+  return out->error ? cfdb_check_device_error(ctx) : CFDB_OK;
 }
 
 int euler_fused_step(cfdb_euler* e, const void* U, void* Un, int64_t s) {
@@ -400,24 +426,20 @@ extern "C" int cfdb_euler_step(cfdb_euler* e, const void* U, void* Un) {
 
 extern "C" int cfdb_euler_status(cfdb_euler* e, double* t, int64_t* steps_done, int* finished) {
   if (!e || !e->ctx) return cfdb_fail(nullptr, CFDB_EINVAL, "cfdb_euler_status: handle is NULL or its context was destroyed");
-  EulerClock ck;
-  CFDB_CUDA(e->ctx, cudaMemcpyAsync(&ck, e->clock, sizeof(ck), cudaMemcpyDeviceToHost, e->ctx->stream));
-  CFDB_CUDA(e->ctx, cudaStreamSynchronize(e->ctx->stream));
-  if (int rc = cfdb_check_device_error(e->ctx)) return rc;
-  const int sl = euler_slot(e->launches);
-  if (t) *t = ck.t[sl];
-  if (steps_done) *steps_done = ck.steps[sl];
-  if (finished) *finished = ck.finished[sl];
+  EulerReport r;
+  if (int rc = euler_report(e, false, &r)) return rc;
+  if (t) *t = r.t;
+  if (steps_done) *steps_done = r.steps;
+  if (finished) *finished = r.finished;
   return CFDB_OK;
 }
 
 extern "C" int cfdb_euler_totals(cfdb_euler* e, double* out, int64_t max_rows, int64_t* rows) {
   if (!e || !e->ctx || !out || max_rows < 0)
     return cfdb_fail(e ? e->ctx : nullptr, CFDB_EINVAL, "cfdb_euler_totals: bad arguments");
-  int64_t steps = 0;
-  if (int rc = euler_fold_pending(e)) return rc;
-  if (int rc = cfdb_euler_status(e, nullptr, &steps, nullptr)) return rc;
-  const int64_t n = std::min<int64_t>(steps + 1, max_rows);
+  EulerReport r;
+  if (int rc = euler_report(e, true, &r)) return rc;
+  const int64_t n = std::min<int64_t>(r.steps + 1, max_rows);
   if (n > 0) CFDB_CUDA(e->ctx, cudaMemcpy(out, e->totals, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost));
   if (rows) *rows = n;
   return CFDB_OK;
@@ -432,21 +454,28 @@ extern "C" int cfdb_euler_run(cfdb_euler* e, void* Ua, void* Ub, int64_t check_e
   if (e->launches & 1) return cfdb_fail(e->ctx, CFDB_EINVAL, "cfdb_euler_run: call after cfdb_euler_begin or an even number of steps");
   int finished = 0;
   int64_t steps = 0;
+  // Steps enqueued before the next clock check: at most check_every, a first few
+  // to learn dt, then what the mean dt so far says is left.  A launch past t_end
+  // still costs 4 to 5 us (it has to run to find the clock finished), a check
+  // about 12.
+  int64_t batch = std::min<int64_t>(check_every, 16);
   while (!finished) {
-    for (int64_t k = 0; k < check_every; ++k) {
+    for (int64_t k = 0; k < batch; ++k) {
       const bool even = (e->launches & 1) == 0;
       if (int rc = cfdb_euler_step(e, even ? Ua : Ub, even ? Ub : Ua)) return rc;
     }
-    if (int rc = euler_fold_pending(e)) return rc;
-    if (int rc = cfdb_euler_status(e, nullptr, &steps, &finished)) return rc;
+    EulerReport r;
+    if (int rc = euler_report(e, true, &r)) return rc;
+    finished = r.finished;
+    steps = r.steps;
+    const double left = r.t > 0 ? std::ceil((e->t_end - r.t) / r.t * double(steps)) + 1.0 : double(check_every);
+    batch = left < double(check_every) ? std::max<int64_t>(1, int64_t(left)) : check_every;
     // the conservation totals of the latest step double as the health check:
     // a NaN or Inf anywhere in the state reaches them (and would otherwise
     // end the run early through a non-finite dt)
-    double last[2] = {0.0, 0.0};
-    CFDB_CUDA(e->ctx, cudaMemcpy(last, e->totals + 2 * steps, sizeof(last), cudaMemcpyDeviceToHost));
-    if (!std::isfinite(last[0]) || !std::isfinite(last[1]))
+    if (!std::isfinite(r.mass) || !std::isfinite(r.energy))
       return cfdb_fail(e->ctx, CFDB_ENUMERIC, "cfdb_euler_run: the state is not finite at step %lld (totals %g, %g)",
-                       (long long)steps, last[0], last[1]);
+                       (long long)steps, r.mass, r.energy);
     if (!finished && e->launches > e->max_steps + check_every)
       return cfdb_fail(e->ctx, CFDB_ENUMERIC, "cfdb_euler_run: the clock did not reach t_end within max_steps");
   }

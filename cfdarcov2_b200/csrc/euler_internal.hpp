@@ -9,7 +9,7 @@
 // FP64 Neumaier totals of the new state: the plain path's reduction launch
 // folds them itself (its last CTA); a fused launch leaves per-CTA partials
 // (buffer s%2) and records its step in pending[s%2], and the next launch, or
-// cfdb_euler_fold before the host reads the totals, folds them, so no launch
+// the report before the host reads the totals, folds them, so no launch
 // ends waiting for a fold.  Once t_end is reached every further launch only
 // copies the clock forward, so the host can enqueue steps without reading dt
 // back (the reference syncs and copies a scalar every step,
