@@ -261,6 +261,13 @@ int cfdb_register_module(const void* anchor_kernel);
 // ---- geometry helpers ------------------------------------------------------
 int cfdb_mesh_need_host_geom(cfdb_mesh* m);
 int cfdb_mesh_need_plain(cfdb_mesh* m, int dtype);
+// The geometry a per-operator kernel of dtype runs on, built where it is not yet.
+// All give the same bits: the tables of a structured mesh (box_ops.cu), a vertex
+// mesh's faces held once (vertex_faces: the operator has such a kernel), or the
+// N x 6 arrays.  Where the arrays are there already, they serve while the stream
+// records a graph; a failed allocation of the others falls back to them.
+enum class Geom { Arrays, Box, Faces };
+int cfdb_mesh_geometry(cfdb_mesh* m, int dtype, bool vertex_faces, Geom* geom);
 // fills the plain arrays of dtype on the device (geometry_dev.cu)
 int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p);
 // samples and checks the lattice constants on the device (geometry_dev.cu)

@@ -365,8 +365,8 @@ static int blocked_pass(cfdb_ctx* ctx, cfdb_mesh* m, const void* src, void* dst,
 // `steps` steps, the state alternating between Ta and Tb per pass, the last one
 // where the one-step sweep would have left it (Tb for odd `steps`); with
 // keep_other the buffer that does not receive the result is left as it was,
-// a workspace taking its part.  CFDB_EUNSUPPORTED (nothing launched) when the
-// mesh or the pointers are not what the TMA kernels take.
+// a workspace taking its part where one can be had.  CFDB_EUNSUPPORTED (nothing
+// launched) when the mesh or the pointers are not what the TMA kernels take.
 int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, double dt, int32_t steps, int use_graph,
                      bool keep_other) {
   if (steps < 1 || check_sweep(ctx, m, {Ta, Tb}) != CFDB_OK) return CFDB_EUNSUPPORTED;
@@ -380,6 +380,12 @@ int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, 
   int32_t n = (steps + most - 1) / most;
   if ((n ^ steps) & 1) ++n;
   const int per = int(steps / n), more = int(steps % n);  // the first `more` passes do per + 1
+  void* ws = nullptr;
+  if (keep_other && n > 1) {
+    const int rc = cfdb_ws_alloc(ctx, m->n * 4, &ws);
+    if (rc && rc != CFDB_ENOMEM) return rc;
+    keep_other = rc == CFDB_OK;
+  }
   if (!keep_other) {
     auto run = [&](void* a, void* b, int32_t passes, int each) {
       return cfdb_run_steps(
@@ -390,9 +396,6 @@ int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, 
       if (int rc = run(Ta, Tb, more, per + 1)) return rc;
     return (more & 1) ? run(Tb, Ta, n - more, per) : run(Ta, Tb, n - more, per);
   }
-  void* ws = nullptr;
-  if (n > 1)
-    if (int rc = cfdb_ws_alloc(ctx, m->n * 4, &ws)) return rc;
   void* const result = (steps & 1) ? Tb : Ta;
   const void* src = Ta;
   int rc = CFDB_OK;

@@ -503,23 +503,13 @@ __global__ void wave_adjoint_plain_k(PlainArgs<R> g, const R* __restrict__ q, co
   }
 }
 
-// Which geometry a mesh operator runs on.
-enum class Geom { Arrays, Box, Faces };
-
-// Checks a mesh operator's handles; with `geom` given, builds the tables of a
-// structured mesh or the faces of a vertex mesh instead of the N x 6 arrays where
-// they serve.
+// Checks a mesh operator's handles and builds the N x 6 arrays, or with `geom`
+// given whichever geometry serves.
 int need(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, Geom* geom = nullptr) {
   if (int rc = cfdb_check_mesh(ctx, m)) return rc;
   if (!dtype_ok(dtype)) return cfdb_fail(ctx, CFDB_EINVAL, "unknown dtype %d", dtype);
   CFDB_CUDA(ctx, cudaSetDevice(ctx->device));
-  if (geom) {
-    bool usable = false;
-    if (int rc = m->uniform ? cfdb_mesh_need_box(m, dtype, &usable) : cfdb_mesh_need_faces(m, dtype, &usable)) return rc;
-    *geom = !usable ? Geom::Arrays : m->uniform ? Geom::Box : Geom::Faces;
-    if (usable) return CFDB_OK;
-  }
-  return cfdb_mesh_need_plain(m, dtype);
+  return geom ? cfdb_mesh_geometry(m, dtype, true, geom) : cfdb_mesh_need_plain(m, dtype);
 }
 
 int check_ptrs(cfdb_ctx* ctx, const char* fn, std::initializer_list<const void*> ps) {
@@ -754,13 +744,11 @@ extern "C" int cfdb_total_fp64(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const voi
   CFDB_CUDA(ctx, cudaSetDevice(ctx->device));
   const void* vol = nullptr;
   if (!m->uniform) {
-    bool faces = false;  // either geometry holds the volumes
+    Geom geom = Geom::Arrays;  // either geometry holds the volumes
     const int p = dtype == CFDB_F64 ? 1 : 0;
     if (!m->plain[p].ready)
-      if (int rc = cfdb_mesh_need_faces(m, dtype, &faces)) return rc;
-    if (!faces)
-      if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
-    vol = faces ? m->faces[p].vol : m->plain[p].volume;
+      if (int rc = cfdb_mesh_geometry(m, dtype, true, &geom)) return rc;
+    vol = geom == Geom::Faces ? m->faces[p].vol : m->plain[p].volume;
   }
   const double vconst = m->dx * m->dy * m->dz;
   const bool vec = aligned16({field, vol});
@@ -781,10 +769,9 @@ extern "C" int cfdb_total_fp64(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const voi
 
 int plain_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* qn, const void* c, double cconst,
                     int mode, double dt) {
-  bool box = false;
-  if (int rc = cfdb_mesh_need_box(m, dtype, &box)) return rc;
-  if (box) return box_wave_step(ctx, m, dtype, q, qn, c, cconst, mode, dt);
-  if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
+  Geom geom = Geom::Arrays;
+  if (int rc = cfdb_mesh_geometry(m, dtype, false, &geom)) return rc;
+  if (geom == Geom::Box) return box_wave_step(ctx, m, dtype, q, qn, c, cconst, mode, dt);
   DISPATCH(dtype, R, wave_plain_k<R><<<grid_for(ctx, m->n, kThreads), kThreads, 0, ctx->stream>>>(
                          plain_args<R>(m, dtype), (const R*)q, (R*)qn, (const R*)c, R(cconst), mode, R(dt)));
   CFDB_LAUNCHED(ctx);

@@ -24,7 +24,6 @@
 
 #include "cfdb_internal.hpp"
 #include "f32x2.cuh"
-#include "heat_cell.cuh"
 
 CFDB_MODULE_ANCHOR
 

@@ -659,6 +659,35 @@ int cfdb_mesh_need_faces(cfdb_mesh* m, int dtype, bool* usable) {
   return CFDB_OK;
 }
 
+int cfdb_mesh_geometry(cfdb_mesh* m, int dtype, bool vertex_faces, Geom* geom) {
+  cfdb_ctx* ctx = m->ctx;
+  const int p = dtype == CFDB_F64 ? 1 : 0;
+  *geom = Geom::Arrays;
+  bool look = m->uniform || vertex_faces;
+  if (look && m->plain[p].ready && (m->uniform ? m->box[p].state : m->faces[p].state) == 0) {
+    // building allocates and copies, which a recording stream does not take
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &st);
+    if (e != cudaSuccess) cudaGetLastError();
+    look = e == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  }
+  if (look) {
+    bool usable = false;
+    int rc = CFDB_OK;
+    try {
+      rc = m->uniform ? cfdb_mesh_need_box(m, dtype, &usable) : cfdb_mesh_need_faces(m, dtype, &usable);
+    } catch (const std::bad_alloc&) {
+      rc = cfdb_fail(ctx, CFDB_ENOMEM, "host staging allocation failed");
+    }
+    if (rc && rc != CFDB_ENOMEM) return rc;
+    if (usable) {
+      *geom = m->uniform ? Geom::Box : Geom::Faces;
+      return CFDB_OK;
+    }
+  }
+  return cfdb_mesh_need_plain(m, dtype);
+}
+
 extern "C" int cfdb_mesh_plain_geometry(cfdb_mesh* m, cfdb_plain_geometry* out) {
   if (!out) return cfdb_fail(m ? m->ctx : nullptr, CFDB_EINVAL, "cfdb_mesh_plain_geometry: out is NULL");
   if (!m || !m->ctx) return cfdb_fail(nullptr, CFDB_EINVAL, "cfdb_mesh_plain_geometry: mesh is NULL or host-only");

@@ -21,13 +21,10 @@ extern "C" int cfdb_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int path, 
   if (T == Tn) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_heat_step: T and T_next must differ (no in-place stencil writes)");
   if (!std::isfinite(k) || !std::isfinite(dt)) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_heat_step: k and dt must be finite");
   if (path == CFDB_PATH_FUSED) return fused_heat_step(ctx, m, dtype, T, Tn, k, dt);
-  bool box = false;
-  if (int rc = cfdb_mesh_need_box(m, dtype, &box)) return rc;
-  if (box) return box_heat_step(ctx, m, dtype, T, Tn, k, dt);
-  bool faces = false;
-  if (int rc = cfdb_mesh_need_faces(m, dtype, &faces)) return rc;
-  if (faces) return vert_heat_step(ctx, m, dtype, T, Tn, k, dt);
-  if (int rc = cfdb_mesh_need_plain(m, dtype)) return rc;
+  Geom geom = Geom::Arrays;
+  if (int rc = cfdb_mesh_geometry(m, dtype, true, &geom)) return rc;
+  if (geom == Geom::Box) return box_heat_step(ctx, m, dtype, T, Tn, k, dt);
+  if (geom == Geom::Faces) return vert_heat_step(ctx, m, dtype, T, Tn, k, dt);
   PlainGeomDev& p = m->plain[dtype == CFDB_F64 ? 1 : 0];
   if (!p.stab_tmp)
     if (int rc = cfdb_dev_alloc(ctx, int64_t(dtype_size(dtype)) * 18 * m->n, &p.stab_tmp)) return rc;

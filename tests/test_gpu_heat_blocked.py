@@ -30,3 +30,19 @@ def test_passes_equal_single_steps(cfdb, ctx, shape):
             assert (final is b) == bool(steps & 1)
             assert torch.equal(final, p), steps
     ctx.sync()
+
+
+def test_passes_without_a_workspace(cfdb):
+    """A field small enough to leave the other buffer alone takes both buffers
+    when the workspace for that cannot be had."""
+    ctx = cfdb.Context(0)
+    m = cfdb.Mesh.structured(ctx, 96, 80, 100, 0.01, 0.01, 0.01)
+    T0 = torch.as_tensor(np.random.default_rng(3).uniform(-1, 1, m.n), dtype=torch.float32, device=DEV)
+    for steps in (7, 8):
+        a, b = T0.clone(), torch.empty_like(T0)
+        want = ctx.heat_run(m, a, b, 0.01, 1e-4, steps).clone()
+        ctx.set_alloc_budget(ctx.allocated_bytes() + m.n)
+        a = T0.clone()
+        assert torch.equal(ctx.heat_run(m, a, b, 0.01, 1e-4, steps), want)
+        ctx.set_alloc_budget(0)
+    ctx.sync()
