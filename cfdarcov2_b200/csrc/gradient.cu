@@ -19,48 +19,49 @@ namespace {
 
 constexpr int kThreads = 256;
 
+// J's partial sum of the CTA, and with `lam` the adjoint seed (p_T - p_target, 0, 0, 0)
+// in the same pass; the last CTA to finish folds the partials in a fixed order.
+// Bound by memory: 2 fields read, 4 written.
 template <class R>
-__global__ void init_adjoint_k(const R* __restrict__ qT, const R* __restrict__ target, R* __restrict__ lam, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    lam[i] = qT[i] - target[i];
-    lam[n + i] = R(0);
-    lam[2 * n + i] = R(0);
-    lam[3 * n + i] = R(0);
-  }
-}
-
-template <class R>
-__global__ void misfit_k(const R* __restrict__ qT, const R* __restrict__ target, long long n, double* __restrict__ part) {
+__global__ void __launch_bounds__(kThreads) misfit_k(const R* __restrict__ qT, const R* __restrict__ target, R* __restrict__ lam,
+                                                     long long n, double* __restrict__ part, unsigned* __restrict__ ticket,
+                                                     double* __restrict__ out) {
   __shared__ double red[kThreads / 32];
+  __shared__ bool last;
   double s = 0;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double d = double(qT[i]) - double(target[i]);
+  for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kThreads) {
+    const R q = qT[i], t = target[i];
+    const double d = double(q) - double(t);
     s += d * d;
+    if (lam) {
+      lam[i] = q - t;
+      lam[n + i] = R(0);
+      lam[2 * n + i] = R(0);
+      lam[3 * n + i] = R(0);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
+  auto cta_sum = [&](double v) {  // on thread 0
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0;
+    if (threadIdx.x == 0)
+      for (int w = 0; w < kThreads / 32; ++w) v += red[w];
+    return v;
+  };
+  s = cta_sum(s);
   if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < int(blockDim.x / 32); ++w) t += red[w];
-    part[blockIdx.x] = t;
+    part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
-}
-
-// one CTA, partials in a fixed order (one thread adding them in turn had
-// cost 13 us)
-__global__ void misfit_final_k(const double* __restrict__ part, int np, double* __restrict__ out) {
-  __shared__ double red[kThreads / 32];
-  double t = 0;
-  for (int k = threadIdx.x; k < np; k += kThreads) t += part[k];
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    t = 0;
-    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-    out[0] = 0.5 * t;
-  }
+  if (!last) return;
+  __threadfence();
+  s = 0;
+  for (int k = threadIdx.x; k < int(gridDim.x); k += kThreads) s += __ldcg(part + k);
+  s = cta_sum(s);
+  if (threadIdx.x == 0) out[0] = 0.5 * s;
 }
 
 struct Run {
@@ -82,20 +83,23 @@ struct Run {
     CFDB_CUDA(ctx, cudaMemcpyAsync(dst, src, 4 * n * esz, cudaMemcpyDeviceToDevice, ctx->stream));
     return CFDB_OK;
   }
-  // J into *host (synchronous) and, when lam != nullptr, the adjoint seed.
-  int misfit(const void* qT, const void* target, void* lam, double* host, void* scratch) const {
+  // J to the end of `scratch` (misfit_bytes()) and, when lam != nullptr, the adjoint
+  // seed; read_misfit() waits for it and returns it.
+  int64_t misfit_bytes() const { return int64_t(8) * (grid_for(ctx, n, kThreads, 2) + 2); }
+  int misfit(const void* qT, const void* target, void* lam, void* scratch) const {
     const int grid = grid_for(ctx, n, kThreads, 2);
     double* part = static_cast<double*>(scratch);
-    double* res = part + grid;
-    if (dtype == CFDB_F64) {
-      misfit_k<double><<<grid, kThreads, 0, ctx->stream>>>((const double*)qT, (const double*)target, n, part);
-      if (lam) init_adjoint_k<double><<<grid_for(ctx, n, kThreads), kThreads, 0, ctx->stream>>>((const double*)qT, (const double*)target, (double*)lam, n);
-    } else {
-      misfit_k<float><<<grid, kThreads, 0, ctx->stream>>>((const float*)qT, (const float*)target, n, part);
-      if (lam) init_adjoint_k<float><<<grid_for(ctx, n, kThreads), kThreads, 0, ctx->stream>>>((const float*)qT, (const float*)target, (float*)lam, n);
-    }
-    misfit_final_k<<<1, kThreads, 0, ctx->stream>>>(part, grid, res);
+    unsigned* ticket = reinterpret_cast<unsigned*>(part + grid + 1);
+    CFDB_CUDA(ctx, cudaMemsetAsync(ticket, 0, sizeof(unsigned), ctx->stream));
+    if (dtype == CFDB_F64)
+      misfit_k<double><<<grid, kThreads, 0, ctx->stream>>>((const double*)qT, (const double*)target, (double*)lam, n, part, ticket, part + grid);
+    else
+      misfit_k<float><<<grid, kThreads, 0, ctx->stream>>>((const float*)qT, (const float*)target, (float*)lam, n, part, ticket, part + grid);
     CFDB_LAUNCHED(ctx);
+    return CFDB_OK;
+  }
+  int read_misfit(const void* scratch, double* host) const {
+    const double* res = static_cast<const double*>(scratch) + grid_for(ctx, n, kThreads, 2);
     CFDB_CUDA(ctx, cudaMemcpyAsync(host, res, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return CFDB_OK;
@@ -140,12 +144,13 @@ extern "C" int cfdb_wave_objective(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int p
   void *a, *b, *scratch;
   if (int rc = B.get(int64_t(4 * R.esz) * R.n, &a)) return rc;
   if (int rc = B.get(int64_t(4 * R.esz) * R.n, &b)) return rc;
-  if (int rc = B.get(int64_t(8) * (grid_for(ctx, R.n, kThreads, 2) + 2), &scratch)) return rc;
+  if (int rc = B.get(R.misfit_bytes(), &scratch)) return rc;
   if (int rc = R.copy(a, q0)) return rc;
   if (int rc = cfdb_run_steps(ctx, a, b, steps, 1, [&](const void* s, void* d) { return R.step(s, d); },
                               graph_key("wave", m, dtype, path, a, b, c, {0.0, 1.0, dt})))
     return rc;
-  return R.misfit((steps & 1) ? b : a, target, nullptr, J_out, scratch);
+  if (int rc = R.misfit((steps & 1) ? b : a, target, nullptr, scratch)) return rc;
+  return R.read_misfit(scratch, J_out);
 }
 
 extern "C" int cfdb_wave_gradient(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int path, const void* q0, const void* c,
@@ -161,7 +166,7 @@ extern "C" int cfdb_wave_gradient(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int pa
   void *lamA, *lamB, *scratch;
   if (int rc = B.get(sb, &lamA)) return rc;
   if (int rc = B.get(sb, &lamB)) return rc;
-  if (int rc = B.get(int64_t(8) * (grid_for(ctx, R.n, kThreads, 2) + 2), &scratch)) return rc;
+  if (int rc = B.get(R.misfit_bytes(), &scratch)) return rc;
   CFDB_CUDA(ctx, cudaMemsetAsync(grad_c, 0, R.esz * R.n, ctx->stream));
   cudaEvent_t e0, e1, e2;
   CFDB_CUDA(ctx, cudaEventCreate(&e0));
@@ -199,7 +204,7 @@ extern "C" int cfdb_wave_gradient(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int pa
     if (rc) return rc;
     st.forward_steps = steps;
     st.snapshots_used = steps + 1;
-    if ((rc = R.misfit(slot(steps), target, lam, J_out, scratch))) return rc;
+    if ((rc = R.misfit(slot(steps), target, lam, scratch))) return rc;
     CfdbRange reverse("cfdb_wave_gradient: reverse sweep");
     for (int t = steps - 1; t >= 0 && !rc; --t) rc = adj(slot(t));
   } else {
@@ -231,7 +236,7 @@ extern "C" int cfdb_wave_gradient(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int pa
           first_turn_seen = true;
           if ((rc = R.step(cur, tmp))) break;  // q_T
           ++st.forward_steps;
-          if ((rc = R.misfit(tmp, target, lam, J_out, scratch))) break;
+          if ((rc = R.misfit(tmp, target, lam, scratch))) break;
           rc = adj(cur);
           break;
         case CFDB_RV_YOUTURN: rc = adj(cur); break;
@@ -245,7 +250,7 @@ extern "C" int cfdb_wave_gradient(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int pa
   // dJ/dp0 = the pressure block of lam_0
   CFDB_CUDA(ctx, cudaMemcpyAsync(grad_p0, lam, R.esz * R.n, cudaMemcpyDeviceToDevice, ctx->stream));
   cudaEventRecord(e2, ctx->stream);
-  CFDB_CUDA(ctx, cudaEventSynchronize(e2));
+  if ((rc = R.read_misfit(scratch, J_out))) return rc;  // the call's one wait
   float f = 0, r = 0;
   cudaEventElapsedTime(&f, e0, e1);
   cudaEventElapsedTime(&r, e1, e2);
