@@ -35,6 +35,7 @@
 // stabilisation at 200^3 FP32, 139 and 565 instructions per cell.)
 // Compiled with --fmad=false like plain_ops.cu.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <limits>
 
@@ -44,7 +45,7 @@ CFDB_MODULE_ANCHOR
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;
 
 template <class R> struct Box {
   int nx, ny, nz;
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(kThreads) box_sum_k(const __grid_constant__ Bo
 // enough that no intermediate overflows; a plane within two of one that is
 // not is computed by the full sums.
 template <class R, int NY, bool UNI, bool FULL>
-__global__ void __launch_bounds__(128) box_stab_k(const __grid_constant__ Box<R> g, const R* __restrict__ phi, R* __restrict__ out, int mask_) {
+__global__ void __launch_bounds__(kThreads) box_stab_k(const __grid_constant__ Box<R> g, const R* __restrict__ phi, R* __restrict__ out, int mask_) {
   constexpr int NR = NY + 4;  // rows -2 .. NY + 1
   March<NY, 2, 2> w;
   if (!w.start(g)) return;
@@ -512,7 +513,7 @@ enum { OUT_SUM = 0, OUT_GRADIENT = 1 };
 // Gradient (OP_GRAD) or Laplacian (OP_LAPL, OP_HEAT) of every cell; OUT_GRADIENT
 // stores the three gradient components (arrays of n) instead of their masked sum.
 template <class R, int OP, int OUT>
-__global__ void __launch_bounds__(128) vert_sum_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
+__global__ void __launch_bounds__(kThreads) vert_sum_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
                                                   R* __restrict__ out, int mask, R k, R dt) {
   March<1, 1, 1> w;
   if (!w.start(g)) return;
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(128) vert_sum_k(const __grid_constant__ Vert<R
 // side is the cell's own value on its opposite face (the reference's ids point
 // back to the cell).
 template <class R>
-__global__ void __launch_bounds__(128) vert_stab_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
+__global__ void __launch_bounds__(kThreads) vert_stab_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
                                                    const R* __restrict__ grad, R* __restrict__ out, int mask) {
   March<1, 1, 1> w;
   if (!w.start(g)) return;
@@ -744,7 +745,7 @@ template <int D, class R> __device__ __forceinline__ void wave_ghost(const R P[4
 // results, which are then computed again by the full sums.
 // 100 x 90 x 96 FP64 (55 MB): floor 9 us.
 template <class R, int NY, bool UNI, bool CF>
-__global__ void __launch_bounds__(128) box_wave_k(const __grid_constant__ Box<R> g, const __grid_constant__ WaveArgs<R> a) {
+__global__ void __launch_bounds__(kThreads) box_wave_k(const __grid_constant__ Box<R> g, const __grid_constant__ WaveArgs<R> a) {
   March<NY, 1, 1> w;
   if (!w.start(g)) return;
   const int64_t pl = g.plane, n = int64_t(g.nx) * pl;
@@ -917,28 +918,67 @@ __global__ void __launch_bounds__(kThreads) box_volume_k(int nx, int ny, int nz,
   if (other) atomicOr(differs, 1);
 }
 
-// Warps of a march over `groups` row groups: tiles of 32 - 2 HZ lanes along
-// (group, z), x cut into chunks for about 32 warps per SM (one wave at 64
-// registers; 24 and 48 measured within 10 %), each at least two planes long: a
-// chunk evaluates the face below it a second time.
-void march_grid(const cfdb_ctx* ctx, const cfdb_mesh* m, int HZ, int threads, unsigned* tiles, unsigned* chunks, unsigned* blocks,
-                int64_t groups = 0) {
-  const int64_t lanes = (groups ? groups : m->ny) * m->nz;
-  *tiles = unsigned((lanes + 32 - 2 * HZ - 1) / (32 - 2 * HZ));
-  const int64_t want = std::max<int64_t>(1, int64_t(ctx->num_sms) * 32 / *tiles);
-  *chunks = unsigned(std::min<int64_t>(std::min(want, int64_t(m->nx)), std::max<int64_t>(1, m->nx / 2)));
-  *blocks = unsigned((int64_t(*tiles) * *chunks * 32 + threads - 1) / threads);
+// A kernel and the CTAs of it that one SM holds.
+template <class K> struct Form {
+  K kern;
+  int resident;
+};
+template <auto kern> Form<decltype(kern)> form(const cfdb_ctx* ctx) {
+  static std::atomic<int> held[kMaxDevices] = {};
+  const bool known = ctx->device >= 0 && ctx->device < kMaxDevices;
+  int r = known ? held[ctx->device].load(std::memory_order_relaxed) : 0;
+  if (r == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, kThreads, 0) != cudaSuccess) cudaGetLastError();
+    r = std::max(r, 1);
+    if (known) held[ctx->device].store(r, std::memory_order_relaxed);
+  }
+  return {kern, r};
 }
 
-// Kernel arguments for NY rows per thread, HZ halo lanes and blocks of
-// `threads`; *blocks = the grid.
-template <class R> Box<R> box_of(const cfdb_ctx* ctx, const cfdb_mesh* m, int NY, int HZ, int threads, unsigned* blocks) {
+// Warps of a march over `groups` row groups: tiles of 32 - 2 HZ lanes along
+// (group, z), x cut into chunks of at least two planes.  Fewer chunks are less
+// work, as each starts with 2 + HZ / 2 planes' worth of loads and faces that its
+// neighbour has too, but they have to fill the SMs evenly.  With w warps on an SM
+// a plane costs 8 + w (8 for latency); after a first wave the CTAs end at
+// different times, so the last one counts for three quarters as a wave and for
+// one as its share of one.  The least sum is within 2 % of the best of 1 to 50
+// chunks over 10 meshes x 5 operators; 32 warps per SM whatever the kernel held
+// had lost 9 % (FP64 gradient at 200^3: 123 us in 501 CTAs on 444 places, now 75;
+// plain FP64 acoustic step there 187 -> 170, vertex gradient at 400k cells 12.7 -> 10.7).
+void march_grid(const cfdb_ctx* ctx, const cfdb_mesh* m, int HZ, int resident, unsigned* tiles, unsigned* chunks,
+                unsigned* blocks, int64_t groups) {
+  *tiles = unsigned((groups * m->nz + 32 - 2 * HZ - 1) / (32 - 2 * HZ));
+  constexpr int per = kThreads / 32;
+  const int64_t sms = std::max(1, ctx->num_sms), places = sms * resident;
+  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(m->nx / 2, 8 * places * per / *tiles));
+  const double wave = 8 + resident * per;
+  double least = 0;
+  *chunks = 1;
+  for (int64_t c = 1; c <= most; c += std::max<int64_t>(1, c / 32)) {
+    const int64_t ctas = (*tiles * c + per - 1) / per, full = ctas / places, last = ctas % places;
+    double waves = double(full) * wave;
+    if (last) {
+      const double own = 8 + double((last + sms - 1) / sms * per);
+      waves += full ? 0.75 * own + 0.25 * wave * double(last) / double(places) : own;
+    }
+    const double cost = (waves + 0.05 * wave) * (double(m->nx) / double(c) + 2 + 0.5 * HZ);
+    if (c == 1 || cost < least) {
+      least = cost;
+      *chunks = unsigned(c);
+    }
+  }
+  *blocks = unsigned((int64_t(*tiles) * *chunks + per - 1) / per);
+}
+
+// Kernel arguments for NY rows per thread, HZ halo lanes and `resident` CTAs per
+// SM; *blocks = the grid.
+template <class R> Box<R> box_of(const cfdb_ctx* ctx, const cfdb_mesh* m, int NY, int HZ, int resident, unsigned* blocks) {
   const BoxGeomDev& b = m->box[sizeof(R) == 8 ? 1 : 0];
   Box<R> g;
   g.nx = int(m->nx); g.ny = int(m->ny); g.nz = int(m->nz);
   g.plane = unsigned(m->ny * m->nz);
   g.groups = int((m->ny + NY - 1) / NY);
-  march_grid(ctx, m, HZ, threads, &g.tiles, &g.chunks, blocks, g.groups);
+  march_grid(ctx, m, HZ, resident, &g.tiles, &g.chunks, blocks, g.groups);
   g.hx = b.h[0]; g.hy = b.h[1]; g.hz = b.h[2];
   auto t = [](const void* p) { return static_cast<const R*>(p); };
   g.ax = t(b.alpha[0]); g.ay = t(b.alpha[1]); g.az = t(b.alpha[2]);
@@ -1057,13 +1097,13 @@ int build_box(cfdb_mesh* m, BoxGeomDev& b) {
   return CFDB_OK;
 }
 
-template <class R> Vert<R> vert_of(const cfdb_ctx* ctx, const cfdb_mesh* m, unsigned* blocks) {
+template <class R> Vert<R> vert_of(const cfdb_ctx* ctx, const cfdb_mesh* m, int resident, unsigned* blocks) {
   const FaceGeomDev& b = m->faces[sizeof(R) == 8 ? 1 : 0];
   Vert<R> g;
   g.nx = int(m->nx); g.ny = int(m->ny); g.nz = int(m->nz);
   g.plane = unsigned(m->ny * m->nz);
   g.groups = g.ny;
-  march_grid(ctx, m, 1, 128, &g.tiles, &g.chunks, blocks);
+  march_grid(ctx, m, 1, resident, &g.tiles, &g.chunks, blocks, g.groups);
   for (int a = 0; a < 3; ++a) {
     for (int d = 0; d < 3; ++d) g.nrm[a][d] = static_cast<const R*>(b.normal[a]) + d * b.count[a];
     g.area[a] = static_cast<const R*>(b.area[a]);
@@ -1095,16 +1135,16 @@ int cfdb_mesh_need_box(cfdb_mesh* m, int dtype, bool* usable) {
 // The kernel of a mesh: one value per direction and all directions, all
 // directions, or neither; NY = 2 rows per thread in FP32 only.
 #define BOX_FORMS(kernel, ...)                                   \
-  (uni && mask == 7 ? kernel<__VA_ARGS__, true, true> : mask == 7 ? kernel<__VA_ARGS__, false, true> : kernel<__VA_ARGS__, false, false>)
+  (uni && mask == 7 ? form<kernel<__VA_ARGS__, true, true>>(ctx) : mask == 7 ? form<kernel<__VA_ARGS__, false, true>>(ctx) : form<kernel<__VA_ARGS__, false, false>>(ctx))
 
 template <class R, int OP> int launch_sum(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask, double k, double dt) {
   constexpr int NY = sizeof(R) == 4 ? 2 : 1;
   const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
-  const Box<R> g = box_of<R>(ctx, m, rows, 1, kThreads, &blocks);
-  auto kern = rows == 1 ? BOX_FORMS(box_sum_k, R, OP, 1) : BOX_FORMS(box_sum_k, R, OP, NY);
-  kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
+  const auto f = rows == 1 ? BOX_FORMS(box_sum_k, R, OP, 1) : BOX_FORMS(box_sum_k, R, OP, NY);
+  const Box<R> g = box_of<R>(ctx, m, rows, 1, f.resident, &blocks);
+  f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
 }
@@ -1114,16 +1154,16 @@ template <class R> int launch_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi,
   const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
-  const Box<R> g = box_of<R>(ctx, m, rows, 2, 128, &blocks);
-  auto kern = rows == 1 ? BOX_FORMS(box_stab_k, R, 1) : BOX_FORMS(box_stab_k, R, NY);
-  kern<<<blocks, 128, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask);
+  const auto f = rows == 1 ? BOX_FORMS(box_stab_k, R, 1) : BOX_FORMS(box_stab_k, R, NY);
+  const Box<R> g = box_of<R>(ctx, m, rows, 2, f.resident, &blocks);
+  f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask);
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
 }
 
-template <class R, int NY> auto wave_kernel(bool uni, bool c) {
-  return uni ? (c ? box_wave_k<R, NY, true, true> : box_wave_k<R, NY, true, false>)
-             : (c ? box_wave_k<R, NY, false, true> : box_wave_k<R, NY, false, false>);
+template <class R, int NY> auto wave_kernel(const cfdb_ctx* ctx, bool uni, bool c) {
+  return uni ? (c ? form<box_wave_k<R, NY, true, true>>(ctx) : form<box_wave_k<R, NY, true, false>>(ctx))
+             : (c ? form<box_wave_k<R, NY, false, true>>(ctx) : form<box_wave_k<R, NY, false, false>>(ctx));
 }
 template <class R>
 int launch_wave(cfdb_ctx* ctx, cfdb_mesh* m, const void* q, void* qn, const void* c, double cconst, int mode, double dt) {
@@ -1131,10 +1171,10 @@ int launch_wave(cfdb_ctx* ctx, cfdb_mesh* m, const void* q, void* qn, const void
   const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
-  const Box<R> g = box_of<R>(ctx, m, rows, 1, 128, &blocks);
+  const auto f = rows == 1 ? wave_kernel<R, 1>(ctx, uni, c != nullptr) : wave_kernel<R, NY>(ctx, uni, c != nullptr);
+  const Box<R> g = box_of<R>(ctx, m, rows, 1, f.resident, &blocks);
   const WaveArgs<R> a{static_cast<const R*>(q), static_cast<R*>(qn), static_cast<const R*>(c), R(cconst), R(dt), mode};
-  auto kern = rows == 1 ? wave_kernel<R, 1>(uni, c != nullptr) : wave_kernel<R, NY>(uni, c != nullptr);
-  kern<<<blocks, 128, 0, ctx->stream>>>(g, a);
+  f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, a);
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
 }
@@ -1166,8 +1206,9 @@ int box_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* q
 template <class R, int OP, int OUT>
 int launch_vert_sum(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask, double k, double dt) {
   unsigned blocks = 0;
-  const Vert<R> g = vert_of<R>(ctx, m, &blocks);
-  vert_sum_k<R, OP, OUT><<<blocks, 128, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
+  const auto f = form<vert_sum_k<R, OP, OUT>>(ctx);
+  const Vert<R> g = vert_of<R>(ctx, m, f.resident, &blocks);
+  f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
 }
@@ -1193,8 +1234,9 @@ template <class R> int launch_vert_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void*
     if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(R)) * 3 * m->n, &b.grad)) return rc;
   if (int rc = launch_vert_sum<R, OP_GRAD, OUT_GRADIENT>(ctx, m, phi, b.grad, 7, 0, 0)) return rc;
   unsigned blocks = 0;
-  const Vert<R> g = vert_of<R>(ctx, m, &blocks);
-  vert_stab_k<R><<<blocks, 128, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<const R*>(b.grad),
+  const auto f = form<vert_stab_k<R>>(ctx);
+  const Vert<R> g = vert_of<R>(ctx, m, f.resident, &blocks);
+  f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<const R*>(b.grad),
                                                   static_cast<R*>(out), mask);
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
