@@ -83,6 +83,7 @@ struct BoxGeomDev {
 struct FaceGeomDev {
   int state = 0;  // 0 not built, 1 usable, 2 this mesh keeps the N x 6 arrays
   int64_t count[3] = {};
+  void* block = nullptr;  // holds all of the following but grad
   void* normal[3] = {};
   void* area[3] = {};
   void* alpha[3] = {};

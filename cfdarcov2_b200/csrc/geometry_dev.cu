@@ -135,21 +135,31 @@ template <class T> int build_faces(cfdb_mesh* m, FaceGeomDev& b) {
   b.count[0] = (m->nx + 1) * m->ny * m->nz;
   b.count[1] = m->nx * (m->ny + 1) * m->nz;
   b.count[2] = m->nx * m->ny * (m->nz + 1);
+  // one block: an allocation apiece had cost as much as the geometry itself
+  int64_t size = 0;
+  auto take = [&](int64_t values) {
+    const int64_t at = size;
+    size += (int64_t(sizeof(T)) * values + 255) & ~int64_t(255);
+    return at;
+  };
+  int64_t on[3], oa[3], ol[3];
+  for (int d = 0; d < 3; ++d) {
+    on[d] = take(3 * b.count[d]);
+    oa[d] = take(b.count[d]);
+    ol[d] = take(b.count[d]);
+  }
+  const int64_t olen = take(6 * m->n), ovol = take(m->n);
+  if (int rc = cfdb_dev_alloc(ctx, size, &b.block)) return rc;
+  auto part = [&](int64_t at) { return reinterpret_cast<T*>(static_cast<char*>(b.block) + at); };
   FaceArrays<T> a{};
   for (int d = 0; d < 3; ++d) {
-    const int64_t bytes = int64_t(sizeof(T)) * b.count[d];
-    if (int rc = cfdb_dev_alloc(ctx, 3 * bytes, &b.normal[d])) return rc;
-    if (int rc = cfdb_dev_alloc(ctx, bytes, &b.area[d])) return rc;
-    if (int rc = cfdb_dev_alloc(ctx, bytes, &b.alpha[d])) return rc;
-    a.normal[d] = static_cast<T*>(b.normal[d]);
-    a.area[d] = static_cast<T*>(b.area[d]);
-    a.alpha[d] = static_cast<T*>(b.alpha[d]);
+    b.normal[d] = a.normal[d] = part(on[d]);
+    b.area[d] = a.area[d] = part(oa[d]);
+    b.alpha[d] = a.alpha[d] = part(ol[d]);
     a.count[d] = b.count[d];
   }
-  if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(T)) * 6 * m->n, &b.len)) return rc;
-  if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(T)) * m->n, &b.vol)) return rc;
-  a.len = static_cast<T*>(b.len);
-  a.vol = static_cast<T*>(b.vol);
+  b.len = a.len = part(olen);
+  b.vol = a.vol = part(ovol);
   void* dverts = nullptr;
   const int64_t vb = int64_t(sizeof(double)) * int64_t(m->verts.size());
   if (int rc = cfdb_dev_alloc(ctx, vb, &dverts)) return rc;

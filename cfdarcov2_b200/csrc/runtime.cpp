@@ -499,13 +499,7 @@ extern "C" int cfdb_mesh_create_from_vertices(cfdb_ctx* ctx, int64_t nx, int64_t
 }
 
 static void free_faces(cfdb_ctx* ctx, FaceGeomDev& b) {
-  for (int d = 0; d < 3; ++d) {
-    cfdb_dev_free(ctx, b.normal[d]);
-    cfdb_dev_free(ctx, b.area[d]);
-    cfdb_dev_free(ctx, b.alpha[d]);
-  }
-  cfdb_dev_free(ctx, b.len);
-  cfdb_dev_free(ctx, b.vol);
+  cfdb_dev_free(ctx, b.block);
   cfdb_dev_free(ctx, b.grad);
   b = FaceGeomDev();
 }
