@@ -39,7 +39,7 @@
 #include <cmath>
 #include <limits>
 
-#include "cfdb_internal.hpp"
+#include "euler_internal.hpp"
 
 CFDB_MODULE_ANCHOR
 
@@ -884,6 +884,227 @@ __global__ void __launch_bounds__(kThreads) box_wave_k(const __grid_constant__ B
   }
 }
 
+// ---- Euler step -----------------------------------------------------------------
+
+// A state and what the fluxes take from it.  u, v, w carry NaN where a velocity or
+// the pressure is not finite (the array form multiplies each by the zero components
+// of a normal), so such a cell and its neighbours come out NaN and take the full form.
+template <class R> struct Gas {
+  R q[5];    // rho, momentum, E
+  R vel[3];
+  R p, a;
+};
+
+// zero or far enough from the ends of the range for Volume::quot
+__device__ __forceinline__ bool moderate(double x) {
+  const unsigned h = unsigned(__double2hiint(x)) & 0x7fffffffu;
+  return h - 0x26f00000u < 0x32000000u || x == 0.0;  // 2^-400 to 2^400
+}
+__device__ __forceinline__ bool moderate(float x) {
+  const float b = fabsf(x);
+  return (b >= 0x1p-60f && b <= 0x1p60f) || b == 0.f;
+}
+
+// prim() of the array kernel: four divisions by rho, as one reciprocal and products
+// corrected to the rounded quotient (Volume).
+template <class R> __device__ __forceinline__ void derive(Gas<R>& s, R gamma) {
+  const R rho = s.q[0], mx = s.q[1], my = s.q[2], mz = s.q[3];
+  const Volume<R> V{rho, R(1) / rho};
+  const bool ok = moderate(rho) && rho != R(0);
+  R u, v, w;
+  if (ok && moderate(mx) && moderate(my) && moderate(mz)) {
+    u = V.quot(mx); v = V.quot(my); w = V.quot(mz);
+  } else {
+    u = mx / rho; v = my / rho; w = mz / rho;
+  }
+  const R ke = R(0.5) * ((mx * u + my * v) + mz * w);
+  s.p = (gamma - R(1)) * (s.q[4] - ke);
+  const R gp = gamma * s.p;
+  s.a = sqrt(ok && moderate(gp) ? V.quot(gp) : gp / rho);
+  const R taint = ((u * R(0) + v * R(0)) + w * R(0)) + s.p * R(0);
+  s.vel[0] = u + taint;
+  s.vel[1] = v + taint;
+  s.vel[2] = w + taint;
+}
+
+// Reflection in a wall normal to D; NaN where the array form's 2 m_D overflows.
+template <int D, class R> __device__ __forceinline__ void mirror(Gas<R>& s) {
+  s.vel[D] = (R(2) * s.q[1 + D]) * R(0) - s.vel[D];
+  s.q[1 + D] = -s.q[1 + D];
+}
+
+// Flux through a face normal to D from L to H.  The array form evaluates it once per
+// side with opposite normals, which gives the same magnitudes.
+template <int D, class R> __device__ __forceinline__ void rusanov(const Gas<R>& L, const Gas<R>& H, R F[5]) {
+  const R ul = L.vel[D], uh = H.vel[D];
+  const R lm = fmax(fabs(ul) + L.a, fabs(uh) + H.a);
+  const R hl = R(0.5) * lm;
+  F[0] = R(0.5) * (L.q[0] * ul + H.q[0] * uh) - hl * (H.q[0] - L.q[0]);
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    R l = L.q[1 + e] * ul, h = H.q[1 + e] * uh;
+    if (e == D) {
+      l = l + L.p;
+      h = h + H.p;
+    }
+    F[1 + e] = R(0.5) * (l + h) - hl * (H.q[1 + e] - L.q[1 + e]);
+  }
+  F[4] = R(0.5) * ((L.q[4] + L.p) * ul + (H.q[4] + H.p) * uh) - hl * (H.q[4] - L.q[4]);
+}
+
+template <class R> struct EulerArgs {
+  const R* __restrict__ U;
+  R* __restrict__ Un;
+  R gamma;
+  double dx, dy, dz, cfl, t_end;
+  const EulerClock* clock;
+  long long step;
+};
+
+// One cell of euler_plain_step_k (euler_plain.cu).
+template <class R> __device__ __noinline__ void euler_full(const Box<R>& g, const EulerArgs<R>& a, R dt, int x, int y, int z) {
+  const int64_t n = int64_t(g.nx) * g.plane;
+  const Cell c{x, y, z};
+  const int64_t i = id_of(g, c);
+  auto prim = [&](const R q[5], R s[5]) {
+    s[0] = q[1] / q[0]; s[1] = q[2] / q[0]; s[2] = q[3] / q[0];
+    const R ke = R(0.5) * ((q[1] * s[0] + q[2] * s[1]) + q[3] * s[2]);
+    s[3] = (a.gamma - R(1)) * (q[4] - ke);
+    s[4] = sqrt(a.gamma * s[3] / q[0]);
+  };
+  R P[5], sP[5], acc[5];
+  for (int k = 0; k < 5; ++k) {
+    P[k] = a.U[k * n + i];
+    acc[k] = R(0);
+  }
+  prim(P, sP);
+  for (int f = 0; f < 6; ++f) {
+    const R nx = outward<R>(f, 0), ny = outward<R>(f, 1), nz = outward<R>(f, 2), A = area_of(g, c, f);
+    const int64_t j = id_of(g, beyond(g, c, f));
+    R N[5], sN[5], F[5];
+    for (int k = 0; k < 5; ++k) N[k] = a.U[k * n + j];
+    if (j == i && f < 4) {
+      const R two_mn = R(2) * ((P[1] * nx + P[2] * ny) + P[3] * nz);
+      N[1] = P[1] - two_mn * nx;
+      N[2] = P[2] - two_mn * ny;
+      N[3] = P[3] - two_mn * nz;
+    }
+    prim(N, sN);
+    const R uP = (sP[0] * nx + sP[1] * ny) + sP[2] * nz, uN = (sN[0] * nx + sN[1] * ny) + sN[2] * nz;
+    const R hl = R(0.5) * fmax(fabs(uP) + sP[4], fabs(uN) + sN[4]);
+    const R m[3] = {nx, ny, nz};
+    F[0] = R(0.5) * (P[0] * uP + N[0] * uN) - hl * (N[0] - P[0]);
+    for (int e = 0; e < 3; ++e)
+      F[1 + e] = R(0.5) * ((P[1 + e] * uP + sP[3] * m[e]) + (N[1 + e] * uN + sN[3] * m[e])) - hl * (N[1 + e] - P[1 + e]);
+    F[4] = R(0.5) * ((P[4] + sP[3]) * uP + (N[4] + sN[3]) * uN) - hl * (N[4] - P[4]);
+    for (int k = 0; k < 5; ++k) acc[k] = acc[k] + F[k] * A;
+  }
+  for (int k = 0; k < 5; ++k) a.Un[k * n + i] = dt * (-(acc[k] / g.volume(i))) + P[k];
+}
+
+// euler_plain_step_k without face arrays: a cell's velocities, pressure and sound
+// speed are derived once for its x and z faces and once per y neighbour (three times
+// instead of seven), x and z faces are evaluated once, and no geometry is read but the
+// edge lengths (31 values per cell in the array form).  FP64 step with its reduction
+// (12 us) at 64^3 65.7 -> 35.0 us, 128^3 330 -> 162; FP32 there 48 -> 25, 188 -> 98.
+// Bound by the chains of divisions and roots at 12 warps per SM (150 registers; 16 warps
+// at 128 spill: the same time).
+template <class R>
+__global__ void __launch_bounds__(kThreads) box_euler_k(const __grid_constant__ Box<R> g, const __grid_constant__ EulerArgs<R> a) {
+  const EulerClock* ck = a.clock;
+  const int ts = int(a.step & 1), ls = int(a.step % 3);
+  if (ck->finished[ts]) return;
+  const double lam[3] = {bits_to_double(ck->lam[ls][0]), bits_to_double(ck->lam[ls][1]), bits_to_double(ck->lam[ls][2])};
+  bool last;
+  const R dt = R(euler_dt(lam, a.dx, a.dy, a.dz, a.cfl, ck->t[ts], a.t_end, &last));
+  March<1, 1, 1> w;
+  if (!w.start(g)) return;
+  const int64_t pl = g.plane, n = pl * g.nx;
+  auto load = [&](int x, int row) {
+    Gas<R> s;
+    const R* q = a.U + x * pl + w.off[1 + row];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) s.q[k] = q[k * n];
+    derive(s, a.gamma);
+    return s;
+  };
+  const double hy = g.hy[w.y0], hz = g.hz[w.z];
+  const R Ax = R(hy * hz);
+  Gas<R> P = load(w.x0, 0);
+  R fx[5];
+  rusanov<0>(w.x0 > 0 ? load(w.x0 - 1, 0) : P, P, fx);
+  for (int x = w.x0; x < w.x1; ++x) {
+    const double hx = g.hx[x];
+    const R Ay = R(hx * hz), Az = R(hx * hy);
+    R acc[5], F[5];
+    {
+      Gas<R> L;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) L.q[k] = __shfl_up_sync(kWarp, P.q[k], 1);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) L.vel[k] = __shfl_up_sync(kWarp, P.vel[k], 1);
+      L.p = __shfl_up_sync(kWarp, P.p, 1);
+      L.a = __shfl_up_sync(kWarp, P.a, 1);
+      if (w.zlo) {
+        L = P;
+        mirror<2>(L);
+      }
+      rusanov<2>(L, P, F);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) acc[k] = R(0) - F[k] * Az;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) F[k] = __shfl_down_sync(kWarp, F[k], 1);
+      if (w.zhi) {
+        L = P;
+        mirror<2>(L);
+        rusanov<2>(P, L, F);
+      }
+#pragma unroll
+      for (int k = 0; k < 5; ++k) acc[k] = acc[k] + F[k] * Az;
+    }
+    {
+      Gas<R> Y = load(x, -1);
+      if (w.y0 == 0) mirror<1>(Y);
+      rusanov<1>(Y, P, F);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) acc[k] = acc[k] - F[k] * Ay;
+    }
+    {
+      Gas<R> Y = load(x, 1);
+      if (w.y0 == g.ny - 1) mirror<1>(Y);
+      rusanov<1>(P, Y, F);
+#pragma unroll
+      for (int k = 0; k < 5; ++k) acc[k] = acc[k] + F[k] * Ay;
+    }
+    const Gas<R> N = x < g.nx - 1 ? load(x + 1, 0) : P;
+    rusanov<0>(P, N, F);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      acc[k] = (acc[k] - fx[k] * Ax) + F[k] * Ax;
+      fx[k] = F[k];
+    }
+    const int64_t i = x * pl + w.off[1];
+    const R vol = g.volume(i);
+    const Volume<R> V{vol, g.vol ? R(1) / vol : g.rv};
+    V.template divide<5>(acc);
+    bool fine = true;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      acc[k] = dt * (-acc[k]) + P.q[k];
+      fine = fine && finite(acc[k]);
+    }
+    if (w.out) {
+      if (fine) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) a.Un[k * n + i] = acc[k];
+      } else {
+        euler_full(g, a, dt, x, w.y0, w.z);
+      }
+    }
+    P = N;
+  }
+}
+
 // ---- tables -------------------------------------------------------------------
 
 // Volume of a cell, the sum of cell_geometry() (geometry_cell.hpp): the face
@@ -1201,6 +1422,22 @@ int box_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* q
                   double dt) {
   return dtype == CFDB_F64 ? launch_wave<double>(ctx, m, q, qn, c, cconst, mode, dt)
                            : launch_wave<float>(ctx, m, q, qn, c, cconst, mode, dt);
+}
+
+template <class R> int launch_euler(cfdb_euler* e, const void* U, void* Un, int64_t step) {
+  cfdb_ctx* ctx = e->ctx;
+  unsigned blocks = 0;
+  const auto f = form<box_euler_k<R>>(ctx);
+  const Box<R> g = box_of<R>(ctx, e->mesh, 1, 1, f.resident, &blocks);
+  const EulerArgs<R> a{static_cast<const R*>(U), static_cast<R*>(Un), R(e->gamma), e->mesh->dx, e->mesh->dy, e->mesh->dz,
+                       e->cfl, e->t_end, e->clock, (long long)step};
+  f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, a);
+  CFDB_LAUNCHED(ctx);
+  return CFDB_OK;
+}
+
+int box_euler_step(cfdb_euler* e, const void* U, void* Un, int64_t step) {
+  return e->dtype == CFDB_F64 ? launch_euler<double>(e, U, Un, step) : launch_euler<float>(e, U, Un, step);
 }
 
 template <class R, int OP, int OUT>

@@ -56,6 +56,9 @@ struct cfdb_euler {
 // The host-visible snapshot of the clock after `launches` launches.
 inline int euler_slot(int64_t launches) { return int(launches & 1); }
 
+// box_ops.cu: the plain step on structured meshes without face arrays
+int box_euler_step(cfdb_euler* e, const void* U, void* Un, int64_t step);
+
 __host__ __device__ inline double euler_dt(const double lam[3], double dx, double dy, double dz, double cfl,
                                            double t, double t_end, bool* last) {
   const double rate = (lam[0] / dx + lam[1] / dy) + lam[2] / dz;

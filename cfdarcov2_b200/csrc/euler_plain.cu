@@ -185,7 +185,12 @@ int euler_reduce_grid(const cfdb_euler* e) { return grid_for(e->ctx, e->mesh->n,
 int euler_plain_step(cfdb_euler* e, const void* U, void* Un, int64_t s) {
   cfdb_ctx* ctx = e->ctx;
   cfdb_mesh* m = e->mesh;
-  if (int rc = cfdb_mesh_need_plain(m, e->dtype)) return rc;
+  Geom geom = Geom::Arrays;
+  if (int rc = cfdb_mesh_geometry(m, e->dtype, false, &geom)) return rc;
+  if (geom == Geom::Box) {
+    if (int rc = box_euler_step(e, U, Un, s)) return rc;
+    return euler_reduce(e, Un, s, 0);
+  }
   const PlainGeomDev& p = m->plain[e->dtype == CFDB_F64 ? 1 : 0];
   const int grid = grid_for(ctx, m->n, kThreads, 8);
   if (e->dtype == CFDB_F64) {
@@ -205,11 +210,18 @@ int euler_reduce(cfdb_euler* e, const void* U, int64_t s, int begin_mode) {
   cfdb_ctx* ctx = e->ctx;
   cfdb_mesh* m = e->mesh;
   const void* vol = nullptr;
+  double vconst = m->dx * m->dy * m->dz;
   if (e->path == CFDB_PATH_PLAIN || !m->uniform) {
-    if (int rc = cfdb_mesh_need_plain(m, e->dtype)) return rc;
-    vol = m->plain[e->dtype == CFDB_F64 ? 1 : 0].volume;
+    Geom geom = Geom::Arrays;
+    if (int rc = cfdb_mesh_geometry(m, e->dtype, false, &geom)) return rc;
+    const int p = e->dtype == CFDB_F64 ? 1 : 0;
+    if (geom == Geom::Box) {  // no array: every cell's volume is v
+      vol = m->box[p].vol;
+      vconst = m->box[p].v;
+    } else {
+      vol = m->plain[p].volume;
+    }
   }
-  const double vconst = m->dx * m->dy * m->dz;
   const int grid = euler_reduce_grid(e);
   if (e->dtype == CFDB_F64)
     euler_reduce_k<double><<<grid, kThreads, 0, ctx->stream>>>((const double*)U, (const double*)vol, vconst, (long long)m->n,

@@ -146,3 +146,42 @@ def test_arrays_serve_when_nothing_else_can_be_built(cfdb, uniform, dtype):
     assert all(same_bits(a, b) for a, b in zip(results(m), want))
     ctx.set_alloc_budget(0)
     assert all(same_bits(a, b) for a, b in zip(results(m), want))
+
+
+@pytest.mark.parametrize("shape,spacing", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_euler_step_equals_the_face_arrays(cfdb, ctx, shape, spacing, dtype):
+    """The plain Euler step, dt and totals included: random states, momenta of
+    zero and far from the others' range, a cell that turns out not finite."""
+    m, a = pair(cfdb, ctx, shape, spacing)
+    n = m.n
+    code = cfdb.F64 if dtype == torch.float64 else cfdb.F32
+    rng = np.random.default_rng(12)
+    q = np.stack([rng.uniform(0.5, 2.0, n), *rng.standard_normal((3, n)), rng.uniform(20.0, 30.0, n)])
+    q[2, ::3] = 0.0
+    q[3, ::5] *= 1e-25
+    plain = torch.as_tensor(q.reshape(-1), dtype=dtype, device=DEV)
+    for i, bad in ((None, 0.0), (0 * n + n // 2, float("nan")), (2 * n + n // 3, float("inf")),
+                   (4 * n + n - 1, -float("inf")), (n // 2, -1.0)):
+        U = plain.clone()
+        if i is not None:
+            U[i] = bad
+        out = []
+        for mesh in (m, a):
+            e = cfdb.Euler(ctx, mesh, code, cfdb.PLAIN, 1.4, 0.4, 1e9, 100)
+            x, y = U.clone(), torch.full_like(U, 7.0)
+            e.begin(plain)  # a finite first dt
+            e.step(x, y)
+            if i is None:
+                for _ in range(2):
+                    x, y = y, x
+                    e.step(x, y)
+                out.append((y, e.status(), e.totals()))
+            else:
+                out.append((y, None, None))
+        ctx.sync()
+        (y0, s0, t0), (y1, s1, t1) = out
+        assert torch.equal(torch.isnan(y0), torch.isnan(y1)), i
+        assert torch.equal(torch.nan_to_num(y0, nan=0.0), torch.nan_to_num(y1, nan=0.0)), i
+        if i is None:
+            assert s0 == s1 and np.array_equal(t0, t1)
