@@ -172,19 +172,18 @@ HostSlots& host_slots() {
 }
 
 // Scratch of the synchronous reductions, held for the life of the context:
-// a 32-byte partial for up to 8 CTAs per SM from the pool, the ticket behind
-// the error word and a page-locked result.
+// a 32-byte partial for up to 8 CTAs per SM, the ticket behind the error word
+// and a page-locked result.  Not from the pool, whose first allocation maps
+// memory (about 1 ms) that many contexts never use.
 int make_reduce(cfdb_ctx* ctx) {
   const size_t parts = size_t(32) * 8 * size_t(std::max(1, ctx->num_sms));
-  CFDB_CUDA(ctx, cudaMallocFromPoolAsync(&ctx->reduce.part, parts, ctx->pool, ctx->stream));
+  CFDB_CUDA(ctx, cudaMalloc(&ctx->reduce.part, parts));
   ctx->reduce.ticket = reinterpret_cast<unsigned int*>(ctx->d_error + 2);
-  if (int rc = host_slots().take(ctx, &ctx->reduce.host)) return rc;
-  CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // the context's stream may change before the first use
-  return CFDB_OK;
+  return host_slots().take(ctx, &ctx->reduce.host);
 }
 
 void free_reduce(cfdb_ctx* ctx) {
-  if (ctx->reduce.part) cudaFreeAsync(ctx->reduce.part, ctx->stream);
+  if (ctx->reduce.part) cudaFree(ctx->reduce.part);
   host_slots().give(ctx->reduce.host);
 }
 }  // namespace
