@@ -205,10 +205,9 @@ template <int NY, int HY, int HZ> struct March {
     const unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= g.tiles * g.chunks) return false;  // whole warps
     const unsigned chunk = w / g.tiles, tile = w - chunk * g.tiles;
-    const int S = g.groups * g.nz;
-    int s = int(tile) * (32 - 2 * HZ) + int(lane) - HZ;
-    out = int(lane) >= HZ && int(lane) < 32 - HZ && s < S;
-    s = min(max(s, 0), S - 1);
+    const int64_t S = int64_t(g.groups) * g.nz, at = int64_t(tile) * (32 - 2 * HZ) + int(lane) - HZ;
+    out = int(lane) >= HZ && int(lane) < 32 - HZ && at < S;
+    const int s = int(min(max(at, int64_t(0)), S - 1));
     const int grp = s / g.nz;
     z = s - grp * g.nz;
     y0 = grp * NY;
