@@ -214,6 +214,8 @@ __device__ __forceinline__ void heat_columns2(const ProbDev& P, const ItemDev& I
 template <int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) batch_step_k(const ProbDev* __restrict__ probs, const ItemDev* __restrict__ items, int n_items,
                              const float* __restrict__ a, float* __restrict__ b, int heat_cols) {
+  stencil::grid_dep_wait();
+  stencil::grid_dep_launch();
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
     const ItemDev I = items[it];
     const ProbDev P = probs[I.prob];
@@ -382,6 +384,8 @@ __global__ void batch_ring_k(const ProbDev* __restrict__ probs, const ItemDev* _
     stencil::fence_mbar_init();
   }
   __syncthreads();
+  stencil::grid_dep_wait();
+  stencil::grid_dep_launch();
   bool bad = false;
   if (threadIdx.x < 32) {
     // Producer warp: lane s < S owns ring slot s and issues every plane
@@ -451,6 +455,9 @@ __global__ void batch_ring_k(const ProbDev* __restrict__ probs, const ItemDev* _
 
 constexpr int64_t kPoolPad = 4;  // spare floats before the first and after the last problem of a pool
 // kernel forms (cfdb_batch_set_staged)
+// Steps per recorded graph (even: every replay starts from pool a); a remainder is
+// launched directly.
+constexpr int32_t kGraphSteps = 16;
 constexpr int kFormMarch = 0, kFormRing = 1, kFormMarch48 = 2;
 
 struct cfdb_batch {
@@ -527,6 +534,28 @@ bool ring_ok(const cfdb_batch* b, int threads, int ctas_per_sm, const void* a, c
   return ring_slots(threads, ctas_per_sm, b->nmax) > 0 && (threads + 32) * ctas_per_sm <= 2048;
 }
 
+// A step of up to 12 items per CTA is launched with programmatic stream
+// serialisation: its CTAs come up as the previous step's leave and wait for all of it
+// before they touch the pools.  With 16 steps per graph instead of two, us per step:
+// 26 mixed cubes of 20 to 51 cells 8.5 -> 7.6, 29 wave cubes of 16 to 29 6.3 -> 5.9,
+// 16 heat cubes of 16 to 40 4.1 -> 3.1 (two-step graphs had kept the host busy), 96
+// wave cubes of 20 to 50 (6 items per CTA) 34.5 -> 33.7, 96 mixed of 16 to 96 (8)
+// 73.2 -> 72.7; 64 wave cubes of 64 (14) lose 0.8 % with it.
+template <class... P, class... A>
+cudaError_t launch_step(void (*kern)(P...), int n_items, int grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = n_items <= 12 * int64_t(grid) ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 int launch(cfdb_batch* b, const void* a, void* out) {
   const int grid = std::max(1, b->ctx->num_sms) * b->ctas_per_sm;
   if (b->staged == kFormRing && ring_ok(b, b->threads, b->ctas_per_sm, a, out)) {
@@ -550,17 +579,14 @@ int launch(cfdb_batch* b, const void* a, void* out) {
     }
     const int rgrid = std::max(1, b->ctx->num_sms) * std::min(b->ctas_per_sm, b->ring_resident);
     RingArgs A{b->threads, ring_cap(b->threads, b->nmax), b->ctx->wait_cycles};
-    kern<<<rgrid, b->threads + 32, smem, b->ctx->stream>>>(b->d_probs, b->d_items, b->n_items,
-                                                           static_cast<const float*>(a), static_cast<float*>(out), A,
-                                                           b->ctx->d_error);
+    CFDB_CUDA(b->ctx, launch_step(kern, b->n_items, rgrid, b->threads + 32, smem, b->ctx->stream, b->d_probs, b->d_items, b->n_items,
+                                  static_cast<const float*>(a), static_cast<float*>(out), A, b->ctx->d_error));
   } else if (b->staged == kFormMarch48 && b->threads <= 256) {
-    batch_step_k<256, 5><<<grid, b->threads, 0, b->ctx->stream>>>(b->d_probs, b->d_items, b->n_items,
-                                                                   static_cast<const float*>(a), static_cast<float*>(out),
-                                                                   b->heat_cols);
+    CFDB_CUDA(b->ctx, launch_step(batch_step_k<256, 5>, b->n_items, grid, b->threads, 0, b->ctx->stream, b->d_probs, b->d_items,
+                                  b->n_items, static_cast<const float*>(a), static_cast<float*>(out), b->heat_cols));
   } else {
-    batch_step_k<1024, 1><<<grid, b->threads, 0, b->ctx->stream>>>(b->d_probs, b->d_items, b->n_items,
-                                                                    static_cast<const float*>(a), static_cast<float*>(out),
-                                                                    b->heat_cols);
+    CFDB_CUDA(b->ctx, launch_step(batch_step_k<1024, 1>, b->n_items, grid, b->threads, 0, b->ctx->stream, b->d_probs, b->d_items,
+                                  b->n_items, static_cast<const float*>(a), static_cast<float*>(out), b->heat_cols));
   }
   CFDB_LAUNCHED(b->ctx);
   return CFDB_OK;
@@ -761,9 +787,9 @@ extern "C" int cfdb_batch_run(cfdb_batch* b, void* a, void* out, int32_t steps, 
     }
     return CFDB_OK;
   }
-  // (re)record the two-step graph a -> out -> a when pools or config changed
-  if (!b->graph || b->graph_a != a || b->graph_b != out || b->graph_cfg[0] != b->cells_per_item ||
-      b->graph_cfg[1] != b->threads || b->graph_cfg[2] != b->ctas_per_sm) {
+  // (re)record the graph of kGraphSteps steps a -> out -> a ... when pools or config changed
+  if (steps >= kGraphSteps && (!b->graph || b->graph_a != a || b->graph_b != out || b->graph_cfg[0] != b->cells_per_item ||
+      b->graph_cfg[1] != b->threads || b->graph_cfg[2] != b->ctas_per_sm)) {
     drop_graph(b);
     cfdb_ctx* ctx = b->ctx;
     if (!ctx->capture_stream)
@@ -775,8 +801,7 @@ extern "C" int cfdb_batch_run(cfdb_batch* b, void* a, void* out, int32_t steps, 
     const int64_t before = ctx->launches;  // recorded launches run only when replayed
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      rc = launch(b, a, out);
-      if (!rc) rc = launch(b, out, a);
+      for (int32_t k = 0; k < kGraphSteps && !rc; ++k) rc = (k & 1) ? launch(b, out, a) : launch(b, a, out);
       cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &g);
       if (!rc && e2 != cudaSuccess) rc = cfdb_cuda_fail(ctx, e2, "cudaStreamEndCapture");
     } else {
@@ -798,13 +823,14 @@ extern "C" int cfdb_batch_run(cfdb_batch* b, void* a, void* out, int32_t steps, 
     b->graph_b = out;
     b->graph_cfg[0] = b->cells_per_item; b->graph_cfg[1] = b->threads; b->graph_cfg[2] = b->ctas_per_sm;
   }
-  for (int32_t k = 0; k + 1 < steps; k += 2) {
+  int32_t k = 0;
+  for (; k + kGraphSteps <= steps; k += kGraphSteps) {
     CFDB_CUDA(b->ctx, cudaGraphLaunch(b->graph, b->ctx->stream));
-    b->last_launches += 2;
-    b->ctx->launches += 2;
+    b->last_launches += kGraphSteps;
+    b->ctx->launches += kGraphSteps;
   }
-  if (steps & 1) {
-    if (int rc = launch(b, a, out)) return rc;
+  for (; k < steps; ++k) {
+    if (int rc = (k & 1) ? launch(b, out, a) : launch(b, a, out)) return rc;
     ++b->last_launches;
   }
   return CFDB_OK;

@@ -397,7 +397,7 @@ int cfdb_batch_tune(cfdb_batch* b, void* pool_a, void* pool_b, const char* cache
 /* One step a -> b (one persistent launch). */
 int cfdb_batch_step(cfdb_batch* b, const void* pool_a, void* pool_b);
 /* steps steps alternating a -> b -> a ...; use_graph replays a captured
- * two-step CUDA graph.  The final state is in a when steps is even. */
+ * CUDA graph of 16 steps (a remainder is launched directly).  The final state is in a when steps is even. */
 int cfdb_batch_run(cfdb_batch* b, void* pool_a, void* pool_b, int32_t steps, int use_graph);
 /* Kernel launches the last cfdb_batch_run enqueued (graph replays count their nodes). */
 int cfdb_batch_launch_count(const cfdb_batch* b, int64_t* out);
