@@ -172,18 +172,19 @@ HostSlots& host_slots() {
 }
 
 // Scratch of the synchronous reductions, held for the life of the context:
-// a 32-byte partial for up to 8 CTAs per SM, the ticket behind the error word
-// and a page-locked result.  Not from the pool, whose first allocation maps
-// memory (about 1 ms) that many contexts never use.
+// a 32-byte partial for up to 8 CTAs per SM and the ticket behind the error
+// word, and a page-locked result.  Not from the pool, whose first allocation
+// maps memory (about 1 ms) that many contexts never use.
+constexpr size_t kErrorBytes = 4 * sizeof(int), kPartOffset = 256;
+size_t part_bytes(const cfdb_ctx* ctx) { return size_t(32) * 8 * size_t(std::max(1, ctx->num_sms)); }
+
 int make_reduce(cfdb_ctx* ctx) {
-  const size_t parts = size_t(32) * 8 * size_t(std::max(1, ctx->num_sms));
-  CFDB_CUDA(ctx, cudaMalloc(&ctx->reduce.part, parts));
+  ctx->reduce.part = reinterpret_cast<char*>(ctx->d_error) + kPartOffset;
   ctx->reduce.ticket = reinterpret_cast<unsigned int*>(ctx->d_error + 2);
   return host_slots().take(ctx, &ctx->reduce.host);
 }
 
 void free_reduce(cfdb_ctx* ctx) {
-  if (ctx->reduce.part) cudaFree(ctx->reduce.part);
   host_slots().give(ctx->reduce.host);
 }
 }  // namespace
@@ -273,13 +274,16 @@ extern "C" int cfdb_ctx_create(int device, cfdb_ctx** out) {
   if (!ctx) return cfdb_fail(nullptr, CFDB_ENOMEM, "cfdb_ctx_create: host allocation failed");
   ctx->device = device;
   cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
-  int rc = cfdb_dev_alloc(ctx, sizeof(int) * 4, reinterpret_cast<void**>(&ctx->d_error));
-  if (rc) {
-    g_err_noctx = ctx->err;
+  int rc = CFDB_OK;
+  e = cudaMalloc(reinterpret_cast<void**>(&ctx->d_error), kPartOffset + part_bytes(ctx));
+  if (e != cudaSuccess) {
+    rc = cfdb_cuda_fail(nullptr, e, "cudaMalloc");
     delete ctx;
     return rc;
   }
-  e = cudaMemset(ctx->d_error, 0, sizeof(int) * 4);
+  ctx->allocs[ctx->d_error] = kErrorBytes;  // what a budget counts
+  ctx->allocated += kErrorBytes;
+  e = cudaMemset(ctx->d_error, 0, kErrorBytes);
   if (e != cudaSuccess) {
     int r = cfdb_cuda_fail(nullptr, e, "cudaMemset");
     cfdb_dev_free(ctx, ctx->d_error);
