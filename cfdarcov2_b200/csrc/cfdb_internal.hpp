@@ -129,6 +129,7 @@ struct cfdb_ctx {
     void* part = nullptr;
     unsigned int* ticket = nullptr;
     void* host = nullptr;
+    unsigned long long host_id = 0;  // the CUDA context `host` was locked in
     std::mutex mu;
   } reduce;
   int* d_error = nullptr;  // device error word written by bounded waits

@@ -134,37 +134,66 @@ int make_pool(cfdb_ctx* ctx) {
 }
 
 // Page-locked words the reduction kernels store their results to, one slot of
-// 64 bytes per context, from one page per process (page-locking costs 0.4 ms,
-// as much as the rest of a context).  The page stays for the life of the
-// process; slots go back when a context is destroyed, and a context beyond
-// the page's slots gets memory of its own.
+// 64 bytes per context, from one page per CUDA context (page-locking costs 0.4
+// ms, as much as the rest of a library context).  A page lives as long as the
+// CUDA context it was locked in: after cudaDeviceReset it is gone, and the next
+// context must not be handed its address, so pages carry the CUDA context's id,
+// which the driver never uses again.  Slots go back when a library context is
+// destroyed; one beyond the page's slots gets memory of its own.
 class HostSlots {
  public:
-  int take(cfdb_ctx* ctx, void** out) {
+  int take(cfdb_ctx* ctx, void** out, unsigned long long* id) {
     std::lock_guard<std::mutex> lock(mu_);
-    if (!page_) CFDB_CUDA(ctx, cudaHostAlloc(&page_, kSlots * 64, cudaHostAllocPortable | cudaHostAllocMapped));
-    for (int k = 0; k < kSlots; ++k)
-      if (!used_[k]) {
-        used_[k] = true;
-        *out = static_cast<char*>(page_) + 64 * k;
-        return CFDB_OK;
+    *id = current_id();
+    if (*id != 0 && ctx->device >= 0 && ctx->device < kMaxDevices) {
+      Page& p = pages_[ctx->device];
+      if (p.id != *id) p = Page();  // of a CUDA context that is gone, and the memory with it
+      if (!p.base) {
+        CFDB_CUDA(ctx, cudaHostAlloc(&p.base, kSlots * 64, cudaHostAllocPortable | cudaHostAllocMapped));
+        p.id = *id;
       }
+      for (int k = 0; k < kSlots; ++k)
+        if (!p.used[k]) {
+          p.used[k] = true;
+          *out = static_cast<char*>(p.base) + 64 * k;
+          return CFDB_OK;
+        }
+    }
     CFDB_CUDA(ctx, cudaHostAlloc(out, 64, cudaHostAllocPortable | cudaHostAllocMapped));
     return CFDB_OK;
   }
-  void give(void* p) {
-    if (!p) return;
+  // with the context's device current
+  void give(const cfdb_ctx* ctx, void* q, unsigned long long id) {
+    if (!q) return;
     std::lock_guard<std::mutex> lock(mu_);
-    const ptrdiff_t off = static_cast<char*>(p) - static_cast<char*>(page_);
-    if (page_ && off >= 0 && off < kSlots * 64) used_[off / 64] = false;
-    else cudaFreeHost(p);
+    if (id != current_id()) return;  // went with its CUDA context
+    if (ctx->device >= 0 && ctx->device < kMaxDevices) {
+      Page& p = pages_[ctx->device];
+      const ptrdiff_t off = static_cast<char*>(q) - static_cast<char*>(p.base);
+      if (p.base && p.id == id && off >= 0 && off < kSlots * 64) {
+        p.used[off / 64] = false;
+        return;
+      }
+    }
+    cudaFreeHost(q);
   }
 
  private:
   static constexpr int kSlots = 64;
+  struct Page {
+    void* base = nullptr;
+    unsigned long long id = 0;
+    bool used[kSlots] = {};
+  };
+  // Id of the current CUDA context, 0 where the driver does not say.
+  static unsigned long long current_id() {
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static const GetId get = driver_fn<GetId>("cuCtxGetId");
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+  }
   std::mutex mu_;
-  void* page_ = nullptr;
-  bool used_[kSlots] = {};
+  Page pages_[kMaxDevices];
 };
 HostSlots& host_slots() {
   static HostSlots* s = new HostSlots();  // not destroyed: contexts may outlive static destructors
@@ -181,11 +210,11 @@ size_t part_bytes(const cfdb_ctx* ctx) { return size_t(32) * 8 * size_t(std::max
 int make_reduce(cfdb_ctx* ctx) {
   ctx->reduce.part = reinterpret_cast<char*>(ctx->d_error) + kPartOffset;
   ctx->reduce.ticket = reinterpret_cast<unsigned int*>(ctx->d_error + 2);
-  return host_slots().take(ctx, &ctx->reduce.host);
+  return host_slots().take(ctx, &ctx->reduce.host, &ctx->reduce.host_id);
 }
 
 void free_reduce(cfdb_ctx* ctx) {
-  host_slots().give(ctx->reduce.host);
+  host_slots().give(ctx, ctx->reduce.host, ctx->reduce.host_id);
 }
 }  // namespace
 
