@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(WARPS * 32, 512 / (WARPS * 32))
 #pragma unroll
         for (int r = 0; r < kRows; ++r) {
           if (x == g.X - 1) up[r] = c[s][r];
-          if (x == 0) e[s][r] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+          if (x == 0) e[s][r] = c[s][r] - c[s][r];  // the wall neighbour is the cell itself (NaN for an infinity)
         }
       }
       const float* lev =

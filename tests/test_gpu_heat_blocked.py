@@ -46,3 +46,27 @@ def test_passes_without_a_workspace(cfdb):
         assert torch.equal(ctx.heat_run(m, a, b, 0.01, 1e-4, steps), want)
         ctx.set_alloc_budget(0)
     ctx.sync()
+
+
+@pytest.mark.parametrize("k", [0.01, -0.01])
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan"), 3e38])
+def test_passes_on_values_that_are_not_finite(cfdb, ctx, k, value):
+    """Infinities on and beside every wall, with a conductivity of either sign
+    (a negative one adds infinities of one sign, so a wall's inf - inf is what
+    makes the cell NaN): the one-step sweep's results."""
+    X, Y, Z = 40, 130, 68
+    m = cfdb.Mesh.structured(ctx, X, Y, Z, 1 / X, 1 / Y, 1 / Z)
+    T0 = torch.as_tensor(np.random.default_rng(3).uniform(-1, 1, (X, Y, Z)), dtype=torch.float32, device=DEV)
+    for i in ((0, 5, 5), (0, 0, 0), (X - 1, 60, 30), (20, 0, 7), (20, Y - 1, 40), (9, 77, 0), (30, 99, Z - 1), (11, 40, 33)):
+        T0[i] = value
+    T0 = T0.reshape(-1).contiguous()
+    dt = 0.1 * min(1 / X, 1 / Y, 1 / Z) ** 2 / 0.01
+    p, q = T0.clone(), torch.empty_like(T0)
+    for steps in range(1, 6):
+        ctx.heat_step(m, p, q, k, dt)
+        p, q = q, p
+        a, b = T0.clone(), torch.empty_like(T0)
+        got = ctx.heat_run(m, a, b, k, dt, steps)
+        assert torch.equal(torch.isnan(got), torch.isnan(p)), steps
+        assert torch.equal(torch.nan_to_num(got, nan=0.0), torch.nan_to_num(p, nan=0.0)), steps
+    ctx.sync()
