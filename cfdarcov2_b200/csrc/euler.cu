@@ -457,8 +457,10 @@ extern "C" int cfdb_euler_run(cfdb_euler* e, void* Ua, void* Ub, int64_t check_e
   // Steps enqueued before the next clock check: at most check_every, a first few
   // to learn dt, then what the mean dt so far says is left.  A launch past t_end
   // still costs 4 to 5 us (it has to run to find the clock finished), a check
-  // about 12.
-  int64_t batch = std::min<int64_t>(check_every, 16);
+  // about 12.  A later run needs an even launch count, so batches of an even
+  // check_every stay even; an odd one is taken as it is.
+  const bool even_batches = check_every % 2 == 0;
+  int64_t batch = even_batches ? std::min<int64_t>(check_every, 16) : check_every;
   while (!finished) {
     for (int64_t k = 0; k < batch; ++k) {
       const bool even = (e->launches & 1) == 0;
@@ -469,7 +471,7 @@ extern "C" int cfdb_euler_run(cfdb_euler* e, void* Ua, void* Ub, int64_t check_e
     finished = r.finished;
     steps = r.steps;
     const double left = r.t > 0 ? std::ceil((e->t_end - r.t) / r.t * double(steps)) + 1.0 : double(check_every);
-    batch = left < double(check_every) ? std::max<int64_t>(1, int64_t(left)) : check_every;
+    batch = even_batches && left < double(check_every) ? std::max<int64_t>(1, int64_t(left) + 1) & ~int64_t(1) : check_every;
     // the conservation totals of the latest step double as the health check:
     // a NaN or Inf anywhere in the state reaches them (and would otherwise
     // end the run early through a non-finite dt)

@@ -155,3 +155,35 @@ def test_euler_rejects_bad_arguments(cfdb, ctx):
     assert ei.value.code == cfdb.capi.EUNSUPPORTED  # nz % 4 != 0 on the TMA path
     with pytest.raises(cfdb.CfdbError):
         cfdb.Euler(ctx, m, dtype=cfdb.F32, path=cfdb.PLAIN, gamma=1.0)
+
+
+@pytest.mark.parametrize("path", ["plain", "fused"])
+@pytest.mark.parametrize("t_end", [0.004, 0.01, 0.021, 0.033, 0.047, 0.06, 0.075])
+def test_run_again_on_a_finished_solver(cfdb, ctx, path, t_end):
+    """A second run of a finished solver returns the same state, whatever
+    number of steps the first one took; after an odd check_every the launch
+    count's parity decides, as it always did."""
+    U0, dx, dy, dz = sod(64, 8, 8)
+    m = cfdb.Mesh.structured(ctx, 64, 8, 8, dx, dy, dz)
+    code, dtype = (cfdb.F64, torch.float64) if path == "plain" else (cfdb.F32, torch.float32)
+    e = cfdb.Euler(ctx, m, code, cfdb.PLAIN if path == "plain" else cfdb.FUSED, 1.4, 0.4, t_end, 1000)
+    a = torch.tensor(U0, dtype=dtype, device=DEV)
+    b = torch.empty_like(a)
+    for check_every in (64, 16, 2, 20):
+        a.copy_(torch.tensor(U0, dtype=dtype))
+        e.begin(a)
+        first = e.run(a, b, check_every)
+        state = (b if first[1] else a).clone()
+        for again in (64, 16, 2):
+            assert e.run(a, b, again) == first
+            assert torch.equal(b if first[1] else a, state)
+        assert e.status() == (t_end, first[0], True)
+    for check_every in (1, 3):
+        a.copy_(torch.tensor(U0, dtype=dtype))
+        e.begin(a)
+        assert e.run(a, b, check_every) == first
+        if -(-first[0] // check_every) * check_every % 2 == 0:
+            assert e.run(a, b, check_every) == first
+        else:
+            with pytest.raises(cfdb.CfdbError):
+                e.run(a, b, check_every)
