@@ -1465,9 +1465,7 @@ int vert_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* T, void* 
 }
 
 template <class R> int launch_vert_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask) {
-  FaceGeomDev& b = m->faces[sizeof(R) == 8 ? 1 : 0];
-  if (!b.grad)
-    if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(R)) * 3 * m->n, &b.grad)) return rc;
+  const FaceGeomDev& b = m->faces[sizeof(R) == 8 ? 1 : 0];
   if (int rc = launch_vert_sum<R, OP_GRAD, OUT_GRADIENT>(ctx, m, phi, b.grad, 7, 0, 0)) return rc;
   unsigned blocks = 0;
   const auto f = form<vert_stab_k<R>>(ctx);

@@ -83,13 +83,14 @@ struct BoxGeomDev {
 struct FaceGeomDev {
   int state = 0;  // 0 not built, 1 usable, 2 this mesh keeps the N x 6 arrays
   int64_t count[3] = {};
-  void* block = nullptr;  // holds all of the following but grad
+  void* block = nullptr;  // holds all of the following
   void* normal[3] = {};
   void* area[3] = {};
   void* alpha[3] = {};
   void* len = nullptr;
   void* vol = nullptr;
-  void* grad = nullptr;  // 3 n, allocated on the first stab call
+  void* grad = nullptr;  // 3 n, the stabilisation's first stage: there with the
+                         // geometry, so that a recorded or budgeted call needs nothing more
 };
 
 // Compact FP32 geometry of vertex meshes for the fused kernels: per cell the

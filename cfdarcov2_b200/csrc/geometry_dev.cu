@@ -148,7 +148,7 @@ template <class T> int build_faces(cfdb_mesh* m, FaceGeomDev& b) {
     oa[d] = take(b.count[d]);
     ol[d] = take(b.count[d]);
   }
-  const int64_t olen = take(6 * m->n), ovol = take(m->n);
+  const int64_t olen = take(6 * m->n), ovol = take(m->n), ograd = take(3 * m->n);
   if (int rc = cfdb_dev_alloc(ctx, size, &b.block)) return rc;
   auto part = [&](int64_t at) { return reinterpret_cast<T*>(static_cast<char*>(b.block) + at); };
   FaceArrays<T> a{};
@@ -160,6 +160,7 @@ template <class T> int build_faces(cfdb_mesh* m, FaceGeomDev& b) {
   }
   b.len = a.len = part(olen);
   b.vol = a.vol = part(ovol);
+  b.grad = part(ograd);
   void* dverts = nullptr;
   const int64_t vb = int64_t(sizeof(double)) * int64_t(m->verts.size());
   if (int rc = cfdb_dev_alloc(ctx, vb, &dverts)) return rc;

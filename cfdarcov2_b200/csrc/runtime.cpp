@@ -532,7 +532,6 @@ extern "C" int cfdb_mesh_create_from_vertices(cfdb_ctx* ctx, int64_t nx, int64_t
 
 static void free_faces(cfdb_ctx* ctx, FaceGeomDev& b) {
   cfdb_dev_free(ctx, b.block);
-  cfdb_dev_free(ctx, b.grad);
   b = FaceGeomDev();
 }
 

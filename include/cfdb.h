@@ -190,8 +190,8 @@ int cfdb_op_grad(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, const void* phi, voi
 int cfdb_op_lapl(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, const void* phi, void* out, int dims_mask);
 
 /* StabVar::evaluate_cu -> eval_stab (src/fvm3d.cpp:938-941; src/cuda_operators.cu:307-487).
- * Vertex meshes hold a mesh-owned 3N temporary from the first call on (18N where
- * the N x 6 geometry serves). */
+ * Vertex meshes hold a mesh-owned 3N temporary beside their geometry (18N, from
+ * the first call on, where the N x 6 geometry serves). */
 int cfdb_op_stab(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, const void* phi, void* out, int dims_mask);
 
 /* add_mtrx / sub_mtrx / mul_mtrx / div_mtrx (src/cuda_operators.cu:27-106);
