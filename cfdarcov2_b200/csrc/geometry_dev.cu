@@ -48,9 +48,7 @@ __global__ void __launch_bounds__(128) plain_geometry_k(Lattice L, int mode, T* 
 
 }  // namespace
 
-// Allocates and fills p (and m->d_ids when it is not built yet) on the
-// context's stream; synchronises before returning.
-int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p) {
+static int build_plain(cfdb_mesh* m, int dtype, PlainGeomDev& p, double** verts) {
   cfdb_ctx* ctx = m->ctx;
   const int64_t n = m->n;
   if (6 * n > int64_t(INT32_MAX)) return cfdb_fail(ctx, CFDB_EUNSUPPORTED, "mesh too large for int32 face ids");
@@ -62,13 +60,12 @@ int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p) {
   const bool need_ids = m->d_ids == nullptr;
   if (need_ids)
     if (int rc = cfdb_dev_alloc(ctx, int64_t(sizeof(int32_t)) * 6 * n, reinterpret_cast<void**>(&m->d_ids))) return rc;
-  double* dverts = nullptr;
   if (!m->uniform) {
     const int64_t bytes = int64_t(sizeof(double)) * int64_t(m->verts.size());
-    if (int rc = cfdb_dev_alloc(ctx, bytes, reinterpret_cast<void**>(&dverts))) return rc;
-    CFDB_CUDA(ctx, cudaMemcpyAsync(dverts, m->verts.data(), size_t(bytes), cudaMemcpyHostToDevice, ctx->stream));
+    if (int rc = cfdb_dev_alloc(ctx, bytes, reinterpret_cast<void**>(verts))) return rc;
+    CFDB_CUDA(ctx, cudaMemcpyAsync(*verts, m->verts.data(), size_t(bytes), cudaMemcpyHostToDevice, ctx->stream));
   }
-  const Lattice L{m->nx, m->ny, m->nz, m->dx, m->dy, m->dz, dverts};
+  const Lattice L{m->nx, m->ny, m->nz, m->dx, m->dy, m->dz, *verts};
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const int64_t want = (n + 127) / 128;
@@ -84,11 +81,24 @@ int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p) {
         L, m->geom_mode, static_cast<float*>(p.normal), static_cast<float*>(p.normal_alt),
         static_cast<float*>(p.area), static_cast<float*>(p.alpha), static_cast<float*>(p.len),
         static_cast<float*>(p.volume), static_cast<float*>(p.isb), ids);
-  CFDB_CUDA(ctx, cudaGetLastError());
   CFDB_LAUNCHED(ctx);
   CFDB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  cfdb_dev_free(ctx, dverts);
   return CFDB_OK;
+}
+
+// Allocates and fills p (and m->d_ids when it is not built yet) on the
+// context's stream; synchronises before returning.  Ids that a failed build
+// has not filled must not be there for the next one.
+int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p) {
+  const bool had_ids = m->d_ids != nullptr;
+  double* verts = nullptr;
+  const int rc = build_plain(m, dtype, p, &verts);
+  cfdb_dev_free(m->ctx, verts);
+  if (rc && !had_ids) {
+    cfdb_dev_free(m->ctx, m->d_ids);
+    m->d_ids = nullptr;
+  }
+  return rc;
 }
 
 // ---- every face once ---------------------------------------------------------

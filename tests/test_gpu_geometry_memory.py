@@ -43,3 +43,29 @@ def test_stab_after_a_heat_step_needs_no_memory(cfdb, uniform, dtype):
     ctx.set_stream(torch.cuda.current_stream().cuda_stream)
     graph.replay()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_arrays_built_after_a_build_that_ran_out_of_memory(cfdb, dtype):
+    """A first build that finds no room for any one of its allocations leaves
+    nothing behind that a later one would take for filled."""
+    ctx = cfdb.Context(0)
+    es = 4 if dtype == torch.float32 else 8
+    want = None
+    for short in (0, 1, 2):
+        m = make(cfdb, ctx, False)
+        q = torch.as_tensor(np.random.default_rng(2).standard_normal(4 * m.n), dtype=dtype, device=DEV)
+        out = torch.empty_like(q)
+        if short:
+            arrays = 56 * m.n * es + (24 * m.n if short == 2 else 0)
+            ctx.set_alloc_budget(ctx.allocated_bytes() + arrays + 64)
+            with pytest.raises(cfdb.CfdbError) as e:
+                ctx.wave_step(m, q, out, 1e-3, path=cfdb.PLAIN)
+            assert e.value.code == cfdb.capi.ENOMEM
+            ctx.set_alloc_budget(0)
+        ctx.wave_step(m, q, out, 1e-3, path=cfdb.PLAIN)
+        ctx.sync()
+        m.close()
+        want = out if want is None else want
+        assert torch.equal(out, want)
+    ctx.sync()
