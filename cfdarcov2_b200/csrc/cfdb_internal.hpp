@@ -268,11 +268,18 @@ int cfdb_mesh_need_plain(cfdb_mesh* m, int dtype);
 // All give the same bits: the tables of a structured mesh (box_ops.cu), a vertex
 // mesh's faces held once (vertex_faces: the operator has such a kernel), or the
 // N x 6 arrays.  Where the arrays are there already, they serve while the stream
-// records a graph; a failed allocation of the others falls back to them.
+// records a graph; a failed allocation of the others falls back to them.  Other
+// calls on the mesh may want the arrays later, so where the budget or the device has
+// room for the arrays (and `array_scratch` bytes that the operator needs with them)
+// but not for both, the arrays serve from the start.
 enum class Geom { Arrays, Box, Faces };
-int cfdb_mesh_geometry(cfdb_mesh* m, int dtype, bool vertex_faces, Geom* geom);
+int cfdb_mesh_geometry(cfdb_mesh* m, int dtype, bool vertex_faces, Geom* geom, int64_t array_scratch = 0);
 // fills the plain arrays of dtype on the device (geometry_dev.cu)
 int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p);
+// Device bytes that the arrays still want (0 when they are there), and those of the
+// tables or the faces held once (geometry_dev.cu).
+int64_t cfdb_plain_bytes(const cfdb_mesh* m, int dtype);
+int64_t cfdb_table_bytes(const cfdb_mesh* m, int dtype);
 // samples and checks the lattice constants on the device (geometry_dev.cu)
 int cfdb_check_lattice_device(cfdb_mesh* m, cfdb_lattice_geometry* out);
 int cfdb_mesh_need_compact(cfdb_mesh* m);

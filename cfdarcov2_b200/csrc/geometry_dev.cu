@@ -101,6 +101,18 @@ int cfdb_build_plain_device(cfdb_mesh* m, int dtype, PlainGeomDev& p) {
   return rc;
 }
 
+int64_t cfdb_plain_bytes(const cfdb_mesh* m, int dtype) {
+  if (m->plain[dtype == CFDB_F64 ? 1 : 0].ready) return 0;
+  return (dtype == CFDB_F64 ? 8 : 4) * 56 * m->n + (m->d_ids ? 0 : int64_t(sizeof(int32_t)) * 6 * m->n);
+}
+
+int64_t cfdb_table_bytes(const cfdb_mesh* m, int dtype) {
+  const int64_t es = dtype == CFDB_F64 ? 8 : 4;
+  if (m->uniform) return es * m->n + 48 * (m->nx + m->ny + m->nz) + 1024;  // five tables per axis, the volumes
+  const int64_t faces = (m->nx + 1) * m->ny * m->nz + m->nx * (m->ny + 1) * m->nz + m->nx * m->ny * (m->nz + 1);
+  return es * (5 * faces + 10 * m->n) + 12 * 256;
+}
+
 // ---- every face once ---------------------------------------------------------
 namespace {
 

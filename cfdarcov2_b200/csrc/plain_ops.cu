@@ -504,12 +504,15 @@ __global__ void wave_adjoint_plain_k(PlainArgs<R> g, const R* __restrict__ q, co
 }
 
 // Checks a mesh operator's handles and builds the N x 6 arrays, or with `geom`
-// given whichever geometry serves.
-int need(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, Geom* geom = nullptr) {
+// given whichever geometry serves (array_scratch: values per cell that the operator
+// holds beside the arrays).
+int need(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, Geom* geom = nullptr, int array_scratch = 0) {
   if (int rc = cfdb_check_mesh(ctx, m)) return rc;
   if (!dtype_ok(dtype)) return cfdb_fail(ctx, CFDB_EINVAL, "unknown dtype %d", dtype);
   CFDB_CUDA(ctx, cudaSetDevice(ctx->device));
-  return geom ? cfdb_mesh_geometry(m, dtype, true, geom) : cfdb_mesh_need_plain(m, dtype);
+  if (!geom) return cfdb_mesh_need_plain(m, dtype);
+  if (m->plain[dtype == CFDB_F64 ? 1 : 0].stab_tmp) array_scratch = 0;
+  return cfdb_mesh_geometry(m, dtype, true, geom, int64_t(dtype_size(dtype)) * array_scratch * m->n);
 }
 
 int check_ptrs(cfdb_ctx* ctx, const char* fn, std::initializer_list<const void*> ps) {
@@ -581,7 +584,7 @@ extern "C" int cfdb_op_lapl(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* 
 
 extern "C" int cfdb_op_stab(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* phi, void* out, int mask) {
   Geom geom = Geom::Arrays;
-  if (int rc = need(ctx, m, dtype, &geom)) return rc;
+  if (int rc = need(ctx, m, dtype, &geom, 18)) return rc;
   if (int rc = check_ptrs(ctx, "cfdb_op_stab", {phi, out})) return rc;
   if (mask < 0 || mask > 7) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_op_stab: dims_mask %d out of range", mask);
   if (geom == Geom::Box) return box_stab(ctx, m, dtype, phi, out, mask);

@@ -684,17 +684,29 @@ int cfdb_mesh_need_faces(cfdb_mesh* m, int dtype, bool* usable) {
   return CFDB_OK;
 }
 
-int cfdb_mesh_geometry(cfdb_mesh* m, int dtype, bool vertex_faces, Geom* geom) {
+int cfdb_mesh_geometry(cfdb_mesh* m, int dtype, bool vertex_faces, Geom* geom, int64_t array_scratch) {
   cfdb_ctx* ctx = m->ctx;
   const int p = dtype == CFDB_F64 ? 1 : 0;
   *geom = Geom::Arrays;
   bool look = m->uniform || vertex_faces;
-  if (look && m->plain[p].ready && (m->uniform ? m->box[p].state : m->faces[p].state) == 0) {
-    // building allocates and copies, which a recording stream does not take
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &st);
-    if (e != cudaSuccess) cudaGetLastError();
-    look = e == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  if (look && (m->uniform ? m->box[p].state : m->faces[p].state) == 0) {
+    if (m->plain[p].ready) {
+      // building allocates and copies, which a recording stream does not take
+      cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+      const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &st);
+      if (e != cudaSuccess) cudaGetLastError();
+      look = e == cudaSuccess && st == cudaStreamCaptureStatusNone;
+    }
+    const int64_t arrays = cfdb_plain_bytes(m, dtype), both = arrays + cfdb_table_bytes(m, dtype);
+    int64_t room = ctx->budget > 0 ? ctx->budget - ctx->allocated : INT64_MAX;
+    size_t left = 0, total = 0;
+    if (look && both > int64_t(4) << 30) {  // the query is worth its time only on a large mesh
+      if (cudaMemGetInfo(&left, &total) == cudaSuccess) room = std::min(room, int64_t(left));
+      else cudaGetLastError();
+    }
+    // a vertex mesh's vertices are on the device while either is built
+    const int64_t verts = arrays ? int64_t(sizeof(double)) * int64_t(m->verts.size()) : 0;
+    if (arrays + std::max(array_scratch, verts) <= room && both + verts > room) look = false;
   }
   if (look) {
     bool usable = false;

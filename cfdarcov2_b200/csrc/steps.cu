@@ -22,12 +22,13 @@ extern "C" int cfdb_heat_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int path, 
   if (!std::isfinite(k) || !std::isfinite(dt)) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_heat_step: k and dt must be finite");
   if (path == CFDB_PATH_FUSED) return fused_heat_step(ctx, m, dtype, T, Tn, k, dt);
   Geom geom = Geom::Arrays;
-  if (int rc = cfdb_mesh_geometry(m, dtype, true, &geom)) return rc;
+  PlainGeomDev& p = m->plain[dtype == CFDB_F64 ? 1 : 0];
+  const int64_t scratch = p.stab_tmp ? 0 : int64_t(dtype_size(dtype)) * 18 * m->n;
+  if (int rc = cfdb_mesh_geometry(m, dtype, true, &geom, scratch)) return rc;
   if (geom == Geom::Box) return box_heat_step(ctx, m, dtype, T, Tn, k, dt);
   if (geom == Geom::Faces) return vert_heat_step(ctx, m, dtype, T, Tn, k, dt);
-  PlainGeomDev& p = m->plain[dtype == CFDB_F64 ? 1 : 0];
   if (!p.stab_tmp)
-    if (int rc = cfdb_dev_alloc(ctx, int64_t(dtype_size(dtype)) * 18 * m->n, &p.stab_tmp)) return rc;
+    if (int rc = cfdb_dev_alloc(ctx, scratch, &p.stab_tmp)) return rc;
   if (int rc = plain_lapl(ctx, m, dtype, T, p.stab_tmp, 7)) return rc;
   return plain_heat_update(ctx, dtype, p.stab_tmp, T, k, dt, Tn, m->n);
 }

@@ -69,3 +69,43 @@ def test_arrays_built_after_a_build_that_ran_out_of_memory(cfdb, dtype):
         want = out if want is None else want
         assert torch.equal(out, want)
     ctx.sync()
+
+
+@pytest.mark.parametrize("uniform", [True, False])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("first", ["grad", "lapl", "stab", "heat", "total"])
+def test_a_budget_for_the_arrays_serves_every_call(cfdb, uniform, dtype, first):
+    """A budget that holds the N x 6 arrays and the stabilisation's scratch, but
+    no second geometry beside them: whichever operator comes first, the calls
+    that need the arrays still go through."""
+    ctx = cfdb.Context(0)
+    ref = make(cfdb, ctx, uniform)
+    phi = field(ref, dtype, 1)
+    lam = torch.as_tensor(np.random.default_rng(2).standard_normal(4 * ref.n), dtype=dtype, device=DEV)
+
+    def call(m, name):
+        if name == "total":
+            return torch.tensor(ctx.total_fp64(m, phi))
+        if name == "heat":
+            out = torch.empty_like(phi)
+            ctx.heat_step(m, phi, out, 0.01, 1e-5, path=cfdb.PLAIN)
+            return out
+        if name == "adjoint":
+            out, gc = torch.empty_like(lam), torch.zeros_like(phi)
+            ctx.wave_adjoint_step(m, lam, lam * 0.5, out, phi * phi + 1, gc, 1e-3, path=cfdb.PLAIN)
+            return torch.cat([out, gc])
+        return getattr(ctx, name)(m, phi)
+
+    names = [first, "adjoint", "grad", "stab"]
+    want = [call(ref, n) for n in names]
+    ctx.sync()
+    ref.close()
+    m = make(cfdb, ctx, uniform)
+    es = phi.element_size()
+    verts = 0 if uniform else 24 * (SHAPE[0] + 1) * (SHAPE[1] + 1) * (SHAPE[2] + 1)
+    # the arrays (56 values per cell), the ids, then the larger of the vertices' copy and the scratch
+    ctx.set_alloc_budget(ctx.allocated_bytes() + (56 * es + 24) * m.n + max(verts, 18 * es * m.n) + 64)
+    for n, w in zip(names, want):
+        got = call(m, n)
+        assert torch.allclose(got, w, rtol=1e-12, atol=0) if n == "total" else torch.equal(got, w), n
+    ctx.sync()
