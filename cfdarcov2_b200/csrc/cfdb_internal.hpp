@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <functional>
@@ -196,6 +197,7 @@ struct cfdb_mesh {
   CompactGeomDev compact;
   BoxGeomDev box[2];  // structured meshes, by precision
   FaceGeomDev faces[2];  // vertex meshes, by precision
+  std::atomic<uint64_t> heat_plan[2] = {};  // passes of 2 and 3 heat steps (heat_blocked.cu); 0: not searched
   int lattice_state = 0;  // 0 not checked, 1 exact lattice, 2 not one
   cfdb_lattice_geometry lattice{};
 };

@@ -23,6 +23,7 @@
 // cells share is formed once and enters the other with the opposite sign, which is exact), so results are those
 // of the one-step sweep bit for bit.
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 
 #include "f32x2.cuh"
@@ -318,11 +319,16 @@ template <int K> int launch_zl(cfdb_ctx* ctx, const cfdb_mesh* m, const Plan& p,
 
 // The cheapest plan for passes of K steps.  A CTA marches its chunk and K planes
 // on each side; an iteration takes about 450 cycles of latency (copy, barrier)
-// plus, per level, a dependent chain of 130 and 21 for every warp of the SM
-// (fitted to 384x400x392, 200^3 and 64^3 at 4 to 16 warps: within 10 %); 1500 to
-// fill a wave of CTAs and 3500 around a launch.  The search weighs the tiles'
-// halo and padding, how evenly the CTAs fill the SMs, and the chunks' overlap.
-Plan plan_for(const cfdb_ctx* ctx, const cfdb_mesh* m, int K) {
+// plus, per level, a dependent chain of 130 and 21 for every warp of the SM,
+// 1500 to fill a wave of CTAs and 3500 around a launch.  Fitted to 384x400x392,
+// where it is right (43.8 us per step by the rule, 44 measured); passes that
+// follow one another hide most of the last two terms, so small fields take less
+// than it says (64^3 3.1 by the rule and 2.2 measured, 128^3 5.1 and 3.8, 160^3 6.8
+// and 5.1).  The search weighs the tiles' halo and padding, how evenly the CTAs
+// fill the SMs, and the chunks' overlap.  Of the chunk counts with equally long
+// chunks the smallest costs least (no other term falls as they grow), so only
+// those are looked at: 2 sqrt(nx) of them.
+Plan plan_search(const cfdb_ctx* ctx, const cfdb_mesh* m, int K) {
   Plan best;
   const int64_t sms = std::max(1, ctx->num_sms);
   for (int ZL : {32, 16, 8})
@@ -332,15 +338,37 @@ Plan plan_for(const cfdb_ctx* ctx, const cfdb_mesh* m, int K) {
       const int64_t tiles = int64_t(tiles_of(int(m->nz), 4 * ZL, kHaloZ)) * tiles_of(int(m->ny), rows, K);
       const int64_t slots = sms * (16 / warps);
       const int64_t most = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(m->nx / 2, 4096), 16 * slots / tiles));
-      for (int64_t chunks = 1; chunks <= most; ++chunks) {
+      for (int64_t chunks = 1; chunks <= most;) {
         const int64_t waves = (tiles * chunks + slots - 1) / slots;
-        const double planes = double((m->nx + chunks - 1) / chunks) + (chunks > 2 ? 2 * K : chunks > 1 ? K : 0) + K;
+        const int64_t longest = (m->nx + chunks - 1) / chunks;
+        const double planes = double(longest) + (chunks > 2 ? 2 * K : chunks > 1 ? K : 0) + K;
         const int64_t per_sm = (std::min(slots, tiles * chunks) + sms - 1) / sms;
         const double cycles = 3500.0 + double(waves) * (1500.0 + planes * (450.0 + K * (130.0 + 21.0 * double(warps * per_sm))));
         if (best.K == 0 || cycles / K < best.cost) best = Plan{K, ZL, warps, int(chunks), cycles / K};
+        if (longest == 1) break;
+        chunks = (m->nx + longest - 2) / (longest - 1);
       }
     }
   return best;
+}
+
+// The same, kept on the mesh (the search takes 2 to 10 us of host time, as much as a
+// short call): one word, so that threads that come together store the same.
+Plan plan_for(const cfdb_ctx* ctx, cfdb_mesh* m, int K) {
+  std::atomic<uint64_t>& word = m->heat_plan[K - 2];
+  uint64_t w = word.load(std::memory_order_relaxed);
+  if (w == 0) {
+    const Plan p = plan_search(ctx, m, K);
+    const float cost = float(p.cost);
+    uint32_t bits;
+    std::memcpy(&bits, &cost, sizeof(bits));
+    w = uint64_t(bits) << 32 | uint64_t(p.chunks) << 16 | uint64_t(p.ZL) << 8 | uint64_t(p.warps);
+    word.store(w, std::memory_order_relaxed);
+  }
+  const uint32_t bits = uint32_t(w >> 32);
+  float cost;
+  std::memcpy(&cost, &bits, sizeof(cost));
+  return Plan{K, int(w >> 8 & 255), int(w & 255), int(w >> 16 & 65535), double(cost)};
 }
 
 }  // namespace
@@ -366,18 +394,22 @@ static int blocked_pass(cfdb_ctx* ctx, cfdb_mesh* m, const void* src, void* dst,
 // where the one-step sweep would have left it (Tb for odd `steps`); with
 // keep_other the buffer that does not receive the result is left as it was,
 // a workspace taking its part where one can be had.  CFDB_EUNSUPPORTED (nothing
-// launched) when the mesh or the pointers are not what the TMA kernels take.
+// launched) when the mesh or the pointers are not what the TMA kernels take, and for
+// one or two steps that need no workspace.
 int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, double dt, int32_t steps, int use_graph,
                      bool keep_other) {
   if (steps < 1 || check_sweep(ctx, m, {Ta, Tb}) != CFDB_OK) return CFDB_EUNSUPPORTED;
   if (ctx->device < 0 || ctx->device >= kMaxDevices)
     return cfdb_fail(ctx, CFDB_EUNSUPPORTED, "device ordinal %d beyond %d", ctx->device, kMaxDevices);
   // passes of two or three steps (four spill registers), as even as possible,
-  // as many as the parity wants
+  // as many as the parity wants; one or two steps are single passes
   Plan plans[4];
-  for (int K : {2, 3}) plans[K] = plan_for(ctx, m, K);
-  const int most = plans[3].cost < plans[2].cost ? 3 : 2;
-  int32_t n = (steps + most - 1) / most;
+  int most = 1;
+  if (steps > 2) {
+    for (int K : {2, 3}) plans[K] = plan_for(ctx, m, K);
+    most = plans[3].cost < plans[2].cost ? 3 : 2;
+  }
+  int32_t n = steps / most + (steps % most != 0);
   if ((n ^ steps) & 1) ++n;
   const int per = int(steps / n), more = int(steps % n);  // the first `more` passes do per + 1
   void* ws = nullptr;
@@ -386,6 +418,7 @@ int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, 
     if (rc && rc != CFDB_ENOMEM) return rc;
     keep_other = rc == CFDB_OK;
   }
+  if (!keep_other && steps <= 2) return CFDB_EUNSUPPORTED;  // the caller's single steps
   if (!keep_other) {
     auto run = [&](void* a, void* b, int32_t passes, int each) {
       return cfdb_run_steps(
