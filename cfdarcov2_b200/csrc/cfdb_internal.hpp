@@ -325,12 +325,13 @@ int fused_d2t_step(cfdb_ctx* ctx, cfdb_mesh* m, const void* u, const void* u_pre
                    const int32_t* masks, int32_t n_terms, double dt, int first_step);
 // All `steps` FP32 heat steps in one thread-block-cluster launch with the
 // field resident in distributed shared memory (resident.cu); CFDB_EUNSUPPORTED
-// when the mesh does not fit (nothing launched).
+// when the mesh does not fit or passes are faster (nothing launched).
 int heat_resident_run(cfdb_ctx* ctx, cfdb_mesh* m, const void* Ta, void* Tb, double k, double dt, int32_t steps,
                       int* launched);
 // The same with several steps per pass over the field (heat_blocked.cu).
 int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, double dt, int32_t steps, int use_graph,
                      bool keep_other);
+double heat_pass_cycles(const cfdb_ctx* ctx, cfdb_mesh* m);
 int fused_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, void* qn, const void* c,
                     double cconst, int mode, double dt);
 // distorted.cu

@@ -1,6 +1,6 @@
-// The fused heat update of one cell in the TMA sweep (one launch per step); the
-// solvers of several steps per launch (resident.cu, heat_blocked.cu) spell the
-// same operations in packed pairs:
+// The fused heat update of one cell in the TMA sweep (one launch per step) and the
+// cluster's slab in shared memory (resident.cu); the other solvers of several steps
+// per launch (resident.cu, heat_blocked.cu) spell the same operations in packed pairs:
 //   T' = T + (cx lx + (cy ly + cz lz)),  l_d = (T_d+ - T) + (T_d- - T)
 // with c_d = dt k / h_d^2 and a wall neighbour equal to the cell itself
 // (zero gradient: the reference's boundary faces point to the cell,

@@ -16,14 +16,18 @@
 // 26 B per cell and step (64^3: 3.1 us per step); now it is 10 B and a step takes 2.1 us, half of it
 // issue on the cluster's SMs, the rest the cluster barrier and one remote load.  The cell update is
 // heat_update() (heat_cell.cuh) in packed pairs, operation by operation, so the
-// results are those of the one-step sweep bit for bit.  Larger fields take several
-// steps per pass over all SMs (heat_blocked.cu).
+// results are those of the one-step sweep bit for bit.
+//
+// Long thin fields (more planes than the registers hold, few cells in each) keep
+// both buffers in shared memory alone (heat_slab_k), where that is faster than several
+// steps per pass over all SMs (heat_blocked.cu), which take the larger ones.
 #include <cooperative_groups.h>
 
 #include <algorithm>
 
 #include "cfdb_internal.hpp"
 #include "f32x2.cuh"
+#include "heat_cell.cuh"
 
 CFDB_MODULE_ANCHOR
 
@@ -34,6 +38,8 @@ namespace {
 constexpr int kThreads = 512;    // at most: row pairs x z groups
 constexpr int kMaxCluster = 16;  // non-portable cluster size
 constexpr int kMaxPlanes = 4;    // planes per slab (eight spill registers)
+constexpr int kSlabThreads = 1024;
+constexpr int kMaxGroups = 8;    // heat_slab_k: groups of four z cells per thread and step
 
 struct ResidentArgs {
   int X, Y, Z;
@@ -176,15 +182,106 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
-template <int P>
-int run_cluster(cfdb_ctx* ctx, const cfdb_mesh* m, const void* Ta, void* out, const ResidentArgs& a, int CL, long long smem) {
-  auto kern = heat_resident_k<P>;
+// The slab in shared memory: a thread updates up to kMaxGroups groups of four z
+// cells wherever they lie in its slab, all neighbours from shared memory (the x
+// neighbours of the slab's end planes from the adjacent CTAs').  Bound by shared
+// memory, 26 B per cell and step on 16 SMs; us per step against passes: 1000x4x4 0.78
+// and 2.80, 96x24x24 1.09 and 1.70, 512x16x16 1.67 and 2.12, 2048x8x16 2.72 and 4.18.
+__global__ void __launch_bounds__(kSlabThreads, 1)
+    heat_slab_k(const float* __restrict__ in, float* __restrict__ out, ResidentArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int c = int(cl.block_rank());
+  const int CL = int(cl.num_blocks());
+  const int x0 = int((long long)c * a.X / CL), x1 = int((long long)(c + 1) * a.X / CL);
+  const int np = x1 - x0;
+  const int plane = a.Y * a.Z;
+  const int buf = a.P * plane;  // floats per buffer
+  const int zq = a.Z / 4;
+  const int groups = np * a.Y * zq;
+  const int tid = int(threadIdx.x);
+
+  // the slab into buffer 0
+  {
+    const float4* src = reinterpret_cast<const float4*>(in + (long long)x0 * plane);
+    float4* dst = reinterpret_cast<float4*>(sm);
+    for (int i = tid; i < np * plane / 4; i += kSlabThreads) dst[i] = src[i];
+  }
+  // this thread's groups: offset in a buffer, offset within the plane and
+  // which neighbours are walls
+  int off[kMaxGroups], inpl[kMaxGroups], flags[kMaxGroups];
+#pragma unroll
+  for (int k = 0; k < kMaxGroups; ++k) {
+    const int g = tid + k * kSlabThreads;
+    off[k] = -1;
+    inpl[k] = 0;
+    flags[k] = 0;
+    if (g < groups) {
+      const int p = g / (a.Y * zq);
+      const int r = g - p * (a.Y * zq);
+      const int y = r / zq;
+      const int z = 4 * (r - y * zq);
+      inpl[k] = y * a.Z + z;
+      off[k] = p * plane + inpl[k];
+      flags[k] = (p == 0 ? 1 : 0) | (p == np - 1 ? 2 : 0) | (y == 0 ? 4 : 0) | (y == a.Y - 1 ? 8 : 0) |
+                 (z == 0 ? 16 : 0) | (z + 4 == a.Z ? 32 : 0);
+    }
+  }
+  // neighbour slabs' shared memory (the plane next to ours in each)
+  const float* lo = c > 0 ? cl.map_shared_rank(sm, c - 1) : sm;
+  const float* hi = c < CL - 1 ? cl.map_shared_rank(sm, c + 1) : sm;
+  const int lo_plane = c > 0 ? (x0 - 1) - int((long long)(c - 1) * a.X / CL) : 0;
+  cl.sync();
+
+  for (int s = 0; s < a.steps; ++s) {
+    const float* A = sm + (s & 1) * buf;
+    float* B = sm + ((s + 1) & 1) * buf;
+    const float* Alo = lo + (s & 1) * buf + lo_plane * plane;  // x0 - 1 in the lower slab
+    const float* Ahi = hi + (s & 1) * buf;                      // x1 in the upper slab
+#pragma unroll
+    for (int k = 0; k < kMaxGroups; ++k) {
+      if (off[k] < 0) continue;
+      const int o = off[k], f = flags[k], yz = inpl[k];
+      const float4 C = *reinterpret_cast<const float4*>(A + o);
+      float4 XM, XP;
+      if (!(f & 1)) XM = *reinterpret_cast<const float4*>(A + o - plane);
+      else if (c > 0) XM = *reinterpret_cast<const float4*>(Alo + yz);
+      else XM = C;
+      if (!(f & 2)) XP = *reinterpret_cast<const float4*>(A + o + plane);
+      else if (c < CL - 1) XP = *reinterpret_cast<const float4*>(Ahi + yz);
+      else XP = C;
+      const float4 YM = (f & 4) ? C : *reinterpret_cast<const float4*>(A + o - a.Z);
+      const float4 YP = (f & 8) ? C : *reinterpret_cast<const float4*>(A + o + a.Z);
+      const float zl = (f & 16) ? C.x : A[o - 1];
+      const float zr = (f & 32) ? C.w : A[o + 4];
+      float4 R;
+      R.x = heat_update(C.x, XM.x, XP.x, YM.x, YP.x, zl, C.y, a.cx, a.cy, a.cz);
+      R.y = heat_update(C.y, XM.y, XP.y, YM.y, YP.y, C.x, C.z, a.cx, a.cy, a.cz);
+      R.z = heat_update(C.z, XM.z, XP.z, YM.z, YP.z, C.y, C.w, a.cx, a.cy, a.cz);
+      R.w = heat_update(C.w, XM.w, XP.w, YM.w, YP.w, C.z, zr, a.cx, a.cy, a.cz);
+      *reinterpret_cast<float4*>(B + o) = R;
+    }
+    cl.sync();  // step s written everywhere, and nobody reads buffer s & 1 any more
+  }
+
+  // the final state to global memory
+  {
+    const float4* src = reinterpret_cast<const float4*>(sm + (a.steps & 1) * buf);
+    float4* dst = reinterpret_cast<float4*>(out + (long long)x0 * plane);
+    for (int i = tid; i < np * plane / 4; i += kSlabThreads) dst[i] = src[i];
+  }
+}
+
+using Kernel = void (*)(const float*, float*, ResidentArgs);
+
+int run_cluster(cfdb_ctx* ctx, Kernel kern, const void* Ta, void* out, const ResidentArgs& a, int CL, int threads,
+                long long smem) {
   // per-device kernel attributes; cheap enough to set on every call
   CFDB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   CFDB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(CL));
-  cfg.blockDim = dim3(unsigned(((m->ny + 1) / 2 * (m->nz / 4) + 31) / 32 * 32));
+  cfg.blockDim = dim3(unsigned(threads));
   cfg.dynamicSmemBytes = size_t(smem);
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
@@ -204,11 +301,25 @@ int run_cluster(cfdb_ctx* ctx, const cfdb_mesh* m, const void* Ta, void* out, co
   return CFDB_OK;
 }
 
+// Whether a slab of P planes in shared memory beats the passes: a step costs 1200
+// SM cycles (cluster barrier, remote loads) and a quarter of one per cell of the
+// CTA; the launch and the field's way in and out 4500 more than a pass's.  Against 48
+// long shapes at 3, 5 and 200 steps: the faster form, or within 8 % of it, but for
+// runs of 3 steps (there within 1.3 of it).  Slabs of few wide planes (their x
+// neighbours all remote) lose at any size: 12x100x60 2.5 us against 1.7.
+bool slab_wins(cfdb_ctx* ctx, cfdb_mesh* m, long long P, int32_t steps) {
+  if (P <= kMaxPlanes) return false;
+  const double step = 1200.0 + 0.255 * double(P) * double(m->ny * m->nz);
+  if (steps <= 2) return steps == 2 && step < 3300.0;  // against single steps: the second launch costs about 2 us
+  return double(steps) * (1.07 * heat_pass_cycles(ctx, m) - step) > 4500.0;
+}
+
 }  // namespace
 
-// Runs `steps` heat steps in one launch when the mesh fits one cluster: planes
-// of at most 512 (row pair, four cells) threads, 4 planes per CTA, two buffers in
-// shared memory.  CFDB_EUNSUPPORTED (nothing launched, no error recorded)
+// Runs `steps` heat steps in one launch when the mesh fits one cluster and that is
+// the faster form.  In registers: planes of at most 512 (row pair, four cells)
+// threads, 4 planes per CTA, two buffers in shared memory.  Beyond that in shared
+// memory alone (slab_wins).  CFDB_EUNSUPPORTED (nothing launched, no error recorded)
 // otherwise, and the caller takes another path.  The result goes to Tb for odd
 // `steps`, else to Ta, as with the ping-pong of the per-step path; the other buffer
 // is left as it was.
@@ -217,10 +328,9 @@ int heat_resident_run(cfdb_ctx* ctx, cfdb_mesh* m, const void* Ta, void* Tb, dou
   *launched = 0;
   if (!m->uniform || m->nz % 4 != 0 || steps < 1) return CFDB_EUNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(Ta) | reinterpret_cast<uintptr_t>(Tb)) & 15u) return CFDB_EUNSUPPORTED;
-  if ((m->ny + 1) / 2 * (m->nz / 4) > kThreads) return CFDB_EUNSUPPORTED;
+  const long long plane = m->ny * m->nz, pairs = (m->ny + 1) / 2 * (m->nz / 4);
   int max_smem = 0;
   CFDB_CUDA(ctx, cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-  const long long plane = m->ny * m->nz;
   ResidentArgs a;
   a.X = int(m->nx); a.Y = int(m->ny); a.Z = int(m->nz);
   a.steps = steps;
@@ -228,12 +338,18 @@ int heat_resident_run(cfdb_ctx* ctx, cfdb_mesh* m, const void* Ta, void* Tb, dou
   a.cy = float(dt * k / (m->dy * m->dy));
   a.cz = float(dt * k / (m->dz * m->dz));
   void* out = (steps & 1) ? Tb : const_cast<void*>(Ta);
-  for (int CL = std::min<long long>(kMaxCluster, m->nx); CL >= 2; CL /= 2) {
+  for (int CL = int(std::min<long long>(kMaxCluster, m->nx)); CL >= 2; CL /= 2) {
     const long long P = (m->nx + CL - 1) / CL;
     const long long smem = 2 * P * plane * 4;
-    if (smem > max_smem || P > kMaxPlanes) break;  // fewer CTAs only make the slabs larger
+    if (smem > max_smem) break;  // fewer CTAs only make the slabs larger
     a.P = int(P);
-    const int rc = P <= 2 ? run_cluster<2>(ctx, m, Ta, out, a, CL, smem) : run_cluster<4>(ctx, m, Ta, out, a, CL, smem);
+    int rc = CFDB_EUNSUPPORTED;
+    if (P <= kMaxPlanes && pairs <= kThreads) {
+      rc = run_cluster(ctx, P <= 2 ? heat_resident_k<2> : heat_resident_k<4>, Ta, out, a, CL, int((pairs + 31) / 32 * 32), smem);
+    } else if (P * plane / 4 <= (long long)kMaxGroups * kSlabThreads) {
+      if (!slab_wins(ctx, m, P, steps)) break;
+      rc = run_cluster(ctx, heat_slab_k, Ta, out, a, CL, kSlabThreads, smem);
+    }
     if (rc == CFDB_OK) *launched = CL;
     if (rc != CFDB_EUNSUPPORTED) return rc;
   }

@@ -90,3 +90,49 @@ def test_short_runs_of_long_meshes_pay_no_search(cfdb, ctx):
             took.append(time.perf_counter() - t)
         assert sorted(took)[4] < 200e-6, (steps, took)
     ctx.sync()
+
+
+def launches_of(ctx, fn):
+    before = ctx.launch_count()
+    fn()
+    return ctx.launch_count() - before
+
+
+@pytest.mark.parametrize("shape,steps", [((96, 24, 24), 40), ((1000, 4, 4), 5), ((2000, 8, 8), 9), ((70, 8, 8), 50),
+                                         ((65, 20, 20), 7), ((512, 16, 16), 30), ((257, 7, 12), 33), ((81, 9, 4), 20),
+                                         ((1000, 1, 64), 6), ((160, 160, 4), 12), ((2048, 8, 16), 11)])
+def test_long_thin_fields_run_in_one_launch(cfdb, ctx, shape, steps):
+    """Fields of many small planes stay in one cluster's shared memory for the
+    whole run: the one-step sweep's bits from a single launch, the other buffer
+    left alone."""
+    X, Y, Z = shape
+    m = cfdb.Mesh.structured(ctx, X, Y, Z, 1 / X, 1 / Y, 1 / Z)
+    T0 = torch.as_tensor(np.random.default_rng(3).uniform(-1, 1, m.n), dtype=torch.float32, device=DEV)
+    k, dt = 0.01, 0.1 * min(1 / X, 1 / Y, 1 / Z) ** 2 / 0.01
+    p, q = T0.clone(), torch.empty_like(T0)
+    for s in range(steps):
+        ctx.heat_step(m, p, q, k, dt)
+        p, q = q, p
+    a, b = T0.clone(), torch.full_like(T0, float("nan"))
+    out = []
+    assert launches_of(ctx, lambda: out.append(ctx.heat_run(m, a, b, k, dt, steps))) == 1
+    assert torch.equal(out[0], p)
+    assert torch.equal(a, T0) if steps & 1 else torch.isnan(b).all()
+    ctx.sync()
+
+
+@pytest.mark.parametrize("shape,steps,launches", [
+    ((64, 64, 64), 37, 1), ((40, 36, 32), 12, 1), ((17, 24, 20), 9, 1), ((8, 8, 8), 1, 1), ((16, 64, 64), 6, 1),
+    # beyond one cluster: as many passes of two or three steps as keep the parity
+    ((128, 64, 64), 23, 9), ((40, 96, 64), 14, 6), ((128, 64, 64), 1, 1), ((128, 64, 64), 2, 2), ((40, 96, 64), 3, 1),
+    ((128, 128, 128), 4, 2)])
+def test_which_form_ran(cfdb, ctx, shape, steps, launches):
+    """The number of launches tells a run on one cluster from passes and from
+    single steps."""
+    X, Y, Z = shape
+    m = cfdb.Mesh.structured(ctx, X, Y, Z, 1 / X, 1 / Y, 1 / Z)
+    a = torch.rand(m.n, device=DEV)
+    b = torch.empty_like(a)
+    for graph in (False, True):
+        assert launches_of(ctx, lambda: ctx.heat_run(m, a, b, 0.01, 1e-7, steps, use_graph=graph)) == launches
+    ctx.sync()
