@@ -89,9 +89,10 @@ extern "C" int cfdb_heat_run(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, int path, v
   if (!Ta || !Tb || Ta == Tb) return cfdb_fail(ctx, CFDB_EINVAL, "cfdb_heat_run: need distinct T_a and T_b");
   if (path == CFDB_PATH_FUSED && dtype == CFDB_F32 && std::isfinite(k) && std::isfinite(dt)) {
     int launched = 0;
-    // a field of at most a few MB leaves the other buffer alone, as on one cluster
+    // fields of up to 2 MB leave the other buffer alone, as on one cluster; larger ones
+    // use both, as single steps do
     int r = heat_resident_run(ctx, m, Ta, Tb, k, dt, steps, &launched);
-    if (r == CFDB_EUNSUPPORTED) r = heat_blocked_run(ctx, m, Ta, Tb, k, dt, steps, use_graph, m->n <= 1 << 20);
+    if (r == CFDB_EUNSUPPORTED) r = heat_blocked_run(ctx, m, Ta, Tb, k, dt, steps, use_graph, m->n <= 1 << 19);
     if (r == CFDB_OK) {
       if (final_in_b) *final_in_b = steps & 1;
       return CFDB_OK;

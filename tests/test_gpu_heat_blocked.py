@@ -136,3 +136,30 @@ def test_which_form_ran(cfdb, ctx, shape, steps, launches):
     for graph in (False, True):
         assert launches_of(ctx, lambda: ctx.heat_run(m, a, b, 0.01, 1e-7, steps, use_graph=graph)) == launches
     ctx.sync()
+
+
+@pytest.mark.parametrize("shape", [(96, 96, 96), (100, 100, 100), (140, 128, 32), (200, 128, 128)])
+def test_recorded_passes_allocate_nothing(cfdb, ctx, shape):
+    """A run recorded into the caller's graph is kernels only, so that the graph
+    can be instantiated and embedded as one of single steps can."""
+    from cuda.bindings import runtime as rt
+    X, Y, Z = shape
+    m = cfdb.Mesh.structured(ctx, X, Y, Z, 1 / X, 1 / Y, 1 / Z)
+    T0 = torch.rand(m.n, device=DEV)
+    a, b = T0.clone(), torch.empty_like(T0)
+    want = ctx.heat_run(m, a, b, 0.01, 1e-7, 7, use_graph=False).clone()
+    a.copy_(T0)
+    torch.cuda.synchronize()
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=side):
+        ctx.set_stream(side.cuda_stream)
+        got = ctx.heat_run(m, a, b, 0.01, 1e-7, 7, use_graph=False)
+    ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+    handle = rt.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, count = rt.cudaGraphGetNodes(handle)
+    err, nodes, count = rt.cudaGraphGetNodes(handle, count)
+    kinds = {rt.cudaGraphNodeGetType(n)[1] for n in nodes[:count]}
+    assert kinds == {rt.cudaGraphNodeType.cudaGraphNodeTypeKernel}
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
