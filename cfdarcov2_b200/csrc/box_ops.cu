@@ -473,8 +473,7 @@ __global__ void __launch_bounds__(kThreads) box_stab_k(const __grid_constant__ B
 // the array form from either side; sums run over the slots in the array form's
 // order, no product is left out, so the results are its bits for any operand.
 // What bounds these kernels is the geometry still read, 16 values per cell for the
-// Laplacian (FP64 80 x 72 x 66: 49 MB, from L2; array kernels 18, 36 and 90 us for
-// gradient, Laplacian and stabilisation).
+// Laplacian (FP64 80 x 72 x 66: 49 MB, from L2).
 
 template <class R> struct Vert {
   int nx, ny, nz;
@@ -511,59 +510,56 @@ enum { OUT_SUM = 0, OUT_GRADIENT = 1 };
 
 // Gradient (OP_GRAD) or Laplacian (OP_LAPL, OP_HEAT) of every cell; OUT_GRADIENT
 // stores the three gradient components (arrays of n) instead of their masked sum.
+// One cell per thread, all of its loads in flight at once: what bounds it is memory
+// beyond L2 and latency below.  Asked for 8 CTAs per SM the compiler keeps the loads
+// together (left alone it takes 32 registers and waits for them one face after the
+// other).  us, array kernels / a march that evaluates every face once / this: FP64
+// 100^3 gradient 38.4 / 32.9 / 22.0, Laplacian 78 / 35.5 / 24.7, FP32 160^3 102 / 65 / 51
+// and 201 / 66 / 60, FP32 32x24x20 2.2 / 3.4 / 1.9 and 2.6 / 3.6 / 1.9.  (The FP32
+// gradient of 0.2 to 0.4 million cells is the array kernels' 3.4 and 5.4 us in 3.8 and
+// 5.8 us: rows of nz + 1 faces start off the 32-byte sectors.)
 template <class R, int OP, int OUT>
-__global__ void __launch_bounds__(kThreads) vert_sum_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
-                                                  R* __restrict__ out, int mask, R k, R dt) {
-  March<1, 1, 1> w;
-  if (!w.start(g)) return;
+__global__ void __launch_bounds__(kThreads, 8) vert_cell_k(const __grid_constant__ Vert<R> g, const R* __restrict__ phi,
+                                                   R* __restrict__ out, int mask, R k, R dt) {
   const int64_t pl = g.plane, n = int64_t(g.nx) * pl;
-  const int y = w.y0, z = w.z;
-  // F[d] = (face value n_d) A between the lower and the upper cell
-  auto face = [&](int axis, int64_t f, R lo, R hi, R F[3]) __attribute__((always_inline)) {
-    R v;
-    if constexpr (OP == OP_GRAD) v = (lo + hi) * R(0.5);
-    else v = (hi - lo) * g.alpha[axis][f];
-    const R A = g.area[axis][f];
+  const int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x;
+  if (i >= n) return;
+  const unsigned x_ = unsigned(i) / g.plane, r = unsigned(i) - x_ * g.plane, y_ = r / unsigned(g.nz);
+  const int x = int(x_), y = int(y_), z = int(r - y_ * unsigned(g.nz));
+  const R P = phi[i], V = g.vol[i];
+  // all loads before the sums: z-, z+, y-, y+, x-, x+
+  R N[6], A[6], al[6], nr[6][3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) F[d] = (v * g.nrm[axis][d][f]) * A;
-  };
-  const R* q = phi + w.x0 * pl;
-  R P = q[w.off[1]], Fx[3];
-  face(0, g.face(0, w.x0, y, z), q[w.off[1] - (w.x0 > 0 ? pl : 0)], P, Fx);
-  for (int x = w.x0; x < w.x1; ++x, q += pl) {
-    const R N = q[w.off[1] + (x < g.nx - 1 ? pl : 0)];
-    const R below = q[w.off[0]], above = q[w.off[2]];
-    const int64_t i = x * pl + w.off[1];
-    const R V = g.vol[i];
-    R Fh[3], Fyl[3], Fyh[3], Fzl[3], Fzh[3];
-    face(0, g.face(0, x + 1, y, z), P, N, Fh);
-    const int64_t fy = g.face(1, x, y, z), fz = g.face(2, x, y, z);
-    face(1, fy, below, P, Fyl);
-    face(1, fy + g.nz, P, above, Fyh);
-    const R zp = __shfl_down_sync(kWarp, P, 1);
-    face(2, fz + 1, P, w.zhi ? P : zp, Fzh);
+  for (int s = 0; s < 6; ++s) {
+    const int axis = 2 - s / 2, up = s & 1;
+    const int64_t step = axis == 0 ? pl : axis == 1 ? g.nz : 1, f = g.face(axis, x, y, z) + up * step;
+    const int at = axis == 0 ? x : axis == 1 ? y : z, wall = up ? (axis == 0 ? g.nx : axis == 1 ? g.ny : g.nz) - 1 : 0;
+    N[s] = phi[at == wall ? i : up ? i + step : i - step];
+    A[s] = g.area[axis][f];
+    al[s] = OP == OP_GRAD ? R(0) : g.alpha[axis][f];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) Fzl[d] = __shfl_up_sync(kWarp, Fzh[d], 1);
-    if (w.zlo) face(2, fz, P, P, Fzl);
-    R acc[3];
+    for (int d = 0; d < 3; ++d) nr[s][d] = g.nrm[axis][d][f];
+  }
+  R acc[3] = {R(0), R(0), R(0)};
 #pragma unroll
-    for (int d = 0; d < 3; ++d) acc[d] = (((((R(0) - Fzl[d]) + Fzh[d]) - Fyl[d]) + Fyh[d]) - Fx[d]) + Fh[d];
-    divide_any(acc, V);
-    if (w.out) {
-      if constexpr (OUT == OUT_GRADIENT) {
+  for (int s = 0; s < 6; ++s) {
+    const R v = OP == OP_GRAD ? (P + N[s]) * R(0.5) : (s & 1 ? N[s] - P : P - N[s]) * al[s];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) out[d * n + i] = acc[d];
-      } else {
-        R res = R(0);
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          if (mask & (1 << d)) res = res + acc[d];
-        out[i] = OP == OP_HEAT ? dt * (k * res) + P : res;
-      }
+    for (int d = 0; d < 3; ++d) {
+      const R F = (v * nr[s][d]) * A[s];
+      acc[d] = s & 1 ? acc[d] + F : acc[d] - F;
     }
-    P = N;
+  }
+  divide_any(acc, V);
+  if constexpr (OUT == OUT_GRADIENT) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) Fx[d] = Fh[d];
+    for (int d = 0; d < 3; ++d) out[d * n + i] = acc[d];
+  } else {
+    R res = R(0);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (mask & (1 << d)) res = res + acc[d];
+    out[i] = OP == OP_HEAT ? dt * (k * res) + P : res;
   }
 }
 
@@ -1317,13 +1313,13 @@ int build_box(cfdb_mesh* m, BoxGeomDev& b) {
   return CFDB_OK;
 }
 
-template <class R> Vert<R> vert_of(const cfdb_ctx* ctx, const cfdb_mesh* m, int resident, unsigned* blocks) {
+template <class R> Vert<R> vert_of(const cfdb_mesh* m) {
   const FaceGeomDev& b = m->faces[sizeof(R) == 8 ? 1 : 0];
   Vert<R> g;
   g.nx = int(m->nx); g.ny = int(m->ny); g.nz = int(m->nz);
   g.plane = unsigned(m->ny * m->nz);
   g.groups = g.ny;
-  march_grid(ctx, m, 1, resident, &g.tiles, &g.chunks, blocks, g.groups);
+  g.tiles = g.chunks = 0;  // of a march
   for (int a = 0; a < 3; ++a) {
     for (int d = 0; d < 3; ++d) g.nrm[a][d] = static_cast<const R*>(b.normal[a]) + d * b.count[a];
     g.area[a] = static_cast<const R*>(b.area[a]);
@@ -1441,10 +1437,8 @@ int box_euler_step(cfdb_euler* e, const void* U, void* Un, int64_t step) {
 
 template <class R, int OP, int OUT>
 int launch_vert_sum(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask, double k, double dt) {
-  unsigned blocks = 0;
-  const auto f = form<vert_sum_k<R, OP, OUT>>(ctx);
-  const Vert<R> g = vert_of<R>(ctx, m, f.resident, &blocks);
-  f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
+  vert_cell_k<R, OP, OUT><<<unsigned((m->n + kThreads - 1) / kThreads), kThreads, 0, ctx->stream>>>(
+      vert_of<R>(m), static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
 }
@@ -1469,7 +1463,8 @@ template <class R> int launch_vert_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void*
   if (int rc = launch_vert_sum<R, OP_GRAD, OUT_GRADIENT>(ctx, m, phi, b.grad, 7, 0, 0)) return rc;
   unsigned blocks = 0;
   const auto f = form<vert_stab_k<R>>(ctx);
-  const Vert<R> g = vert_of<R>(ctx, m, f.resident, &blocks);
+  Vert<R> g = vert_of<R>(m);
+  march_grid(ctx, m, 1, f.resident, &g.tiles, &g.chunks, &blocks, g.groups);
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<const R*>(b.grad),
                                                   static_cast<R*>(out), mask);
   CFDB_LAUNCHED(ctx);
