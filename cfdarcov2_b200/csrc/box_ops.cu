@@ -1134,12 +1134,20 @@ __global__ void __launch_bounds__(kThreads) box_volume_k(int nx, int ny, int nz,
   if (other) atomicOr(differs, 1);
 }
 
-// A kernel and the CTAs of it that one SM holds.
+// A marching kernel, the CTAs of it that one SM holds, and its place among the marches.
+struct MarchPlan {
+  int resident, id;
+};
 template <class K> struct Form {
   K kern;
-  int resident;
+  MarchPlan plan;
 };
+int next_march() {
+  static std::atomic<int> next{0};
+  return next++;
+}
 template <auto kern> Form<decltype(kern)> form(const cfdb_ctx* ctx) {
+  static const int id = next_march();
   static std::atomic<int> held[kMaxDevices] = {};
   const bool known = ctx->device >= 0 && ctx->device < kMaxDevices;
   int r = known ? held[ctx->device].load(std::memory_order_relaxed) : 0;
@@ -1148,53 +1156,69 @@ template <auto kern> Form<decltype(kern)> form(const cfdb_ctx* ctx) {
     r = std::max(r, 1);
     if (known) held[ctx->device].store(r, std::memory_order_relaxed);
   }
-  return {kern, r};
+  return {kern, {r, id}};
 }
 
-// Warps of a march over `groups` row groups: tiles of 32 - 2 HZ lanes along
-// (group, z), x cut into chunks of at least two planes.  Fewer chunks are less
-// work, as each starts with 2 + HZ / 2 planes' worth of loads and faces that its
-// neighbour has too, but they have to fill the SMs evenly.  With w warps on an SM
-// a plane costs 8 + w (8 for latency); after a first wave the CTAs end at
-// different times, so the last one counts for three quarters as a wave and for
-// one as its share of one.  The least sum is within 2 % of the best of 1 to 50
-// chunks over 10 meshes x 5 operators; 32 warps per SM whatever the kernel held
-// had lost 9 % (FP64 gradient at 200^3: 123 us in 501 CTAs on 444 places, now 75;
-// plain FP64 acoustic step there 187 -> 170, vertex gradient at 400k cells 12.7 -> 10.7).
-void march_grid(const cfdb_ctx* ctx, const cfdb_mesh* m, int HZ, int resident, unsigned* tiles, unsigned* chunks,
-                unsigned* blocks, int64_t groups) {
-  *tiles = unsigned((groups * m->nz + 32 - 2 * HZ - 1) / (32 - 2 * HZ));
+// Chunks of x.  Fewer are less work, as each starts with 2 + HZ / 2 planes' worth of
+// loads and faces that its neighbour has too, but they have to fill the SMs evenly.
+// With w warps on an SM a plane costs 8 + w (8 for latency); after a first wave the
+// CTAs end at different times, so the last one counts for three quarters as a wave
+// and for one as its share of one.  The least sum is within 2 % of the best of 1 to 50
+// chunks over 10 meshes x 5 operators; 32 warps per SM whatever the kernel held had
+// lost 9 % (FP64 gradient at 200^3: 123 us in 501 CTAs on 444 places, now 75).
+// A mesh that does not fill the SMs once, even with a plane per chunk, is all latency:
+// there a plane costs 16 + w and a chunk's start one plane, and chunks of one plane
+// count too (us with at least two planes and now: FP32 gradient 16^3 2.4 and 2.1,
+// 512x1x1 2.4 and 2.2, FP64 stabilisation 32x24x20 3.7 and 2.9).
+unsigned march_chunks(const cfdb_ctx* ctx, const cfdb_mesh* m, int HZ, int resident, int64_t tiles) {
   constexpr int per = kThreads / 32;
-  const int64_t sms = std::max(1, ctx->num_sms), places = sms * resident;
-  const int64_t most = std::max<int64_t>(1, std::min<int64_t>(m->nx / 2, 8 * places * per / *tiles));
-  const double wave = 8 + resident * per;
+  const int64_t sms = std::max(1, ctx->num_sms), places = sms * resident, nx = m->nx;
+  const bool small = (tiles * nx + per - 1) / per <= places;
+  const int64_t most = small ? nx : std::max<int64_t>(1, std::min<int64_t>(nx / 2, 8 * places * per / tiles));
+  const double latency = small ? 16 : 8, start = (small ? 1 : 2) + 0.5 * HZ, wave = latency + resident * per;
   double least = 0;
-  *chunks = 1;
-  for (int64_t c = 1; c <= most; c += std::max<int64_t>(1, c / 32)) {
-    const int64_t ctas = (*tiles * c + per - 1) / per, full = ctas / places, last = ctas % places;
+  int64_t chunks = 1;
+  for (int64_t c = 1; c <= most; c += small ? 1 : std::max<int64_t>(1, c / 32)) {
+    const int64_t ctas = (tiles * c + per - 1) / per, full = ctas / places, last = ctas % places;
     double waves = double(full) * wave;
     if (last) {
-      const double own = 8 + double((last + sms - 1) / sms * per);
+      const double own = latency + double((last + sms - 1) / sms * per);
       waves += full ? 0.75 * own + 0.25 * wave * double(last) / double(places) : own;
     }
-    const double cost = (waves + 0.05 * wave) * (double(m->nx) / double(c) + 2 + 0.5 * HZ);
+    const double planes = small ? double((nx + c - 1) / c) : double(nx) / double(c);
+    const double cost = (waves + 0.05 * wave) * (planes + start);
     if (c == 1 || cost < least) {
       least = cost;
-      *chunks = unsigned(c);
+      chunks = c;
     }
   }
+  return unsigned(chunks);
+}
+
+// Warps of a march over `groups` row groups: tiles of 32 - 2 HZ lanes along (group, z),
+// x cut into chunks.  The chunk count stays on the mesh (finding it had cost the host
+// up to 0.6 us of every call).
+void march_grid(const cfdb_ctx* ctx, cfdb_mesh* m, int HZ, MarchPlan plan, unsigned* tiles, unsigned* chunks,
+                unsigned* blocks, int64_t groups) {
+  *tiles = unsigned((groups * m->nz + 32 - 2 * HZ - 1) / (32 - 2 * HZ));
+  std::atomic<uint32_t>* kept = plan.id < kMarches ? &m->march_chunks[plan.id] : nullptr;
+  *chunks = kept ? kept->load(std::memory_order_relaxed) : 0;
+  if (*chunks == 0) {
+    *chunks = march_chunks(ctx, m, HZ, plan.resident, *tiles);
+    if (kept) kept->store(*chunks, std::memory_order_relaxed);
+  }
+  constexpr int per = kThreads / 32;
   *blocks = unsigned((int64_t(*tiles) * *chunks + per - 1) / per);
 }
 
-// Kernel arguments for NY rows per thread, HZ halo lanes and `resident` CTAs per
-// SM; *blocks = the grid.
-template <class R> Box<R> box_of(const cfdb_ctx* ctx, const cfdb_mesh* m, int NY, int HZ, int resident, unsigned* blocks) {
+// Kernel arguments for NY rows per thread and HZ halo lanes; *blocks = the grid.
+template <class R> Box<R> box_of(const cfdb_ctx* ctx, cfdb_mesh* m, int NY, int HZ, MarchPlan plan, unsigned* blocks) {
   const BoxGeomDev& b = m->box[sizeof(R) == 8 ? 1 : 0];
   Box<R> g;
   g.nx = int(m->nx); g.ny = int(m->ny); g.nz = int(m->nz);
   g.plane = unsigned(m->ny * m->nz);
   g.groups = int((m->ny + NY - 1) / NY);
-  march_grid(ctx, m, HZ, resident, &g.tiles, &g.chunks, blocks, g.groups);
+  march_grid(ctx, m, HZ, plan, &g.tiles, &g.chunks, blocks, g.groups);
   g.hx = b.h[0]; g.hy = b.h[1]; g.hz = b.h[2];
   auto t = [](const void* p) { return static_cast<const R*>(p); };
   g.ax = t(b.alpha[0]); g.ay = t(b.alpha[1]); g.az = t(b.alpha[2]);
@@ -1359,7 +1383,7 @@ template <class R, int OP> int launch_sum(cfdb_ctx* ctx, cfdb_mesh* m, const voi
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
   const auto f = rows == 1 ? BOX_FORMS(box_sum_k, R, OP, 1) : BOX_FORMS(box_sum_k, R, OP, NY);
-  const Box<R> g = box_of<R>(ctx, m, rows, 1, f.resident, &blocks);
+  const Box<R> g = box_of<R>(ctx, m, rows, 1, f.plan, &blocks);
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
@@ -1371,7 +1395,7 @@ template <class R> int launch_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi,
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
   const auto f = rows == 1 ? BOX_FORMS(box_stab_k, R, 1) : BOX_FORMS(box_stab_k, R, NY);
-  const Box<R> g = box_of<R>(ctx, m, rows, 2, f.resident, &blocks);
+  const Box<R> g = box_of<R>(ctx, m, rows, 2, f.plan, &blocks);
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask);
   CFDB_LAUNCHED(ctx);
   return CFDB_OK;
@@ -1388,7 +1412,7 @@ int launch_wave(cfdb_ctx* ctx, cfdb_mesh* m, const void* q, void* qn, const void
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
   const auto f = rows == 1 ? wave_kernel<R, 1>(ctx, uni, c != nullptr) : wave_kernel<R, NY>(ctx, uni, c != nullptr);
-  const Box<R> g = box_of<R>(ctx, m, rows, 1, f.resident, &blocks);
+  const Box<R> g = box_of<R>(ctx, m, rows, 1, f.plan, &blocks);
   const WaveArgs<R> a{static_cast<const R*>(q), static_cast<R*>(qn), static_cast<const R*>(c), R(cconst), R(dt), mode};
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, a);
   CFDB_LAUNCHED(ctx);
@@ -1423,7 +1447,7 @@ template <class R> int launch_euler(cfdb_euler* e, const void* U, void* Un, int6
   cfdb_ctx* ctx = e->ctx;
   unsigned blocks = 0;
   const auto f = form<box_euler_k<R>>(ctx);
-  const Box<R> g = box_of<R>(ctx, e->mesh, 1, 1, f.resident, &blocks);
+  const Box<R> g = box_of<R>(ctx, e->mesh, 1, 1, f.plan, &blocks);
   const EulerArgs<R> a{static_cast<const R*>(U), static_cast<R*>(Un), R(e->gamma), e->mesh->dx, e->mesh->dy, e->mesh->dz,
                        e->cfl, e->t_end, e->clock, (long long)step};
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, a);
@@ -1464,7 +1488,7 @@ template <class R> int launch_vert_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void*
   unsigned blocks = 0;
   const auto f = form<vert_stab_k<R>>(ctx);
   Vert<R> g = vert_of<R>(m);
-  march_grid(ctx, m, 1, f.resident, &g.tiles, &g.chunks, &blocks, g.groups);
+  march_grid(ctx, m, 1, f.plan, &g.tiles, &g.chunks, &blocks, g.groups);
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<const R*>(b.grad),
                                                   static_cast<R*>(out), mask);
   CFDB_LAUNCHED(ctx);

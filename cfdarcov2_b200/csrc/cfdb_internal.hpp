@@ -183,6 +183,9 @@ void cfdb_jit_release(cfdb_ctx* ctx);  // unloads the context's run-time compile
 std::string graph_key(const char* kind, const struct cfdb_mesh* m, int dtype, int path, const void* a, const void* b,
                       const void* c, std::initializer_list<double> params);
 
+// Marching kernels whose chunk count a mesh keeps (box_ops.cu has 40).
+constexpr int kMarches = 64;
+
 struct cfdb_mesh {
   cfdb_ctx* ctx = nullptr;
   uint64_t uid = 0;  // process-unique, never reused (keys of cached step graphs)
@@ -197,6 +200,7 @@ struct cfdb_mesh {
   CompactGeomDev compact;
   BoxGeomDev box[2];  // structured meshes, by precision
   FaceGeomDev faces[2];  // vertex meshes, by precision
+  std::atomic<uint32_t> march_chunks[kMarches] = {};  // by kernel; 0: not chosen
   std::atomic<uint64_t> heat_plan[2] = {};  // passes of 2 and 3 heat steps (heat_blocked.cu); 0: not searched
   int lattice_state = 0;  // 0 not checked, 1 exact lattice, 2 not one
   cfdb_lattice_geometry lattice{};
