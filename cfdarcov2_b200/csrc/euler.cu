@@ -312,13 +312,28 @@ int launch_euler(cfdb_euler* e, const void* U, void* Un, int64_t s) {
   return CFDB_OK;
 }
 
-// Tiles of 64 x 8 or 32 x 16 cells (256 threads either way), whichever covers
-// fewer cells with its padding of rows and columns: 96^3 14.3 us per step with 32,
-// 17.4 with 64; 128 x 64 x 32 7.8 against 11.4 (a 32 x 8 tile left half of the SM's
-// threads out); 100^3 20.0 with 32, 19.5 with 64; 512 x 64 x 64 the same.
-bool wide_tiles(const cfdb_mesh* m) {
-  auto cover = [&](int64_t tz, int64_t ty) { return double((m->nz + tz - 1) / tz * tz) * double((m->ny + ty - 1) / ty * ty); };
-  return cover(64, 8) <= 1.05 * cover(32, 16);
+// Tiles of 64 x 8 or 32 x 16 cells (256 threads either way), or 32 x 8 (128), by what
+// a step takes: a CTA pays a start and its planes, both more when two share an SM,
+// and CTAs beyond those that fit at once another round.  us, fitted to 44 meshes of 512
+// cells to 8M (the choice is the best of the three or within 3 % of it): 96^3 17.3 with
+// 64 x 8, 14.1 with 32 x 16, 16.1 with 32 x 8; 128 x 32 x 32 8.2, 7.1 and 6.4; 24^3 6.6,
+// 6.2 and 5.4; 100^3 19.3, 20.0 and 23.4; 512 x 64 x 64 25.9, 25.9 and 31.4.  Within 3 %
+// of the least 64 x 8 is taken.
+double step_time(const cfdb_ctx* ctx, const cfdb_mesh* m, int tz, int ty) {
+  const int64_t sms = std::max(1, ctx->num_sms), slots = sms * kEulerCtasPerSm;
+  const stencil::SweepShape sh = stencil::sweep_shape(ctx, m, tz, ty, kEulerCtasPerSm);
+  const int64_t ctas = int64_t(sh.tiles) * sh.chunks, left = ctas % slots;
+  const double planes = double((m->nx + sh.chunks - 1) / sh.chunks);
+  auto round = [&](int64_t n) {
+    if (tz * ty == 256) return (n > sms ? 4.8 : 4.2) + 0.9 * planes;
+    return n > sms ? 5.8 + 1.4 * planes : 4.6 + planes;
+  };
+  return double(ctas / slots) * round(slots) + (left ? round(left) : 0.0);
+}
+enum class Tile { W64x8, W32x16, W32x8 };
+Tile tile_for(const cfdb_ctx* ctx, const cfdb_mesh* m) {
+  const double a = step_time(ctx, m, 64, 8), b = step_time(ctx, m, 32, 16), c = step_time(ctx, m, 32, 8);
+  return a <= 1.03 * std::min(b, c) ? Tile::W64x8 : b <= c ? Tile::W32x16 : Tile::W32x8;
 }
 
 }  // namespace
@@ -326,8 +341,9 @@ bool wide_tiles(const cfdb_mesh* m) {
 // Upper bound of the fused Euler grid (sizes the per-CTA partials): at most
 // kEulerCtasPerSm resident CTAs per SM are ever requested.
 int euler_fused_grid(const cfdb_euler* e) {
-  const bool wide = wide_tiles(e->mesh);
-  const stencil::SweepShape sh = stencil::sweep_shape(e->ctx, e->mesh, wide ? 64 : 32, wide ? 8 : 16, kEulerCtasPerSm);
+  const Tile t = tile_for(e->ctx, e->mesh);
+  const stencil::SweepShape sh = stencil::sweep_shape(e->ctx, e->mesh, t == Tile::W64x8 ? 64 : 32, t == Tile::W32x16 ? 16 : 8,
+                                                      kEulerCtasPerSm);
   return sh.tiles * sh.chunks;
 }
 
@@ -349,7 +365,11 @@ static int euler_report(cfdb_euler* e, bool fold, EulerReport* out) {
 }
 
 int euler_fused_step(cfdb_euler* e, const void* U, void* Un, int64_t s) {
-  return wide_tiles(e->mesh) ? launch_euler<64, 8>(e, U, Un, s) : launch_euler<32, 16>(e, U, Un, s);
+  switch (tile_for(e->ctx, e->mesh)) {
+    case Tile::W64x8: return launch_euler<64, 8>(e, U, Un, s);
+    case Tile::W32x16: return launch_euler<32, 16>(e, U, Un, s);
+    default: return launch_euler<32, 8>(e, U, Un, s);
+  }
 }
 
 // ---------------------------------------------------------------------------
