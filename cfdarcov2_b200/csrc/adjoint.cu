@@ -247,11 +247,17 @@ int fused_wave_adjoint(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, co
     p.iV = float(1.0 / (m->dx * m->dy * m->dz));
     p.dt = float(dt);
     p.gc = static_cast<float*>(gc);
-    // 32-wide tiles of 16 rows: two CTAs per SM whatever the row length, 96^3 12.5 us
-    // against 15.8 with 64 x 8 (128 cells per row), 200^3 105 against 150, 128^3 27.6 the
-    // same; 48 x 8 where it pads the rows less (60 x 72 x 48: 6.3 against 9.4)
-    const double c48 = 1.1 * double((m->nz + 47) / 48 * 48), c32 = double((m->nz + 31) / 32 * 32);
-    if (c48 < c32) return stencil::launch_sweep<AdjPhys, 48, 8, 4, 2>(ctx, m, lam1, q, c, lam0, p, 0);
+    // 32 x 16 tiles: two CTAs per SM whatever the row length, 96^3 12.5 us against 15.8
+    // with 64 x 8 (128 cells per row), 200^3 105 against 150, 128^3 27.6 the same; 48 x 8
+    // where they pad the rows less (60 x 72 x 48: 6.3 against 9.4), 64 x 8 where 8 rows do
+    // (180 x 20 x 120: 10.2 against 11.9, 100^3 17.7 against 18.2); small meshes 32 x 8
+    // (16^3 2.5 against 3.1) or 64 x 8 (16 x 16 x 256 3.0 against 3.6)
+    const int few = stencil::few_tiles(ctx, m);
+    if (few == 32) return stencil::launch_sweep<AdjPhys, 32, 8, 4, 2>(ctx, m, lam1, q, c, lam0, p, 0);
+    const double c48 = 1.1 * stencil::tile_cover(m, 48, 8), c64 = stencil::tile_cover(m, 64, 8) / 0.94;
+    const double c32 = stencil::tile_cover(m, 32, 16);
+    if (!few && c48 < c32 && c48 < c64) return stencil::launch_sweep<AdjPhys, 48, 8, 4, 2>(ctx, m, lam1, q, c, lam0, p, 0);
+    if (few || c64 < c32) return stencil::launch_sweep<AdjPhys, 64, 8, 4, 2>(ctx, m, lam1, q, c, lam0, p, 0);
     return stencil::launch_sweep<AdjPhys, 32, 16, 3, 2>(ctx, m, lam1, q, c, lam0, p, 0);
   }
   // shapes the sweep cannot stage (nz % 4 != 0 or unaligned pointers): gather form

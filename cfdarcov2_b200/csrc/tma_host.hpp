@@ -91,6 +91,21 @@ inline SweepShape sweep_shape(const cfdb_ctx* ctx, const cfdb_mesh* m, int tz, i
   return s;
 }
 
+// Cells that tiles of tz x ty cover with their padding, per plane.
+inline double tile_cover(const cfdb_mesh* m, int64_t tz, int64_t ty) {
+  return double((m->nz + tz - 1) / tz * tz) * double((m->ny + ty - 1) / ty * ty);
+}
+
+// A mesh whose 8-row tiles, a CTA for every plane of each, are at most one per SM (32
+// wide, or 64 wide where those are no more than that) or two (32 wide) is all latency:
+// the smallest tile, with the fewest threads behind each barrier, is the fastest.
+// Its width, and 0 for other meshes.
+inline int few_tiles(const cfdb_ctx* ctx, const cfdb_mesh* m) {
+  const int64_t sms = std::max(1, ctx->num_sms), rows = (m->ny + 7) / 8 * m->nx;
+  const int64_t n32 = (m->nz + 31) / 32 * rows, n64 = (m->nz + 63) / 64 * rows;
+  return n32 <= sms ? 32 : m->nz >= 64 && n64 <= sms ? 64 : n32 <= 2 * sms ? 32 : 0;
+}
+
 // Launches one sweep: q holds the NF state fields, aux the NA auxiliary
 // fields (may be NULL when NA == 0), c the coefficient field (HAS_C), out
 // receives the NF new state fields.
