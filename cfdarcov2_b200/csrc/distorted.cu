@@ -183,7 +183,10 @@ int compact_wave_step(cfdb_ctx* ctx, cfdb_mesh* m, int dtype, const void* q, voi
     // cost per covered cell: 64 x 8 (two cells per thread) 1, 96 x 4 1.05 (half the
     // rows: more halo), 48 x 8 1.13, 32 x 8 1.12 (fewer threads per CTA).  96^3: 12.4 us
     // with 96, 14.5 with 32 and one cell per thread, 15.5 with 64; 96 x 96 x 48: 8.4 with
-    // 48, 10.1 with 64; 128^3: 29.4 with 64, 31.6 with 32, 40.4 with 96.
+    // 48, 10.1 with 64; 128^3: 29.4 with 64, 31.6 with 32, 40.4 with 96.  At most one tile
+    // and plane per SM: one cell per thread (64 x 8 x 8 2.54 against 2.59 with two).
+    if (stencil::few_tiles(ctx, m) == 32 && (m->nz + 31) / 32 * ((m->ny + 7) / 8) * m->nx <= ctx->num_sms)
+      return stencil::launch_face_sweep<DistFacePhys, 32, 8, 3, 1>(ctx, m, q, pg, qn, p, 0);
     auto cover = [&](int64_t tz) { return double((m->nz + tz - 1) / tz * tz); };
     const double c64 = cover(64), c96 = 1.05 * cover(96), c48 = 1.13 * cover(48), c32 = 1.12 * cover(32);
     const double least = std::min(std::min(c64, c96), std::min(c48, c32));
