@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 
 #include "heat_cell.cuh"
 #include "tma_host.hpp"
@@ -218,16 +219,17 @@ int dispatch_tz(cfdb_ctx* ctx, const cfdb_mesh* m, const void* q, void* out, con
 
 // Tile of the leapfrog sweep and of the heat sweep with the boundary copy, by
 // the cells it covers with its padding of rows and columns, times its cost per
-// covered cell (128- and 64-wide tiles of 8 rows 1, 40 and 32 wide ones of 16 rows
-// 1.07: more of their loads are halo).  200^3 d2t: 19.0 us with 40 (no padding),
-// 22.3 with 128 or 64 (256 cells per row), 21.4 with 32; 200 x 200 x 96: 10.2 us
-// with 32 against 12.2; 200 x 200 x 300: 27.6 us with 64 against 29.7 with 40.  (The
-// plain heat sweep keeps its own, below.)
+// covered cell: 128- and 64-wide tiles of 8 rows 1, 40 and 32 wide ones of 16 rows
+// 1.07, with the copy 1.15 (more of their loads are halo).  200^3 d2t: 19.0 us with 40
+// (no padding), 22.3 with 128 or 64 (256 cells per row), 21.4 with 32; 200 x 200 x 96:
+// 10.2 us with 32 against 12.2; 200 x 200 x 300: 27.6 us with 64 against 29.7 with 40;
+// 60 x 72 x 48 4.2 with 64 against 4.7 with 32; with the copy 90 x 90 x 224 5.6 with 128
+// against 5.9 with 32.  (The plain heat sweep keeps its own, below.)
 template <class Phys>
 int dispatch_padded(cfdb_ctx* ctx, const cfdb_mesh* m, const void* u, void* u_next, const typename Phys::Params& prm) {
-  auto cover = [&](int64_t tz, int64_t ty) { return double((m->nz + tz - 1) / tz * tz) * double((m->ny + ty - 1) / ty * ty); };
-  const double c128 = m->nz >= 128 ? cover(128, 8) : INFINITY, c64 = m->nz >= 64 ? cover(64, 8) : INFINITY;
-  const double c40 = 1.07 * cover(40, 16), c32 = 1.07 * cover(32, 16);
+  constexpr double narrow = std::is_same_v<Phys, HeatPhys<true>> ? 1.15 : 1.07;
+  const double c128 = m->nz >= 128 ? stencil::tile_cover(m, 128, 8) : INFINITY, c64 = stencil::tile_cover(m, 64, 8);
+  const double c40 = narrow * stencil::tile_cover(m, 40, 16), c32 = narrow * stencil::tile_cover(m, 32, 16);
   const double least = std::min(std::min(c128, c64), std::min(c40, c32));
   if (c128 == least) return stencil::launch_sweep<Phys, 128, 8, 6>(ctx, m, u, nullptr, nullptr, u_next, prm, 0);
   if (c64 == least) return stencil::launch_sweep<Phys, 64, 8, 6>(ctx, m, u, nullptr, nullptr, u_next, prm, 0);
@@ -238,15 +240,22 @@ int dispatch_padded(cfdb_ctx* ctx, const cfdb_mesh* m, const void* u, void* u_ne
 // Tile of the acoustic sweeps, by the cells it covers with its padding times its
 // cost per covered cell: 128 x 8 and 64 x 8 tiles 1 (the wider one first where
 // they tie with constant c, the narrower with a c field, whose fifth staged field
-// leaves it one more CTA per SM), 32 x 16 1.08, 40 x 16 and 48 x 8 1.15.  Constant c /
-// c field, us per step: 96^3 6.5 / 8.4 with 32, 7.9 / 10.9 with 64; 200^3 48.6 / 59.5
-// with 40, 56.3 / 70.6 with 128; 60 x 72 x 48 5.7 / 5.9 with 48, 7.2 / 7.7 with 32;
-// 128^3 11.2 / 16.3 with 128, 11.4 / 16.1 with 32; 100^3 9.1 with 128, 10.9 with 32.
+// leaves it one more CTA per SM, once there is more than one), 32 x 16 1.08, 40 x 16 and
+// 48 x 8 1.15.  Constant c / c field, us per step: 96^3 6.5 / 8.4 with 32, 7.9 / 10.9
+// with 64; 200^3 48.6 / 59.5 with 40, 56.3 / 70.6 with 128; 60 x 72 x 48 5.7 / 5.9 with 48,
+// 7.2 / 7.7 with 32; 128^3 11.2 / 16.3 with 128, 11.4 / 16.1 with 32; 100^3 9.1 with
+// 128, 10.9 with 32; 30 x 30 x 128 2.7 / 3.2 with 128 (120 CTAs), 2.7 / 3.6 with 64.  Small
+// meshes 32 x 8: 16^3 1.94 / 2.11 against 2.10 / 2.21 with 32 x 16.
 template <class Phys>
 int dispatch_wave(cfdb_ctx* ctx, const cfdb_mesh* m, const void* q, void* qn, const void* c, const typename Phys::Params& p) {
-  auto cover = [&](int64_t tz, int64_t ty) { return double((m->nz + tz - 1) / tz * tz) * double((m->ny + ty - 1) / ty * ty); };
-  const double c128 = (Phys::HAS_C ? 1.01 : 1.0) * cover(128, 8), c64 = (Phys::HAS_C ? 1.0 : 1.01) * cover(64, 8);
-  const double c48 = 1.15 * cover(48, 8), c40 = 1.15 * cover(40, 16), c32 = 1.08 * cover(32, 16);
+  const int few = stencil::few_tiles(ctx, m);
+  if (few == 32) return stencil::launch_sweep<Phys, 32, 8, 4>(ctx, m, q, nullptr, c, qn, p, 0);
+  if (few == 64) return stencil::launch_sweep<Phys, 64, 8, 4>(ctx, m, q, nullptr, c, qn, p, 0);
+  using stencil::tile_cover;
+  const bool one = (m->nz + 127) / 128 * ((m->ny + 7) / 8) * m->nx <= ctx->num_sms;  // 128 x 8: at most one CTA per SM
+  const bool narrow = Phys::HAS_C && !one;
+  const double c128 = (narrow ? 1.01 : 1.0) * tile_cover(m, 128, 8), c64 = (narrow ? 1.0 : 1.01) * tile_cover(m, 64, 8);
+  const double c48 = 1.15 * tile_cover(m, 48, 8), c40 = 1.15 * tile_cover(m, 40, 16), c32 = 1.08 * tile_cover(m, 32, 16);
   const double least = std::min({c128, c64, c48, c40, c32});
   if (c128 == least) return stencil::launch_sweep<Phys, 128, 8, 3>(ctx, m, q, nullptr, c, qn, p, 0);
   if (c64 == least) return stencil::launch_sweep<Phys, 64, 8, 4>(ctx, m, q, nullptr, c, qn, p, 0);
