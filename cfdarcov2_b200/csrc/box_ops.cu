@@ -1373,16 +1373,23 @@ int cfdb_mesh_need_box(cfdb_mesh* m, int dtype, bool* usable) {
 }
 
 // The kernel of a mesh: one value per direction and all directions, all
-// directions, or neither; NY = 2 rows per thread in FP32 only.
-#define BOX_FORMS(kernel, ...)                                   \
-  (uni && mask == 7 ? form<kernel<__VA_ARGS__, true, true>>(ctx) : mask == 7 ? form<kernel<__VA_ARGS__, false, true>>(ctx) : form<kernel<__VA_ARGS__, false, false>>(ctx))
+// directions, or neither (the heat step takes all); NY = 2 rows per thread in FP32 only.
+template <class R, int OP, int NY> auto sum_kernel(const cfdb_ctx* ctx, bool uni, int mask) {
+  if constexpr (OP != OP_HEAT)
+    if (mask != 7) return form<box_sum_k<R, OP, NY, false, false>>(ctx);
+  return uni ? form<box_sum_k<R, OP, NY, true, true>>(ctx) : form<box_sum_k<R, OP, NY, false, true>>(ctx);
+}
+template <class R, int NY> auto stab_kernel(const cfdb_ctx* ctx, bool uni, int mask) {
+  if (mask != 7) return form<box_stab_k<R, NY, false, false>>(ctx);
+  return uni ? form<box_stab_k<R, NY, true, true>>(ctx) : form<box_stab_k<R, NY, false, true>>(ctx);
+}
 
 template <class R, int OP> int launch_sum(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi, void* out, int mask, double k, double dt) {
   constexpr int NY = sizeof(R) == 4 ? 2 : 1;
   const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
-  const auto f = rows == 1 ? BOX_FORMS(box_sum_k, R, OP, 1) : BOX_FORMS(box_sum_k, R, OP, NY);
+  const auto f = rows == 1 ? sum_kernel<R, OP, 1>(ctx, uni, mask) : sum_kernel<R, OP, NY>(ctx, uni, mask);
   const Box<R> g = box_of<R>(ctx, m, rows, 1, f.plan, &blocks);
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask, R(k), R(dt));
   CFDB_LAUNCHED(ctx);
@@ -1394,7 +1401,7 @@ template <class R> int launch_stab(cfdb_ctx* ctx, cfdb_mesh* m, const void* phi,
   const bool uni = m->box[sizeof(R) == 8 ? 1 : 0].uni;
   const int rows = rows_per_thread<R>(ctx, m);
   unsigned blocks = 0;
-  const auto f = rows == 1 ? BOX_FORMS(box_stab_k, R, 1) : BOX_FORMS(box_stab_k, R, NY);
+  const auto f = rows == 1 ? stab_kernel<R, 1>(ctx, uni, mask) : stab_kernel<R, NY>(ctx, uni, mask);
   const Box<R> g = box_of<R>(ctx, m, rows, 2, f.plan, &blocks);
   f.kern<<<blocks, kThreads, 0, ctx->stream>>>(g, static_cast<const R*>(phi), static_cast<R*>(out), mask);
   CFDB_LAUNCHED(ctx);

@@ -183,7 +183,7 @@ void cfdb_jit_release(cfdb_ctx* ctx);  // unloads the context's run-time compile
 std::string graph_key(const char* kind, const struct cfdb_mesh* m, int dtype, int path, const void* a, const void* b,
                       const void* c, std::initializer_list<double> params);
 
-// Marching kernels whose chunk count a mesh keeps (box_ops.cu has 40).
+// Marching kernels whose chunk count a mesh keeps (box_ops.cu has 49).
 constexpr int kMarches = 64;
 
 struct cfdb_mesh {
