@@ -536,11 +536,13 @@ bool ring_ok(const cfdb_batch* b, int threads, int ctas_per_sm, const void* a, c
 
 // A step of up to 12 items per CTA is launched with programmatic stream
 // serialisation: its CTAs come up as the previous step's leave and wait for all of it
-// before they touch the pools.  With 16 steps per graph instead of two, us per step:
-// 26 mixed cubes of 20 to 51 cells 8.5 -> 7.6, 29 wave cubes of 16 to 29 6.3 -> 5.9,
-// 16 heat cubes of 16 to 40 4.1 -> 3.1 (two-step graphs had kept the host busy), 96
-// wave cubes of 20 to 50 (6 items per CTA) 34.5 -> 33.7, 96 mixed of 16 to 96 (8)
-// 73.2 -> 72.7; 64 wave cubes of 64 (14) lose 0.8 % with it.
+// before they touch the pools.  With 16 steps per graph instead of two, us per step
+// before and now: 4 mixed cubes of 16 to 24 cells 3.1 to 4.1 and 2.2, 16 heat cubes of 16
+// to 40 4.1 and 3.1 (two-step graphs had kept the host busy), 26 mixed of 20 to 51 8.2 and
+// 7.6 or 8.35 (the tuner finds either configuration); 29 wave cubes of 16 to 29 5.15 and
+// 5.35 (without it a step lasts whole microseconds, which it happened to meet).  With 6 to
+// 8 items per CTA (96 cubes) no more than the runs differ; 64 wave cubes of 64 (14) lose
+// 0.8 % with it.
 template <class... P, class... A>
 cudaError_t launch_step(void (*kern)(P...), int n_items, int grid, int threads, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg{};
