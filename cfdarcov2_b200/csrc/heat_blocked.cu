@@ -284,11 +284,8 @@ template <int K, int ZL, int WARPS> int launch(cfdb_ctx* ctx, const cfdb_mesh* m
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return cfdb_fail(ctx, CFDB_ECUDA, "cuTensorMapEncodeTiled (heat) failed with %d", int(r));
   auto kern = heat_blocked_k<K, ZL, WARPS>;
-  static std::atomic<bool> ready[kMaxDevices] = {};
-  if (!ready[ctx->device].load(std::memory_order_acquire)) {
-    CFDB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(L::SMEM)));
-    ready[ctx->device].store(true, std::memory_order_release);
-  }
+  // a setting of the CUDA context; cheap enough for every pass
+  CFDB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(L::SMEM)));
   a.ztiles = tiles_of(a.Z, L::EZ, kHaloZ);
   a.out = static_cast<float*>(dst);
   cudaLaunchConfig_t cfg{};
@@ -406,8 +403,6 @@ static int blocked_pass(cfdb_ctx* ctx, cfdb_mesh* m, const void* src, void* dst,
 int heat_blocked_run(cfdb_ctx* ctx, cfdb_mesh* m, void* Ta, void* Tb, double k, double dt, int32_t steps, int use_graph,
                      bool keep_other) {
   if (steps < 1 || check_sweep(ctx, m, {Ta, Tb}) != CFDB_OK) return CFDB_EUNSUPPORTED;
-  if (ctx->device < 0 || ctx->device >= kMaxDevices)
-    return cfdb_fail(ctx, CFDB_EUNSUPPORTED, "device ordinal %d beyond %d", ctx->device, kMaxDevices);
   // passes of two or three steps (four spill registers), as even as possible,
   // as many as the parity wants; one or two steps are single passes
   Plan plans[4];
