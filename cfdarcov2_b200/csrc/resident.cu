@@ -24,6 +24,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "cfdb_internal.hpp"
 #include "f32x2.cuh"
@@ -301,17 +302,19 @@ int run_cluster(cfdb_ctx* ctx, Kernel kern, const void* Ta, void* out, const Res
   return CFDB_OK;
 }
 
-// Whether a slab of P planes in shared memory beats the passes: a step costs 1200
-// SM cycles (cluster barrier, remote loads) and a quarter of one per cell of the
-// CTA; the launch and the field's way in and out 4500 more than a pass's.  Against 48
-// long shapes at 3, 5 and 200 steps: the faster form, or within 8 % of it, but for
-// runs of 3 steps (there within 1.3 of it).  Slabs of few wide planes (their x
-// neighbours all remote) lose at any size: 12x100x60 2.5 us against 1.7.
+// Whether a slab of P planes in shared memory beats the passes.  A step costs 1075 SM
+// cycles (cluster barrier), 112 for every 1024 cells of a plane that the neighbours
+// read remotely, and per 1024 groups of the CTA 731 and, begun ones, 331; the launch and
+// the field's way in and out 4500 more than passes' (12000 more than the single pass of
+// three steps).  Fitted to 48 long shapes at 200 steps (within 8 %); the choice is the
+// faster form or within 3 % of it but for 65x16x128 (8 %).  Slabs of few wide planes
+// (their x neighbours all remote) lose at any size: 12x100x60 2.5 us against 1.7.
 bool slab_wins(cfdb_ctx* ctx, cfdb_mesh* m, long long P, int32_t steps) {
   if (P <= kMaxPlanes) return false;
-  const double step = 1200.0 + 0.255 * double(P) * double(m->ny * m->nz);
+  const double plane = double(m->ny * m->nz), groups = double(P) * plane / (4.0 * kSlabThreads);
+  const double step = 1075.0 + 112.0 * plane / 1024.0 + 731.0 * groups + 331.0 * std::ceil(groups);
   if (steps <= 2) return steps == 2 && step < 3300.0;  // against single steps: the second launch costs about 2 us
-  return double(steps) * (1.07 * heat_pass_cycles(ctx, m) - step) > 4500.0;
+  return double(steps) * (1.03 * heat_pass_cycles(ctx, m) - step) > (steps == 3 ? 12000.0 : 4500.0);
 }
 
 }  // namespace
