@@ -316,10 +316,10 @@ int cfdb_wave_step(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, int path, const vo
  * graph (after two eager steps that perform any one-time setup) and replays
  * it, so host launch latency never gaps the device.  Asynchronous.
  * cfdb_heat_run, fused FP32: a uniform mesh whose field fits twice into the
- * shared memory of one thread-block cluster (e.g. 64^3) runs all steps in one
- * launch, field resident on chip; a larger one takes two or three steps per
- * pass over the field; same arithmetic, same result.  Only the buffer
- * *final_in_b names is defined afterwards. */
+ * shared memory of one thread-block cluster (e.g. 64^3, 512 x 16 x 16) runs all
+ * steps in one launch, field resident on chip, where that is the faster form;
+ * other fields take two or three steps per pass over the field; same arithmetic,
+ * same result.  Only the buffer *final_in_b names is defined afterwards. */
 int cfdb_heat_run(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, int path, void* T_a, void* T_b, double k, double dt,
                   int32_t steps, int use_graph, int* final_in_b);
 int cfdb_wave_run(cfdb_ctx* ctx, cfdb_mesh* mesh, int dtype, int path, void* q_a, void* q_b, const void* c_field,
@@ -347,8 +347,10 @@ int cfdb_euler_step(cfdb_euler* e, const void* U, void* U_next);
 int cfdb_euler_status(cfdb_euler* e, double* t, int64_t* steps_done, int* finished);
 /* Synchronous: totals rows (2 doubles each: sum rho V, sum E V), row 0 = initial state. */
 int cfdb_euler_totals(cfdb_euler* e, double* out, int64_t max_rows, int64_t* rows);
-/* Runs to t_end alternating U_a -> U_b -> U_a ..., checking the clock every
- * check_every steps; *final_in_b = 1 when the last state is in U_b.  At each
+/* Runs to t_end alternating U_a -> U_b -> U_a ..., checking the clock at least
+ * every check_every steps; wants an even number of launches since
+ * cfdb_euler_begin, which it leaves behind itself when check_every is even, so
+ * that a finished solver can be run again.  *final_in_b = 1 when the last state is in U_b.  At each
  * check a non-finite conservation total (a NaN or Inf in the state) stops
  * the run with CFDB_ENUMERIC. */
 int cfdb_euler_run(cfdb_euler* e, void* U_a, void* U_b, int64_t check_every, int64_t* steps_done,
