@@ -350,9 +350,9 @@ int cfdb_euler_totals(cfdb_euler* e, double* out, int64_t max_rows, int64_t* row
 /* Runs to t_end alternating U_a -> U_b -> U_a ..., checking the clock at least
  * every check_every steps; wants an even number of launches since
  * cfdb_euler_begin, which it leaves behind itself when check_every is even, so
- * that a finished solver can be run again.  *final_in_b = 1 when the last state is in U_b.  At each
- * check a non-finite conservation total (a NaN or Inf in the state) stops
- * the run with CFDB_ENUMERIC. */
+ * that a finished solver can be run again.  *final_in_b = 1 when the last state
+ * is in U_b.  At each check a non-finite conservation total (a NaN or Inf in the
+ * state) stops the run with CFDB_ENUMERIC. */
 int cfdb_euler_run(cfdb_euler* e, void* U_a, void* U_b, int64_t check_every, int64_t* steps_done,
                    int* final_in_b);
 
